@@ -61,8 +61,8 @@ _SIGNATURES = {
                                      I, I, I, I, I, I, P, STREAM]),
     # gated_delta.cu
     "fb_gdr_prepare": (I, [P, L, I, L, P, I, I, I, P, P, I, P, L, L, P, P, P, P, I, P, P, P, I, I, I, I, I, F, F, STREAM]),
-    "fb_gdr_recurrent": (I, [P, P, P, P, L, P, P, P, I, P, I, I, I, I, STREAM]),
-    "fb_gdr_channel_recurrent": (I, [P, P, P, P, L, P, P, P, I, P, I, I, I, I, STREAM]),
+    "fb_gdr_recurrent": (I, [P, P, P, P, L, P, P, P, I, I, P, I, I, I, I, STREAM]),
+    "fb_gdr_channel_recurrent": (I, [P, P, P, P, L, P, P, P, I, I, P, I, I, I, I, STREAM]),
     "fb_gdr_out_norm": (I, [P, P, L, I, L, I, I, P, I, F, P, I, I, I, I, STREAM]),
     # low_rank.cu
     "fb_low_rank_maps": (I, [P, L, I, L, I, I, P, I, P, P, P, P, P, P, P, P, STREAM]),

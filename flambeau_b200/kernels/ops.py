@@ -1060,8 +1060,8 @@ def gdr_recurrent(qkv, beta, decay, state, batch, o, G: int, H: int, dk: int, dv
         raise KernelError("gated delta: bad output or state")
     check(lib().fb_gdr_recurrent(qkv.data_ptr(), beta.data_ptr(), decay.data_ptr(), state.data_ptr(), state.stride(0),
                                  batch.seq_q_start_d.data_ptr(), batch.seq_q_len_d.data_ptr(),
-                                 batch.seq_slot_d.data_ptr(), batch.n_seqs, o.data_ptr(), G, H, dk, dv, _stream()),
-          "gdr_recurrent")
+                                 batch.seq_slot_d.data_ptr(), batch.n_seqs, int(qkv.shape[0]), o.data_ptr(),
+                                 G, H, dk, dv, _stream()), "gdr_recurrent")
 
 
 def gdr_channel_recurrent(qkv, beta, decay, state, batch, o, G: int, H: int, dk: int, dv: int) -> None:
@@ -1075,8 +1075,8 @@ def gdr_channel_recurrent(qkv, beta, decay, state, batch, o, G: int, H: int, dk:
         raise KernelError("gated delta: bad output, decay or state")
     check(lib().fb_gdr_channel_recurrent(qkv.data_ptr(), beta.data_ptr(), decay.data_ptr(), state.data_ptr(),
                                          state.stride(0), batch.seq_q_start_d.data_ptr(), batch.seq_q_len_d.data_ptr(),
-                                         batch.seq_slot_d.data_ptr(), batch.n_seqs, o.data_ptr(), G, H, dk, dv, _stream()),
-          "gdr_channel_recurrent")
+                                         batch.seq_slot_d.data_ptr(), batch.n_seqs, int(n), o.data_ptr(),
+                                         G, H, dk, dv, _stream()), "gdr_channel_recurrent")
 
 
 LOW_RANK_FUNCTIONS = {"plain": 0, "sigmoid": 1, "decay": 2}
