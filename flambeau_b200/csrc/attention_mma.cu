@@ -6,8 +6,9 @@
 // heads wider than 128), so that every K/V fragment fetched from shared memory feeds two row blocks; each walks
 // all visible key tiles with an online softmax.  CTAs are numbered heaviest first over all heads and sequences.
 // Sequences of a step with at most 16 rows (decoded tokens, portions of a few tokens) go to the split-key
-// arrangement instead (attention_split.cu); heads of 64 and 128 with pages that tile 64 keys go to the tcgen05
-// kernel (attention_tc.cu) unless that is switched off.
+// arrangement instead (attention_split.cu); heads of 64 and 128, and of 256 whose key rows are the values as well, with
+// pages that tile 64 keys go to the tcgen05 kernel (attention_tc.cu) unless that is switched off, or a cap, a gate, a
+// penalty on distance or kept first keys ask for this one.
 //
 // Keys and values come through the block table in tiles of 64 keys through a two-stage pipeline: whole pages by
 // tensor-map copies (128-byte swizzle) when a tile is a whole number of pages and the head a whole number of

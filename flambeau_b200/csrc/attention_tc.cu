@@ -1,5 +1,6 @@
 // Paged causal (sliding-window) attention for portions of prompts on the 5th-generation tensor cores
-// (tcgen05.mma, accumulators in tensor memory), for heads of 64 or 128 bfloat16 and pages that tile 64 keys.
+// (tcgen05.mma, accumulators in tensor memory), for heads of 64 or 128 bfloat16 and pages that tile 64 keys, and for heads
+// of 256 whose key rows are the values as well (attention over latents).
 //
 // A CTA owns one key/value head and 256 query rows = (256 / G) tokens x the G query heads that share the head, as
 // two row tiles of 128 that use every K/V tile fetched (one row tile when two would leave SMs without work), and
@@ -9,7 +10,9 @@
 //                  buffers per row tile: the scores run two key tiles ahead of the softmax;
 //   softmax        one thread per row (the row = its tensor-memory lane): the row's 64 scores in one tcgen05.ld
 //                  round trip, base-2 online softmax in float32, P rounded to bfloat16 and stored with tcgen05.st
-//                  over the scores it came from;
+//                  over the scores it came from; where the caller wants 16 bits of mantissa, what the rounding left is
+//                  stored behind it as bfloat16 again (two numbers a weight fill the columns that one score had), and
+//                  the product runs over both;
 //   O += P V       tcgen05.mma with P read from tensor memory and V as it lies in the cache ([key][dim], the
 //                  MN-major operand); O in tensor memory.
 //
@@ -22,6 +25,11 @@
 // phase that is current or just completed: one barrier per buffer, and one of its own for the last product.  Every
 // wait is bounded in time; when one runs out the kernel flags it, leaves its loops, frees its tensor memory and
 // returns.
+//
+// Heads of 256 (one row tile: O takes 256 columns): a tile is fetched once and serves as K and as V, its slot is free when
+// its product is through.  An MMA of 64 columns takes as long as one of 128 (62 to 72 cycles), so a key tile costs 16 x 65 for
+// the scores and 2 x 4 x 130 for the product with both parts of the weights, which bounds it.  2,048 tokens of 32 heads of
+// 256 over one latent row: 570 us on the mma.sync kernel (7 % of the tensor pipes' rate), 153 here.
 //
 // Formulas: crates/kernels-hip/src/kernels/attention_prefill_flash_tile_f16.cu:73-213 (tile + online softmax).
 #include "attention_common.cuh"
@@ -46,29 +54,31 @@ __device__ __forceinline__ float fast_exp2(float x) {
     return y;
 }
 
-template <int HD, int RT> struct TcSmem {
+template <int HD, int RT, bool SHARED> struct TcSmem {
     static constexpr int Q_BYTES = BM * HD * 2;                 // one row tile: [HD/64 column blocks][128 rows][128 bytes]
     static constexpr int KV_BYTES = BN * HD * 2;                // one K or V tile: [HD/64][64 keys][128 bytes]
     static constexpr int TAIL_BYTES = 256;                      // barriers, tensor-memory address, flag
-    static constexpr int USED = RT * Q_BYTES + NKV * 2 * KV_BYTES + TAIL_BYTES + 1024 /* alignment */;
+    static constexpr int USED = RT * Q_BYTES + NKV * (SHARED ? 1 : 2) * KV_BYTES + TAIL_BYTES + 1024 /* alignment */;
     // one CTA per SM: two would both want all of tensor memory
     static constexpr int BYTES = USED > 120 * 1024 ? USED : 120 * 1024;
 };
 
 // RT row tiles of 128 rows per CTA: with two, both use every K/V tile that is fetched and the tensor pipe works for
 // one under the softmax of the other; with one, a short portion still spreads over enough CTAs.
-template <int HD, int RT>
+// HILO: the weights enter the product as two bfloat16 numbers each.  SHARED: the key rows are the values as well.
+template <int HD, int RT, bool HILO, bool SHARED>
 __global__ void __launch_bounds__(tc_threads(RT), 1)
 attention_tc_kernel(const __grid_constant__ AttnArgs a) {
     fb_pdl_launch_dependents();
-    using SM = TcSmem<HD, RT>;
+    static_assert(RT * 128 + RT * (HD > 128 ? HD : 128) <= TMEM_COLS, "tensor memory");
+    using SM = TcSmem<HD, RT, SHARED>;
     constexpr int CB = HD / 64;                                 // 64-column blocks of a head
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     uint8_t* Qs = smem;                                         // [RT] row tiles
     uint8_t* Ks = Qs + RT * SM::Q_BYTES;                        // [NKV] tiles
-    uint8_t* Vs = Ks + NKV * SM::KV_BYTES;                      // [NKV] tiles
+    uint8_t* Vs = SHARED ? Ks : Ks + NKV * SM::KV_BYTES;        // [NKV] tiles
     uint8_t* tail = Vs + NKV * SM::KV_BYTES;
     uint64_t* bars = reinterpret_cast<uint64_t*>(tail);
     uint64_t* k_full = bars;                                    // [NKV] a K tile has landed
@@ -203,10 +213,15 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
         for (int j = 0; j < n_tiles; ++j) {
             const int s = j % NKV;
             const uint32_t reuse = (uint32_t)(j / NKV - 1) & 1u;
-            if (j >= NKV && !wait(&k_empty[s], reuse)) break;
-            issue(Ks + s * SM::KV_BYTES, &a.map_k, &k_full[s], page);
-            if (j >= NKV && !wait(&v_empty[s], reuse)) break;
-            issue(Vs + s * SM::KV_BYTES, &a.map_v, &v_full[s], page);
+            if constexpr (SHARED) {                             // (the tile's product is the last to read it)
+                if (j >= NKV && !wait(&v_empty[s], reuse)) break;
+                issue(Ks + s * SM::KV_BYTES, &a.map_k, &k_full[s], page);
+            } else {
+                if (j >= NKV && !wait(&k_empty[s], reuse)) break;
+                issue(Ks + s * SM::KV_BYTES, &a.map_k, &k_full[s], page);
+                if (j >= NKV && !wait(&v_empty[s], reuse)) break;
+                issue(Vs + s * SM::KV_BYTES, &a.map_v, &v_full[s], page);
+            }
             page = lookup(j + 1);                               // in flight while this warp waits for the next slot
         }
     } else if (warp < 4) {
@@ -241,11 +256,11 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
                 tmem_fence_after();
                 issue_s(j);
                 umma_commit(smem_u32(&s_full[2 * t + (j & 1)]));
-                umma_commit(smem_u32(&k_empty[j % NKV]));
+                if (!SHARED) umma_commit(smem_u32(&k_empty[j % NKV]));
             }
             for (int j = 0; ok && j < n_tiles; ++j) {
                 const bool more = j + 2 < n_tiles;              // there are scores left to compute
-                ok = wait(&v_full[j % NKV], (uint32_t)(j / NKV) & 1u);
+                if (!SHARED) ok = wait(&v_full[j % NKV], (uint32_t)(j / NKV) & 1u);
                 if (ok && more) ok = wait(&k_full[(j + 2) % NKV], (uint32_t)((j + 2) / NKV) & 1u);
                 // (the barrier's first phase is tile 0's clearing if tile 0 has rows to clear, else the last tile's)
                 if (ok && t > 0 && has_dead(j)) ok = wait(v_clean, (j > 0 && has_dead(0)) ? 1u : 0u);
@@ -259,6 +274,7 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
                 for (int kk = 0; kk < BN / UMMA_K; ++kk) {      // 16 keys = 8 columns of P each
                     const uint64_t db = umma_desc_mn(v_addr + (uint32_t)(kk * 16 * 128), BN * 128, 1024);
                     umma_bf16_ts(d, p_addr + (uint32_t)(kk * 8), db, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
+                    if (HILO) umma_bf16_ts(d, p_addr + (uint32_t)(BN / 2 + kk * 8), db, idesc_o, 1u);
                 }
                 if (more) issue_s(j + 2);
                 umma_commit(smem_u32(&pv_done[t]));
@@ -266,7 +282,7 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
                 umma_commit(smem_u32(&v_empty[j % NKV]));
                 if (more) {
                     umma_commit(smem_u32(&s_full[2 * t + (j & 1)]));
-                    umma_commit(smem_u32(&k_empty[(j + 2) % NKV]));
+                    if (!SHARED) umma_commit(smem_u32(&k_empty[(j + 2) % NKV]));
                 }
             }
         }
@@ -357,7 +373,7 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
             float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
             for (int c = 0; c < BN / 32; ++c) {
-                uint32_t pk[16];
+                uint32_t pk[16], rest[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     // a masked score is -inf: 2^-inf = 0
@@ -365,13 +381,15 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
                     const float p1 = fast_exp2(fmaf(__uint_as_float(v[c][2 * i + 1]), a.scale_log2e, neg_ref));
                     sum4[i & 3] += p0 + p1;
                     pk[i] = pack_bf16(p0, p1);
+                    if (HILO) rest[i] = pack_bf16_remainder(p0, p1);
                 }
                 tmem_st16(s_addr + (uint32_t)(c * 16), pk);
+                if (HILO) tmem_st16(s_addr + (uint32_t)(BN / 2 + c * 16), rest);
             }
             l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
             if (t == 0 && has_dead(j)) {                        // (only the first and the last tile can)
                 const int dead_lo = dead_lo_of(j), dead_hi = dead_hi_of(j);
-                ok = __all_sync(0xffffffffu, wait(&v_full[j % NKV], (uint32_t)(j / NKV) & 1u));
+                ok = __all_sync(0xffffffffu, wait(SHARED ? &k_full[j % NKV] : &v_full[j % NKV], (uint32_t)(j / NKV) & 1u));
                 if (!ok) continue;
                 uint8_t* vt = Vs + (j % NKV) * SM::KV_BYTES;
                 const int n_dead = dead_lo + (BN - dead_hi);
@@ -422,10 +440,10 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
     }
 }
 
-template <int HD, int RT>
+template <int HD, int RT, bool HILO, bool SHARED>
 int launch_tc(const AttnArgs& a, int n_seqs, int max_q_len, cudaStream_t stream) {
-    auto kern = attention_tc_kernel<HD, RT>;
-    using SM = TcSmem<HD, RT>;
+    auto kern = attention_tc_kernel<HD, RT, HILO, SHARED>;
+    using SM = TcSmem<HD, RT, SHARED>;
     static bool configured[FB_MAX_DEVICES] = {};
     if (fb_needs_setup(configured)) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::BYTES);
@@ -440,25 +458,33 @@ int launch_tc(const AttnArgs& a, int n_seqs, int max_q_len, cudaStream_t stream)
 }
 
 // Two row tiles per CTA when that still gives every SM a CTA, else one.
-template <int HD>
+template <int HD, bool HILO>
 int launch_tc(const AttnArgs& a, int n_seqs, int max_q_len, cudaStream_t stream) {
     const int sms = fb_sm_count();
     const int TQ2 = 2 * BM / (a.nh / a.nkv);
     const long ctas2 = (long)((max_q_len + TQ2 - 1) / TQ2) * a.nkv * portion_seqs(a);   // an upper bound: short ones leave early
-    return ctas2 >= sms ? launch_tc<HD, 2>(a, n_seqs, max_q_len, stream) : launch_tc<HD, 1>(a, n_seqs, max_q_len, stream);
+    return ctas2 >= sms ? launch_tc<HD, 2, HILO, false>(a, n_seqs, max_q_len, stream)
+                        : launch_tc<HD, 1, HILO, false>(a, n_seqs, max_q_len, stream);
+}
+
+template <bool HILO>
+int launch_tc(const AttnArgs& a, int n_seqs, int max_q_len, cudaStream_t stream) {
+    return a.hd == 64    ? launch_tc<64, HILO>(a, n_seqs, max_q_len, stream)
+           : a.hd == 128 ? launch_tc<128, HILO>(a, n_seqs, max_q_len, stream)
+                         : launch_tc<256, 1, HILO, true>(a, n_seqs, max_q_len, stream);
 }
 
 }  // namespace
 
 bool fb_attention_tc_takes(const AttnArgs& a, bool tma) {
     const int G = a.nh / a.nkv;
-    // (its weights are bfloat16 in tensor memory: steps that want them in two parts run on the mma.sync kernel)
-    // (nor does it walk kept first keys behind a window, cap scores or gate heads)
-    return tma && !a.score_slopes && !a.weights_hi_lo && a.keep_first == 0 && a.cap_log2e == 0.0f && !a.head_gate && (a.hd == 64 || a.hd == 128) && G <= BM && BN % a.page_size == 0 &&
+    // (it does not walk kept first keys behind a window, cap scores or gate heads)
+    return tma && !a.score_slopes && a.keep_first == 0 && a.cap_log2e == 0.0f && !a.head_gate &&
+           (a.hd == 64 || a.hd == 128 || (a.hd == 256 && a.k_pool == a.v_pool)) && G <= BM && BN % a.page_size == 0 &&
            a.out_stride % 8 == 0 &&
            (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
 }
 
 int fb_launch_attention_tc(const AttnArgs& a, int n_seqs, int max_q_len, cudaStream_t stream) {
-    return a.hd == 64 ? launch_tc<64>(a, n_seqs, max_q_len, stream) : launch_tc<128>(a, n_seqs, max_q_len, stream);
+    return a.weights_hi_lo ? launch_tc<true>(a, n_seqs, max_q_len, stream) : launch_tc<false>(a, n_seqs, max_q_len, stream);
 }
