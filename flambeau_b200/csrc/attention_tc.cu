@@ -31,6 +31,11 @@
 // the scores and 2 x 4 x 130 for the product with both parts of the weights, which bounds it.  2,048 tokens of 32 heads of
 // 256 over one latent row: 570 us on the mma.sync kernel (7 % of the tensor pipes' rate), 153 here.
 //
+// Differential attention (two score maps of 64 a head over values of 128): the row tiles are the two maps of the same 128
+// rows, each with its column block of Q and K and both on one V tile.  At the end the threads of both take half of the
+// columns each, read both maps' O from tensor memory and form the difference, its norm and the gate.  A key tile costs 8 x 65
+// for the scores and 16 x 65 for the products.  2,048 tokens of 32 heads: 373 us on the mma.sync kernel, 141 here.
+//
 // Formulas: crates/kernels-hip/src/kernels/attention_prefill_flash_tile_f16.cu:73-213 (tile + online softmax).
 #include "attention_common.cuh"
 #include "umma.cuh"
@@ -54,11 +59,12 @@ __device__ __forceinline__ float fast_exp2(float x) {
     return y;
 }
 
-template <int HD, int RT, bool SHARED> struct TcSmem {
+template <int HD, int RT, bool SHARED, bool DIFF> struct TcSmem {
+    static constexpr int Q_TILES = DIFF ? 1 : RT;               // (the maps' rows lie side by side in one)
     static constexpr int Q_BYTES = BM * HD * 2;                 // one row tile: [HD/64 column blocks][128 rows][128 bytes]
     static constexpr int KV_BYTES = BN * HD * 2;                // one K or V tile: [HD/64][64 keys][128 bytes]
-    static constexpr int TAIL_BYTES = 256;                      // barriers, tensor-memory address, flag
-    static constexpr int USED = RT * Q_BYTES + NKV * (SHARED ? 1 : 2) * KV_BYTES + TAIL_BYTES + 1024 /* alignment */;
+    static constexpr int TAIL_BYTES = 256 + (DIFF ? 4 * BM * 4 : 0);                      // barriers, tensor-memory address, flag
+    static constexpr int USED = Q_TILES * Q_BYTES + NKV * (SHARED ? 1 : 2) * KV_BYTES + TAIL_BYTES + 1024 /* alignment */;
     // one CTA per SM: two would both want all of tensor memory
     static constexpr int BYTES = USED > 120 * 1024 ? USED : 120 * 1024;
 };
@@ -66,18 +72,21 @@ template <int HD, int RT, bool SHARED> struct TcSmem {
 // RT row tiles of 128 rows per CTA: with two, both use every K/V tile that is fetched and the tensor pipe works for
 // one under the softmax of the other; with one, a short portion still spreads over enough CTAs.
 // HILO: the weights enter the product as two bfloat16 numbers each.  SHARED: the key rows are the values as well.
-template <int HD, int RT, bool HILO, bool SHARED>
+// DIFF: differential attention; the row tiles are the two maps of the same rows.
+template <int HD, int RT, bool HILO, bool SHARED, bool DIFF>
 __global__ void __launch_bounds__(tc_threads(RT), 1)
 attention_tc_kernel(const __grid_constant__ AttnArgs a) {
     fb_pdl_launch_dependents();
     static_assert(RT * 128 + RT * (HD > 128 ? HD : 128) <= TMEM_COLS, "tensor memory");
-    using SM = TcSmem<HD, RT, SHARED>;
+    static_assert(!DIFF || (HD == 128 && RT == 2 && !SHARED), "two maps of 64 over values of 128");
+    using SM = TcSmem<HD, RT, SHARED, DIFF>;
+    constexpr int ROWS = DIFF ? BM : RT * BM;                   // query rows of the CTA
     constexpr int CB = HD / 64;                                 // 64-column blocks of a head
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     uint8_t* Qs = smem;                                         // [RT] row tiles
-    uint8_t* Ks = Qs + RT * SM::Q_BYTES;                        // [NKV] tiles
+    uint8_t* Ks = Qs + SM::Q_TILES * SM::Q_BYTES;                        // [NKV] tiles
     uint8_t* Vs = SHARED ? Ks : Ks + NKV * SM::KV_BYTES;        // [NKV] tiles
     uint8_t* tail = Vs + NKV * SM::KV_BYTES;
     uint64_t* bars = reinterpret_cast<uint64_t*>(tail);
@@ -107,14 +116,14 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
     const int q_tiles = gridDim.x / pairs;
     const int q_len = a.seq_q_len[seq];
     if (q_len * G <= a.short_rows) return;                      // the split-key arrangement's
-    const int TQ = RT * BM / G;
+    const int TQ = ROWS / G;
     const int tok0 = (q_tiles - 1 - rank) * TQ;               // later tokens see more keys: start them first
     if (tok0 >= q_len) return;
     const int ntok = min(TQ, q_len - tok0);
     const int q_start = a.seq_q_start[seq], pos0 = a.seq_pos_start[seq];
     const int rows_valid = ntok * G;                            // of the CTA's RT * 128 rows
     const int p_first = pos0 + tok0, p_last = pos0 + tok0 + ntok - 1;
-    const int t_lo = (a.window > 0 && p_first - a.window + 1 > 0) ? p_first - a.window + 1 : 0;
+    const int t_lo = fb_first_key(p_first, a.window, DIFF ? a.chunk : 0);
     const int t_hi = p_last;
     const int k_begin = (t_lo / BN) * BN, k_end = t_hi + 1;
     const int n_tiles = (k_end - k_begin + BN - 1) / BN;        // both row tiles walk all of them
@@ -239,12 +248,12 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
         if (t < RT && elect_one()) {
             constexpr uint32_t idesc_s = umma_idesc(BN);
             constexpr uint32_t idesc_o = umma_idesc(HD, true);
-            const uint32_t q_addr = smem_u32(Qs + t * SM::Q_BYTES);
+            const uint32_t q_addr = smem_u32(Qs + t * (DIFF ? BM * 128 : SM::Q_BYTES));
             auto issue_s = [&](int j) {                         // S buffer j & 1 of the row tile = Q_t K_j^T
-                const uint32_t k_addr = smem_u32(Ks + (j % NKV) * SM::KV_BYTES);
+                const uint32_t k_addr = smem_u32(Ks + (j % NKV) * SM::KV_BYTES + (DIFF ? t * (BN * 128) : 0));
                 const uint32_t d = tmem_base + (uint32_t)((2 * t + (j & 1)) * BN);
 #pragma unroll
-                for (int kk = 0; kk < HD / UMMA_K; ++kk)
+                for (int kk = 0; kk < (DIFF ? 64 : HD) / UMMA_K; ++kk)
                     umma_bf16(d, umma_desc(q_addr + (uint32_t)((kk / 4) * (BM * 128) + (kk % 4) * 32)),
                               umma_desc(k_addr + (uint32_t)((kk / 4) * (BN * 128) + (kk % 4) * 32)), idesc_s,
                               kk > 0 ? 1u : 0u);
@@ -291,15 +300,15 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
         // ================= softmax: thread = query row = tensor-memory lane; warps 4..7 row tile 0, 8..11 row tile 1 =====
         const int quarter = warp & 3;                           // the lanes this warp may read
         const int t = (warp - 4) >> 2;                          // its row tile
-        const int r = t * BM + quarter * 32 + lane;             // row of the CTA
+        const int r = (DIFF ? 0 : t * BM) + quarter * 32 + lane;   // row of the CTA
         const bool valid = r < rows_valid;
         const int token = q_start + tok0 + r / G, head = kvh * G + r % G;
         // ---- stage Q (zero rows beyond the CTA's share) ----
         {
-            const __nv_bfloat16* src = a.q + (size_t)token * a.q_stride + (size_t)head * hd;
-            uint8_t* qrow = Qs + t * SM::Q_BYTES + (r - t * BM) * 128;
+            const __nv_bfloat16* src = a.q + (size_t)token * a.q_stride + (size_t)head * hd + (DIFF ? t * 64 : 0);
+            uint8_t* qrow = Qs + t * (DIFF ? BM * 128 : SM::Q_BYTES) + (quarter * 32 + lane) * 128;
 #pragma unroll
-            for (int c = 0; c < HD / 8; ++c) {
+            for (int c = 0; c < (DIFF ? 64 : HD) / 8; ++c) {
                 uint4 v = make_uint4(0, 0, 0, 0);
                 if (valid) v = *reinterpret_cast<const uint4*>(src + c * 8);
                 *reinterpret_cast<uint4*>(qrow + (c / 8) * (BM * 128) + (((c & 7) ^ (r & 7)) << 4)) = v;
@@ -308,7 +317,7 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
             mbar_arrive(smem_u32(q_full));
         }
         const int p_row = valid ? pos0 + tok0 + r / G : -1;     // a row beyond the share sees nothing
-        const int t0_row = (a.window > 0 && p_row - a.window + 1 > 0) ? p_row - a.window + 1 : 0;
+        const int t0_row = valid ? fb_first_key(p_row, a.window, DIFF ? a.chunk : 0) : 0;
         const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
         const uint32_t o_addr = lane_addr + (uint32_t)(RT * 128 + t * 128); // O of this row
         float m_ref = -INFINITY;                                // reference point of the exponentials (scaled, base 2)
@@ -408,7 +417,45 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
         // ---- O / l, written as bfloat16 ----
         // (a barrier of its own: pv_done may be one or two phases on by now, and a wait names a phase by its parity)
         if (ok) ok = __all_sync(0xffffffffu, wait(&o_done[t], 0));
-        if (ok) {
+        if constexpr (DIFF) {
+            // out = (a_1 - lambda a_2) / rms * out_scale * gate with a_m = O_m / l_m: this thread's half of the columns
+            float* inv_of = reinterpret_cast<float*>(tail + 256);       // [2 maps][128 rows]
+            float* squares = inv_of + 2 * BM;                           // [2 halves][128 rows]
+            const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+            inv_of[t * BM + r] = inv;
+            if (ok) ok = __all_sync(0xffffffffu, wait(&o_done[1 - t], 0));
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            tmem_fence_after();
+            const float inv1 = inv_of[r], inv2 = a.lambda * inv_of[BM + r];
+            const uint32_t o1 = lane_addr + (uint32_t)(RT * 128 + t * 64), o2 = o1 + 128;
+            float d[64], ss = 0.0f;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                uint32_t v1[32], v2[32];
+                tmem_ld32_nowait(o1 + (uint32_t)(c * 32), v1);
+                tmem_ld32_nowait(o2 + (uint32_t)(c * 32), v2);
+                tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    d[c * 32 + i] = __uint_as_float(v1[i]) * inv1 - inv2 * __uint_as_float(v2[i]);
+                    ss = fmaf(d[c * 32 + i], d[c * 32 + i], ss);
+                }
+            }
+            squares[t * BM + r] = ss;
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            if (ok && valid) {
+                const float f = a.out_scale * (a.row_gate ? a.row_gate[(size_t)token * a.nh + head] : 1.0f) /
+                                sqrtf((squares[r] + squares[BM + r]) * (1.0f / HD) + a.eps);
+                __nv_bfloat16* dst = a.out + (size_t)token * a.out_stride + (size_t)head * HD + t * 64;
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    uint32_t w[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) w[e] = pack_bf16(d[8 * c + 2 * e] * f, d[8 * c + 2 * e + 1] * f);
+                    *reinterpret_cast<uint4*>(dst + 8 * c) = make_uint4(w[0], w[1], w[2], w[3]);
+                }
+            }
+        } else if (ok) {
             tmem_fence_after();
             l += sink_term(a, head, m_ref);
             const float inv = l > 0.0f ? 1.0f / l : 0.0f;
@@ -440,10 +487,10 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
     }
 }
 
-template <int HD, int RT, bool HILO, bool SHARED>
+template <int HD, int RT, bool HILO, bool SHARED, bool DIFF = false>
 int launch_tc(const AttnArgs& a, int n_seqs, int max_q_len, cudaStream_t stream) {
-    auto kern = attention_tc_kernel<HD, RT, HILO, SHARED>;
-    using SM = TcSmem<HD, RT, SHARED>;
+    auto kern = attention_tc_kernel<HD, RT, HILO, SHARED, DIFF>;
+    using SM = TcSmem<HD, RT, SHARED, DIFF>;
     static bool configured[FB_MAX_DEVICES] = {};
     if (fb_needs_setup(configured)) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::BYTES);
@@ -451,7 +498,7 @@ int launch_tc(const AttnArgs& a, int n_seqs, int max_q_len, cudaStream_t stream)
                                              SM::BYTES, cudaGetErrorString(e));
         fb_setup_done(configured);
     }
-    const int TQ = RT * BM / (a.nh / a.nkv);
+    const int TQ = (DIFF ? 1 : RT) * BM / (a.nh / a.nkv);
     const dim3 grid(((max_q_len + TQ - 1) / TQ) * a.nkv * portion_seqs(a));
     fb_launch_class(FB_LAUNCH_ATTENTION_TC, (kern), grid, tc_threads(RT), (size_t)SM::BYTES, stream, a);
     return fb_check_launch("attention_tc");
@@ -487,4 +534,14 @@ bool fb_attention_tc_takes(const AttnArgs& a, bool tma) {
 
 int fb_launch_attention_tc(const AttnArgs& a, int n_seqs, int max_q_len, cudaStream_t stream) {
     return a.weights_hi_lo ? launch_tc<true>(a, n_seqs, max_q_len, stream) : launch_tc<false>(a, n_seqs, max_q_len, stream);
+}
+
+// Differential attention over portions: maps of 64, values of 128, pages that tile 64 keys, rows that leave in 16-byte pieces.
+bool fb_diff_attention_tc_takes(int nh, int nkv, int kd, int vd, int page_size, const void* out, long out_stride) {
+    return kd == 64 && vd == 128 && nh / nkv <= BM && page_size >= 8 && page_size <= BN && BN % page_size == 0 &&
+           out_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+}
+
+int fb_launch_diff_attention_tc(const AttnArgs& a, int n_seqs, int max_q_len, cudaStream_t stream) {
+    return launch_tc<128, 2, true, false, true>(a, n_seqs, max_q_len, stream);
 }

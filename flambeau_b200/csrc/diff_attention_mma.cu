@@ -6,7 +6,8 @@
 // rows of a CTA share every K/V tile it fetches, so grouped heads cost no second read of the cache.  A warp owns 16
 // rows of ONE map; the warps of map 1 and the warps of map 2 of the same rows sit in one CTA and meet at the end.
 //
-// Two arrangements of one kernel:
+// Portions with maps of 64 over values of 128 run on the tcgen05 kernel (attention_tc.cu).  Else two arrangements of one
+// kernel:
 //   portions  (rows of the sequence > short_rows): a CTA owns 64 rows (4 warps per map), walks the 64-key tiles its
 //             rows can see, every warp scoring the whole tile for its 16 rows (32 keys at a time), and ends with the epilogue
 //             (a1 - lambda a2, head norm, gate) through shared memory.
@@ -584,7 +585,23 @@ FB_API int fb_diff_attention_mma(const void* q, long long q_stride, void* out, l
     a.part_o = nullptr; a.part_ml = nullptr;
     a.status = status;
     const int HG = nh / nkv;
-    if (any_long) {
+    if (any_long && fb_diff_attention_tc_takes(nh, nkv, kd, vd, page_size, out, (long)out_stride)) {
+        AttnArgs t = {};
+        const long pool_rows = (long)n_pages * nkv * page_size;
+        int rc = fb_tensor_map_bf16(&t.map_k, k_pool, pool_rows, 2 * kd, 2 * kd, 64, page_size);
+        if (rc) return rc;
+        rc = fb_tensor_map_bf16(&t.map_v, v_pool, pool_rows, vd, vd, 64, page_size);
+        if (rc) return rc;
+        t.q = a.q; t.q_stride = a.q_stride; t.out = a.out; t.out_stride = a.out_stride;
+        t.k_pool = a.k_pool; t.v_pool = a.v_pool; t.page_size = page_size; t.n_pages = n_pages;
+        t.block_table = block_table; t.table_stride = table_stride; t.table_base = table_base;
+        t.seq_q_start = seq_q_start; t.seq_q_len = seq_q_len; t.seq_pos_start = seq_pos_start;
+        t.n_seqs = n_seqs; t.nh = nh; t.nkv = nkv; t.hd = 2 * kd; t.window = window; t.chunk = chunk;
+        t.scale_log2e = a.scale_log2e; t.lambda = lambda; t.eps = eps; t.out_scale = out_scale; t.row_gate = gate;
+        t.short_rows = a.short_rows; t.status = status;
+        rc = fb_launch_diff_attention_tc(t, n_seqs, max_q_len, stream);
+        if (rc) return rc;
+    } else if (any_long) {
         a.n_stages = stages_for(kd, vd, false);
         const long rows = (long)max_q_len * HG;
         const int rc = dispatch_diff_mma<false>(a, dim3((unsigned)((rows + 63) / 64), nkv, n_seqs), stream);
