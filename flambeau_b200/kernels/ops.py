@@ -484,6 +484,52 @@ def paged_attention_simt(q, out, k_pool, v_pool, block_table, positions, row_seq
         "paged_attention_simt")
 
 
+def f32_attention_supported(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, nh: int, nkv: int,
+                            hd: int, vd: int) -> bool:
+    """Whether the tiled float32 kernel takes this geometry: sizes that are multiples of 4 up to 256, up to 64 query heads a
+    key/value head, rows that start on 16-byte borders."""
+    return (q.dtype == out.dtype == k_pool.dtype == v_pool.dtype == torch.float32 and hd % 4 == 0 and vd % 4 == 0 and hd <= 256
+            and vd <= 256 and nh % nkv == 0 and nh // nkv <= 64 and q.stride(1) == 1 and out.stride(1) == 1
+            and q.stride(0) % 4 == 0 and out.stride(0) % 4 == 0
+            and all(t.data_ptr() % 16 == 0 for t in (q, out, k_pool, v_pool)))
+
+
+def paged_attention_f32(q, out, k_pool, v_pool, block_table, seq_q_start, seq_q_len, seq_pos_start, n_seqs: int, max_q_len: int,
+                        max_kv_len: int, any_short: bool, any_long: bool, nh: int, nkv: int, hd: int, window: int, scale: float,
+                        status, table_base=None, score_slopes=None, sinks=None, vd: int = 0, keep_first: int = 0,
+                        table_head: int = 0, softcap: float = 0.0, head_gate=None, alloc=None) -> None:
+    """paged_attention_simt's result in float32, tile by tile (csrc/attention_f32.cu); sequences are described per entry of
+    the step (first row, rows, first position).  any_short / any_long: whether the step holds sequences with rows * (nh / nkv)
+    <= 16 / > 16 (groups of more than 16 heads count as long).  `alloc(n)` returns n float32 of scratch for the results of
+    stretches of keys (default: a fresh tensor)."""
+    _cuda(q, out, k_pool, v_pool, block_table, seq_q_start, seq_q_len, seq_pos_start, status, table_base, sinks)
+    _i32(table_base, "table_base")
+    n = q.shape[0]
+    vd = int(vd) or hd
+    n_pages, pool_kv, page_size, pool_hd = k_pool.shape
+    if pool_kv != nkv or pool_hd != hd or q.shape[1] != nh * hd or out.shape[1] != nh * vd or out.shape[0] != n \
+            or tuple(v_pool.shape) != (n_pages, nkv, page_size, vd):
+        raise KernelError("attention: shapes do not match the head counts")
+    if sinks is not None and (sinks.dtype != torch.float32 or sinks.numel() != nh or not sinks.is_contiguous()):
+        raise KernelError("attention: sinks are one float32 per query head")
+    if not f32_attention_supported(q, out, k_pool, v_pool, nh, nkv, hd, vd):
+        raise KernelError("attention_f32: float32 operands with sizes that are multiples of 4 up to 256")
+    if not k_pool.is_contiguous() or not v_pool.is_contiguous():
+        raise KernelError("attention: cache pools must be contiguous")
+    max_keys = max_kv_len if not window else min(max_kv_len, window + int(keep_first) + max_q_len)
+    splits = lib().fb_attention_f32_splits(n_seqs, nkv, nh // nkv, max_q_len, int(max_keys))
+    part, floats = None, 0
+    if splits > 1:
+        floats = splits * n * nh * (vd + 2)
+        part = alloc(floats) if alloc is not None else torch.empty(floats, dtype=torch.float32, device=q.device)
+    check(lib().fb_paged_attention_f32(
+        q.data_ptr(), _rows(q), out.data_ptr(), _rows(out), k_pool.data_ptr(), v_pool.data_ptr(), page_size, n_pages,
+        block_table.data_ptr(), block_table.stride(0), _ptr(table_base), int(table_head), seq_q_start.data_ptr(),
+        seq_q_len.data_ptr(), seq_pos_start.data_ptr(), n_seqs, max_q_len, 1 if any_short else 0, 1 if any_long else 0, n, nh, nkv,
+        hd, vd, int(window), int(keep_first), float(scale), float(softcap), _slopes(score_slopes, nh), _ptr(sinks),
+        *_head_gate(head_gate, n, nh), splits, _ptr(part), floats, status.data_ptr(), _stream()), "paged_attention_f32")
+
+
 def apply_penalties(logits, rows, tokens, counts, repetition, presence, frequency) -> None:
     _cuda(logits, rows, tokens, counts, repetition, presence, frequency)
     check(lib().fb_apply_penalties(logits.data_ptr(), _rows(logits), logits.shape[1], rows.data_ptr(),
@@ -891,6 +937,17 @@ def paged_attention(ctx, q, out, cache, nh: int, nkv: int, hd: int, window: int,
                             score_slopes=score_slopes, sinks=sinks, weights_float32=weights_float32,
                             keep_first=keep_first, table_head=cache.table_head, softcap=softcap,
                             head_gate=head_gate)
+    elif f32_attention_supported(q, out, cache.k_pool, cache.v_pool, nh, nkv, hd, vd):
+        G = nh // nkv
+        short = [G <= 16 and ql * G <= 16 for ql in b.seq_q_len]
+        # (a step of single tokens may be replayed from a CUDA graph at any context length: its stretches, and the scratch
+        # that goes with them, are sized by the longest context the engine allows, in the eager run as in the captured one)
+        longest = ctx.engine.max_seq_len if b.max_q_len == 1 else b.max_kv_len
+        paged_attention_f32(q, out, cache.k_pool, cache.v_pool, cache.block_table, b.seq_q_start_d, b.seq_q_len_d, b.seq_pos_start_d,
+                            b.n_seqs, b.max_q_len, longest, any(short), not all(short), nh, nkv, hd, window, scale,
+                            ctx.runtime.status, table_base=cache.table_base, score_slopes=score_slopes, sinks=sinks, vd=vd,
+                            keep_first=keep_first, table_head=cache.table_head, softcap=softcap, head_gate=head_gate,
+                            alloc=lambda floats: ctx.ws.alloc((floats,), torch.float32))
     else:
         paged_attention_simt(q, out, cache.k_pool, cache.v_pool, cache.block_table, b.positions, b.row_seq,
                              nh, nkv, hd, window, scale, ctx.runtime.status, table_base=cache.table_base,

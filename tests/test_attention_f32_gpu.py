@@ -1,0 +1,70 @@
+"""The tiled float32 attention against the kernel that takes a row and head at a time, over every form both accept: head and
+value sizes, groups of 1 to 64 query heads, portions beside decoded tokens, stretches of keys that are merged, windows that
+keep first keys, sinks, caps, gates as shares, slopes, a missing page, and a later token's NaN that earlier rows must not see."""
+import pytest
+import torch
+
+from test_attention_gpu import Scene
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+SIZES = [(32, 8, 128, 128), (4, 2, 24, 24), (6, 3, 40, 72), (32, 1, 64, 64), (2, 1, 256, 256), (64, 1, 20, 12), (3, 3, 4, 4), (34, 2, 128, 64)]
+SEQS = {"mixed": [(0, 1), (500, 1), (37, 70), (129, 200), (5, 4), (63, 65)], "decoding": [(900, 1), (31, 1), (32, 1)], "portion": [(0, 33)]}
+
+
+def both(sc, vd, options, poison=None, drop_page=None):
+    from flambeau_b200.kernels import ops
+    g = torch.Generator().manual_seed(3)
+    v_pool = torch.randn(*sc.k_pool.shape[:3], vd, generator=g)
+    k, v, table = sc.k_pool.nan_to_num(0.0).to(DEV), v_pool.to(DEV), sc.table.clone()
+    if poison is not None:                             # a position of the last sequence whose value is not a number
+        v[int(sc.table[-1, poison // sc.ps]), :, poison % sc.ps] = float("nan")
+    if drop_page is not None:
+        table[drop_page] = -1
+    table, q = table.to(DEV), sc.q_flat.to(DEV)
+    n = q.shape[0]
+    kw = dict(vd=vd)
+    if "window" in options:
+        kw.update(keep_first=7)
+    if "extras" in options:
+        gate = torch.randn(2, n, sc.nh + 3, generator=g).to(DEV)
+        kw.update(softcap=20.0, sinks=torch.randn(sc.nh, generator=g).to(DEV), head_gate=(gate[0][:, :sc.nh], 2, gate.stride(0)),
+                  score_slopes=(-torch.rand(sc.nh, generator=g) * 0.05).to(DEV))
+    window, scale = 50 if "window" in options else 0, 2.0 * sc.hd ** -0.5
+    outs, flags = [], []
+    lens = [m for _, m in sc.seqs]
+    G = sc.nh // sc.nkv
+    for tiled in (False, True):
+        out, status = torch.full((n, sc.nh * vd), float("nan"), device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+        if tiled:
+            short = [G <= 16 and m * G <= 16 for m in lens]
+            ops.paged_attention_f32(q, out, k, v, table, sc.seq_q_start.to(DEV), sc.seq_q_len.to(DEV), sc.seq_pos_start.to(DEV),
+                                    len(lens), max(lens), max(c + m for c, m in sc.seqs), any(short), not all(short), sc.nh, sc.nkv,
+                                    sc.hd, window, scale, status, **kw)
+        else:
+            ops.paged_attention_simt(q, out, k, v, table, sc.positions.to(DEV), sc.row_seq.to(DEV), sc.nh, sc.nkv, sc.hd, window,
+                                     scale, status, **kw)
+        outs.append(out.double().cpu())
+        flags.append(int(status.item()))
+    return outs, flags
+
+
+@pytest.mark.parametrize("options", ["plain", "window", "extras", "window extras"])
+@pytest.mark.parametrize("seqs", list(SEQS))
+@pytest.mark.parametrize("sizes", SIZES, ids=str)
+def test_tiles_equal_rows(sizes, seqs, options):
+    nh, nkv, hd, vd = sizes
+    sc = Scene(SEQS[seqs], nh, nkv, hd, 0, torch.float32, seed=hd)
+    (a, b), flags = both(sc, vd, options)
+    assert flags == [0, 0] and bool(torch.isfinite(b).all())
+    # two orders of float32 sums over at most 900 keys and 256 channels
+    assert float((a - b).abs().max() / a.abs().max()) < 5e-6
+
+
+def test_a_later_value_that_is_no_number_and_a_missing_page():
+    sc = Scene([(3, 90)], 8, 2, 64, 0, torch.float32, seed=1)
+    (a, b), _ = both(sc, 64, "plain", poison=60)
+    assert torch.equal(torch.isnan(a), torch.isnan(b)) and bool(torch.isfinite(b[:57]).all()) and bool(torch.isnan(b[57:]).all())
+    (a, b), flags = both(sc, 64, "plain", drop_page=(0, 2))
+    assert flags[0] == flags[1] != 0 and float((a - b).abs().max() / a.abs().max()) < 5e-6
