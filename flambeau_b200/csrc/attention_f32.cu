@@ -11,7 +11,8 @@
 // output, and a warp per (row, head) merges them.
 //
 // What bounds it: multiply-adds over portions (2 x 128 x 128 a row and tile of 32 keys at heads of 128; the scores read 24
-// cycles of shared memory for 64 multiply-adds of a warp), the stream of keys and values for decoded tokens.
+// cycles of shared memory for 64 multiply-adds of a warp), the stream of keys and values for decoded tokens.  301 tokens
+// behind 500 (32 heads of 128 on 8): 3,340 us with a warp a (row, head), about 140 here.
 //
 // Sums run in float32 throughout; sinks, caps, gates, slopes and kept first keys as in attention_simt.cu.
 #include <type_traits>
@@ -48,7 +49,7 @@ __device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_
 template <int LEFT> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
 
 template <int BM, int VDP>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, VDP <= 128 ? 3 : 1)
 attention_f32_kernel(const F32Args a) {
     fb_pdl_launch_dependents();
     fb_pdl_wait();
@@ -338,13 +339,13 @@ int launch(const F32Args& a, int max_q_len, cudaStream_t stream) {
 
 }  // namespace
 
-// Into how many stretches the tiles of a step are cut: as many CTAs as make four (decoded tokens, whose CTAs wait for
-// memory) or about one and a half (portions) a multiprocessor, at least two tiles each, at most 32.
+// Into how many stretches the tiles of a step are cut: as many as make four CTAs a multiprocessor, at least two tiles each,
+// at most 32.  (One CTA a multiprocessor leaves its four warps waiting on each other's loads, and CTAs that start while the
+// kernel ahead still runs then share the SMs that are free first: 301 tokens behind 500 took 560 us so.)
 FB_API int fb_attention_f32_splits(int n_seqs, int nkv, int G, int max_q_len, int max_keys) {
     const long rows = (long)max_q_len * G;
     const long ctas = (long)n_seqs * nkv * (rows <= 16 ? 1 : (max_q_len + 64 / G - 1) / (64 / G));
-    const long want = (rows <= 16 ? 4L : 1L) * fb_sm_count() + (rows <= 16 ? 0 : fb_sm_count() / 2);
-    long s = ctas > 0 ? want / ctas : 1;
+    long s = ctas > 0 ? 4L * fb_sm_count() / ctas : 1;
     const long most = max_keys / (2 * KEYS);
     if (s > most) s = most;
     if (s > MAX_SPLITS) s = MAX_SPLITS;
