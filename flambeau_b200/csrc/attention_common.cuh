@@ -8,6 +8,7 @@
 namespace fb_attn {
 
 constexpr int KT = 64;             // keys per tile
+constexpr int FB_SPLIT_COUNTERS = 1 << 16;   // arrival counters at the start of the split-key arrangement's scratch
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return smem_u32(p); }
 
@@ -74,6 +75,7 @@ struct AttnArgs {
     int kv_share;                      // split-key arrangement only: this many of the `nkv` key/value heads it is given
                                        // are one stored head (a group of more than 16 query heads is cut into
                                        // stretches that read the same cache rows); 1 as a rule
+    int k_splits, split_rows;          // tcgen05 kernel over decoded tokens: stretches of a sequence's keys, rows of a partial
     int chunk;                         // differential attention: a query sees the keys of its own chunk of positions (0: all)
     float lambda, eps, out_scale;      // what becomes of the two maps' outputs: (a_1 - lambda a_2) / rms * out_scale
     const float* row_gate;             // [rows][query heads] or nullptr: times this number
@@ -149,6 +151,9 @@ int fb_launch_attention_split(fb_attn::AttnArgs& a, int hd_max, bool tma, int n_
 // The tcgen05 arrangement for portions of prompts (attention_tc.cu): whether it takes this geometry, and its launch.
 bool fb_attention_tc_takes(const fb_attn::AttnArgs& a, bool tma);
 int fb_launch_attention_tc(const fb_attn::AttnArgs& a, int n_seqs, int max_q_len, cudaStream_t stream);
+// Decoded tokens on the tcgen05 kernel: whether it takes this geometry (a.short_rows set), and its launch (1: too little room).
+bool fb_attention_tc_split_takes(const fb_attn::AttnArgs& a, bool tma);
+int fb_launch_attention_tc_split(fb_attn::AttnArgs& a, int n_seqs, float* part, long long floats, cudaStream_t stream);
 // The same for differential attention over portions (fills in nothing: a.hd is the width of a key row, 128).
 bool fb_diff_attention_tc_takes(int nh, int nkv, int kd, int vd, int page_size, const void* out, long out_stride);
 int fb_launch_diff_attention_tc(const fb_attn::AttnArgs& a, int n_seqs, int max_q_len, cudaStream_t stream);

@@ -544,6 +544,11 @@ FB_API int fb_paged_attention_mma(const void* q, long long q_stride, void* out, 
                            : launch_long(a, HD_MAX, tma, n_seqs, max_q_len, stream);
         if (rc) return rc;
     }
+    if (any_short && attention_tc_enabled() && fb_attention_tc_split_takes(a, tma)) {
+        // (the arrival counters at the start of the scratch stay zero)
+        const int rc = fb_launch_attention_tc_split(a, n_seqs, scratch + FB_SPLIT_COUNTERS, scratch_floats - FB_SPLIT_COUNTERS, stream);
+        if (rc <= 0) return rc;
+    }
     if (any_short) {
         a.nkv = nkv * share;
         a.kv_share = share;

@@ -137,7 +137,7 @@ __host__ __device__ constexpr int split_stages(int hd_max) { return hd_max <= 12
 
 constexpr int SPLIT_SCORERS = 4;
 constexpr int SPLIT_THREADS = 32 * (SPLIT_SCORERS + 1);
-constexpr int SPLIT_COUNTERS = 1 << 16;      // arrival counters at the start of the scratch buffer
+constexpr int SPLIT_COUNTERS = FB_SPLIT_COUNTERS;
 
 __device__ __forceinline__ void scorer_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(32 * SPLIT_SCORERS) : "memory"); }
 

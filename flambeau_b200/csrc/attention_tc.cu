@@ -31,6 +31,9 @@
 // the scores and 2 x 4 x 130 for the product with both parts of the weights, which bounds it.  2,048 tokens of 32 heads of
 // 256 over one latent row: 570 us on the mma.sync kernel (7 % of the tensor pipes' rate), 153 here.
 //
+// Decoded tokens over latents (SPLIT): the rows of a sequence are fewer than a row tile, which costs a key tile no more; a CTA
+// takes a stretch of a sequence's key tiles and leaves its rows' maximum, sum and unnormalised O, and a warp per row merges them.
+//
 // Differential attention (two score maps of 64 a head over values of 128): the row tiles are the two maps of the same 128
 // rows, each with its column block of Q and K and both on one V tile.  At the end the threads of both take half of the
 // columns each, read both maps' O from tensor memory and form the difference, its norm and the gate.  A key tile costs 8 x 65
@@ -59,6 +62,12 @@ __device__ __forceinline__ float fast_exp2(float x) {
     return y;
 }
 
+// Key tiles a CTA takes of a sequence that `splits` CTAs share: a stretch of fewer than four would be mostly set-up.
+__host__ __device__ __forceinline__ int split_tiles(int n_tiles, int splits) {
+    const int per = (n_tiles + splits - 1) / splits;
+    return per < 4 ? 4 : per;
+}
+
 template <int HD, int RT, bool SHARED, bool DIFF> struct TcSmem {
     static constexpr int Q_TILES = DIFF ? 1 : RT;               // (the maps' rows lie side by side in one)
     static constexpr int Q_BYTES = BM * HD * 2;                 // one row tile: [HD/64 column blocks][128 rows][128 bytes]
@@ -72,8 +81,9 @@ template <int HD, int RT, bool SHARED, bool DIFF> struct TcSmem {
 // RT row tiles of 128 rows per CTA: with two, both use every K/V tile that is fetched and the tensor pipe works for
 // one under the softmax of the other; with one, a short portion still spreads over enough CTAs.
 // HILO: the weights enter the product as two bfloat16 numbers each.  SHARED: the key rows are the values as well.
-// DIFF: differential attention; the row tiles are the two maps of the same rows.
-template <int HD, int RT, bool HILO, bool SHARED, bool DIFF>
+// DIFF: differential attention; the row tiles are the two maps of the same rows.  SPLIT: a stretch of the keys of a sequence
+// whose rows fit a row tile.
+template <int HD, int RT, bool HILO, bool SHARED, bool DIFF, bool SPLIT>
 __global__ void __launch_bounds__(tc_threads(RT), 1)
 attention_tc_kernel(const __grid_constant__ AttnArgs a) {
     fb_pdl_launch_dependents();
@@ -110,22 +120,28 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
     // ---- what this CTA has to do: query tokens [tok0, tok0 + ntok) of a sequence, one key/value head ----
     // CTAs are numbered heaviest first over the whole step: the last tokens of every sequence and head (they see
     // the most keys) get the first SMs, whatever head or sequence they belong to
-    const int pairs = a.nkv * portion_seqs(a);
-    const int rank = blockIdx.x / pairs, pair = blockIdx.x - rank * pairs;
-    const int seq = portion_seq(a, pair / a.nkv), kvh = pair % a.nkv;
-    const int q_tiles = gridDim.x / pairs;
+    const int pairs = a.nkv * (SPLIT ? a.n_seqs : portion_seqs(a));
+    const int rank = SPLIT ? 0 : blockIdx.x / pairs, pair = SPLIT ? blockIdx.x / a.k_splits : blockIdx.x - rank * pairs;
+    const int seq = SPLIT ? pair / a.nkv : portion_seq(a, pair / a.nkv), kvh = pair % a.nkv;
+    const int q_tiles = SPLIT ? 1 : gridDim.x / pairs;
     const int q_len = a.seq_q_len[seq];
-    if (q_len * G <= a.short_rows) return;                      // the split-key arrangement's
+    if ((q_len * G <= a.short_rows) != SPLIT) return;           // the other arrangement's
     const int TQ = ROWS / G;
     const int tok0 = (q_tiles - 1 - rank) * TQ;               // later tokens see more keys: start them first
     if (tok0 >= q_len) return;
     const int ntok = min(TQ, q_len - tok0);
     const int q_start = a.seq_q_start[seq], pos0 = a.seq_pos_start[seq];
-    const int rows_valid = ntok * G;                            // of the CTA's RT * 128 rows
+    const int rows_valid = ntok * G;                            // of the CTA's rows
     const int p_first = pos0 + tok0, p_last = pos0 + tok0 + ntok - 1;
     const int t_lo = fb_first_key(p_first, a.window, DIFF ? a.chunk : 0);
     const int t_hi = p_last;
-    const int k_begin = (t_lo / BN) * BN, k_end = t_hi + 1;
+    int k_begin = (t_lo / BN) * BN, k_end = t_hi + 1;
+    if constexpr (SPLIT) {                                      // this CTA's stretch
+        const int per = split_tiles((k_end - k_begin + BN - 1) / BN, a.k_splits);
+        k_begin += (int)(blockIdx.x % a.k_splits) * per * BN;
+        if (k_begin >= k_end) return;
+        k_end = min(k_end, k_begin + per * BN);
+    }
     const int n_tiles = (k_end - k_begin + BN - 1) / BN;        // both row tiles walk all of them
     const int* table = a.block_table + (size_t)seq * a.table_stride;
     const int pages_per_tile = BN / a.page_size;
@@ -136,7 +152,7 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
     // not arrive at all, and their slots hold whatever was there.  The probabilities of such keys are 0, but
     // 0 * NaN is NaN: the softmax of row tile 0 clears those rows, 128 bytes per key and column block, before it
     // lets its product start, and says so on a barrier that the thread of row tile 1's products waits for.
-    const int dead_lo_first = ((t_lo - k_begin) / a.page_size) * a.page_size;      // rows [0, dead_lo_first) of tile 0
+    const int dead_lo_first = max(0, t_lo - k_begin) / a.page_size * a.page_size;      // rows [0, dead_lo_first) of tile 0
     const int dead_hi_last = k_end - (k_begin + (n_tiles - 1) * BN);               // rows [dead_hi_last, BN) of the last tile
     auto dead_lo_of = [&](int j) { return j == 0 ? dead_lo_first : 0; };
     auto dead_hi_of = [&](int j) { return j == n_tiles - 1 ? dead_hi_last : BN; };
@@ -455,6 +471,24 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
                     *reinterpret_cast<uint4*>(dst + 8 * c) = make_uint4(w[0], w[1], w[2], w[3]);
                 }
             }
+        } else if constexpr (SPLIT) {
+            if (ok) {
+                tmem_fence_after();
+                const size_t at = (size_t)blockIdx.x * a.split_rows + r;
+                if (valid) *reinterpret_cast<float2*>(a.part_ml + 2 * at) = make_float2(m_ref, l);
+                float* po = a.part_o + at * HD;
+#pragma unroll
+                for (int c = 0; c < HD / 32; ++c) {
+                    uint32_t v[32];
+                    tmem_ld32_nowait(o_addr + (uint32_t)(c * 32), v);
+                    tmem_wait_ld();
+                    if (valid) {
+#pragma unroll
+                        for (int e = 0; e < 32; e += 4)
+                            *reinterpret_cast<uint4*>(po + c * 32 + e) = make_uint4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+                    }
+                }
+            }
         } else if (ok) {
             tmem_fence_after();
             l += sink_term(a, head, m_ref);
@@ -487,9 +521,54 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
     }
 }
 
-template <int HD, int RT, bool HILO, bool SHARED, bool DIFF = false>
+// One warp per (pair, row) of sequences whose keys were cut into stretches: their results made one.
+template <int HD>
+__global__ void __launch_bounds__(128)
+attention_tc_merge_kernel(const __grid_constant__ AttnArgs a) {
+    fb_pdl_launch_dependents();
+    fb_pdl_wait();
+    const int item = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int pair = item / a.split_rows, r = item - pair * a.split_rows, seq = pair / a.nkv, kvh = pair - seq * a.nkv;
+    if (seq >= a.n_seqs) return;
+    const int G = a.nh / a.nkv, q_len = a.seq_q_len[seq], pos0 = a.seq_pos_start[seq];
+    if (q_len * G > a.short_rows || r >= q_len * G) return;
+    const int k_begin = fb_first_key(pos0, a.window, 0) / BN * BN, n_tiles = (pos0 + q_len - k_begin + BN - 1) / BN;
+    const int per = split_tiles(n_tiles, a.k_splits), chunks = (n_tiles + per - 1) / per;
+    const size_t slot0 = ((size_t)pair * a.k_splits) * a.split_rows + r;
+    float m = -INFINITY;
+    for (int s = lane; s < chunks; s += 32) m = fmaxf(m, a.part_ml[2 * (slot0 + (size_t)s * a.split_rows)]);
+    m = fb_warp_max(m);
+    float acc[HD / 32], l = 0.0f;
+#pragma unroll
+    for (int i = 0; i < HD / 32; ++i) acc[i] = 0.0f;
+    if (m > -INFINITY) {
+#pragma unroll 4
+        for (int s = 0; s < chunks; ++s) {
+            const size_t at = slot0 + (size_t)s * a.split_rows;
+            const float2 ml = *reinterpret_cast<const float2*>(a.part_ml + 2 * at);
+            const float w = exp2f(ml.x - m);                    // 0 where a stretch saw nothing
+            l = fmaf(w, ml.y, l);
+#pragma unroll
+            for (int i = 0; i < HD / 128; ++i) {
+                const float4 v = *reinterpret_cast<const float4*>(a.part_o + at * HD + 128 * i + 4 * lane);
+                acc[4 * i] = fmaf(w, v.x, acc[4 * i]); acc[4 * i + 1] = fmaf(w, v.y, acc[4 * i + 1]);
+                acc[4 * i + 2] = fmaf(w, v.z, acc[4 * i + 2]); acc[4 * i + 3] = fmaf(w, v.w, acc[4 * i + 3]);
+            }
+        }
+    }
+    const int token = a.seq_q_start[seq] + r / G, head = kvh * G + r % G;
+    l += sink_term(a, head, m);
+    const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+    __nv_bfloat16* dst = a.out + (size_t)token * a.out_stride + (size_t)head * HD;
+#pragma unroll
+    for (int i = 0; i < HD / 128; ++i)
+        *reinterpret_cast<uint2*>(dst + 128 * i + 4 * lane) = make_uint2(pack_bf16(acc[4 * i] * inv, acc[4 * i + 1] * inv),
+                                                                         pack_bf16(acc[4 * i + 2] * inv, acc[4 * i + 3] * inv));
+}
+
+template <int HD, int RT, bool HILO, bool SHARED, bool DIFF = false, bool SPLIT = false>
 int launch_tc(const AttnArgs& a, int n_seqs, int max_q_len, cudaStream_t stream) {
-    auto kern = attention_tc_kernel<HD, RT, HILO, SHARED, DIFF>;
+    auto kern = attention_tc_kernel<HD, RT, HILO, SHARED, DIFF, SPLIT>;
     using SM = TcSmem<HD, RT, SHARED, DIFF>;
     static bool configured[FB_MAX_DEVICES] = {};
     if (fb_needs_setup(configured)) {
@@ -499,7 +578,7 @@ int launch_tc(const AttnArgs& a, int n_seqs, int max_q_len, cudaStream_t stream)
         fb_setup_done(configured);
     }
     const int TQ = (DIFF ? 1 : RT) * BM / (a.nh / a.nkv);
-    const dim3 grid(((max_q_len + TQ - 1) / TQ) * a.nkv * portion_seqs(a));
+    const dim3 grid(SPLIT ? n_seqs * a.nkv * a.k_splits : ((max_q_len + TQ - 1) / TQ) * a.nkv * portion_seqs(a));
     fb_launch_class(FB_LAUNCH_ATTENTION_TC, (kern), grid, tc_threads(RT), (size_t)SM::BYTES, stream, a);
     return fb_check_launch("attention_tc");
 }
@@ -544,4 +623,30 @@ bool fb_diff_attention_tc_takes(int nh, int nkv, int kd, int vd, int page_size, 
 
 int fb_launch_diff_attention_tc(const AttnArgs& a, int n_seqs, int max_q_len, cudaStream_t stream) {
     return launch_tc<128, 2, true, false, true>(a, n_seqs, max_q_len, stream);
+}
+
+// Decoded tokens (rows up to 16 a stretch of heads, short_rows in all) over rows of 256 that are keys and values at once.
+// Measured with 8 sequences of 8,172 rows and 32 heads: 54 us on the split-key kernel, which fetches a row four times (as key
+// and as value, for two stretches of 16 heads), 25 here with the merge.
+bool fb_attention_tc_split_takes(const AttnArgs& a, bool tma) { return a.hd == 256 && fb_attention_tc_takes(a, tma) && a.short_rows <= BM; }
+
+// part: room for partial results, `floats` of them; 1 where it does not do (nothing was launched).
+int fb_launch_attention_tc_split(AttnArgs& a, int n_seqs, float* part, long long floats, cudaStream_t stream) {
+    const long pairs = (long)n_seqs * a.nkv;
+    a.split_rows = a.short_rows;
+    const long long each = pairs * a.split_rows * (a.hd + 2);
+    // One CTA a multiprocessor while the pairs leave room for more than four stretches each; else four, so that sequences of
+    // different lengths spread.
+    long splits = fb_sm_count() / pairs;
+    if (splits < 4) splits = 4;
+    if (splits > floats / each) splits = (long)(floats / each);
+    if (splits < 1) return 1;
+    a.k_splits = (int)splits;
+    a.part_o = part;
+    a.part_ml = part + splits * pairs * a.split_rows * a.hd;
+    const int rc = a.weights_hi_lo ? launch_tc<256, 1, true, true, false, true>(a, n_seqs, 1, stream)
+                                   : launch_tc<256, 1, false, true, false, true>(a, n_seqs, 1, stream);
+    if (rc) return rc;
+    fb_launch((attention_tc_merge_kernel<256>), dim3((unsigned)((pairs * a.split_rows + 3) / 4)), dim3(128), 0, stream, a);
+    return fb_check_launch("attention_tc_merge");
 }

@@ -1,6 +1,6 @@
 """Portions of prompts on the tcgen05 attention kernel with softmax weights of two bfloat16 numbers each, and over cache rows
 that are keys and values at once, against a softmax in float64: heads of 64, 128 and 256, one to 64 query heads a key/value
-head, portions around the edges of row tiles and key tiles, windows that cut a page, pages of 8 to 64 keys, sinks, poison in
+head, portions around the edges of row tiles and key tiles, decoded tokens whose keys are cut into stretches, windows that cut a page, pages of 8 to 64 keys, sinks, poison in
 every slot that was not written."""
 import pytest
 import torch
@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 # (query heads, key/value heads, head size, values are the keys)
 GEOMETRY = [(32, 1, 256, True), (3, 1, 256, True), (8, 2, 256, True), (64, 1, 256, True), (8, 2, 128, False), (4, 4, 64, False), (20, 2, 128, False)]
-SEQS = [[(0, 129), (37, 70)], [(100, 333)], [(5, 64), (200, 1), (63, 65)]]
+SEQS = [[(0, 129), (37, 70)], [(100, 333)], [(5, 64), (200, 1), (63, 65)], [(1500, 1), (64, 1), (0, 1), (319, 1), (62, 2)], [(127, 1)] * 60]
 
 
 def softmax_over_pages(sc, sinks, scale):
