@@ -73,7 +73,7 @@ _SIGNATURES = {
     # moe.cu
     "fb_moe_choose": (I, [P, L, I, L, P, I, I, I, I, I, P, P, P, I, F, I, I, I, STREAM]),
     "fb_moe_max_tiles": (I, [I, I, I]),
-    "fb_moe_gather_rows": (I, [P, L, I, P, P, I, I, P, P, STREAM]),
+    "fb_moe_gather_rows": (I, [P, L, I, P, P, I, I, P, P, P, I, STREAM]),
     "fb_moe_sort": (I, [P, I, I, I, I, I, P, P, P, P, STREAM]),
     "fb_moe_combine": (I, [P, L, P, P, I, P, I, L, P, P, I, I, P, I, L, I, STREAM]),
     # layer_norm.cu

@@ -694,10 +694,13 @@ def grouped_tile(pairs: int, groups: int, tensor_cores: bool) -> int:
     return 64
 
 
-def gather_rows(h: torch.Tensor, place_token: torch.Tensor, out: torch.Tensor, share=None, place_pair=None) -> None:
+def gather_rows(h: torch.Tensor, place_token: torch.Tensor, out: torch.Tensor, share=None, place_pair=None, tile_group=None,
+                tile: int = 0) -> None:
     """out[i] = h[place_token[i]], zeros where place_token[i] < 0.  With share (float32, one per (token, choice) pair)
-    and place_pair (the pair of every place): out[i] = share[place_pair[i]] * h[place_token[i]]."""
-    _cuda(h, place_token, out, share, place_pair)
+    and place_pair (the pair of every place): out[i] = share[place_pair[i]] * h[place_token[i]].  With tile_group (the group
+    of every `tile` rows): rows of tiles without a group (negative), which a grouped product skips, may stay as they are."""
+    _cuda(h, place_token, out, share, place_pair, tile_group)
+    _i32(tile_group, "tile_group")
     _i32(place_token, "place_token")
     _i32(place_pair, "place_pair")
     if (share is None) != (place_pair is None) or (share is not None and share.dtype != torch.float32):
@@ -706,7 +709,7 @@ def gather_rows(h: torch.Tensor, place_token: torch.Tensor, out: torch.Tensor, s
     if h.dtype != out.dtype or h.shape[1] != D or not out.is_contiguous() or place_token.numel() < rows:
         raise KernelError("gather_rows: shapes or dtypes do not agree")
     check(lib().fb_moe_gather_rows(h.data_ptr(), _rows(h), dtype_code(h), place_token.data_ptr(), out.data_ptr(), rows,
-                                   D, _ptr(share), _ptr(place_pair), _stream()), "moe_gather_rows")
+                                   D, _ptr(share), _ptr(place_pair), _ptr(tile_group), int(tile), _stream()), "moe_gather_rows")
 
 
 def gemm_tc_grouped(a: torch.Tensor, w: torch.Tensor, tile_group: torch.Tensor, tile: int, out: torch.Tensor,
@@ -751,7 +754,7 @@ def grouped_gated_linear(a: torch.Tensor, row_index, w: torch.Tensor, tile_group
             side = a
             if row_index is not None:
                 side = ctx.ws.alloc((out.shape[0], a.shape[1]), a.dtype)
-                gather_rows(a, row_index, side, row_share, row_pair)
+                gather_rows(a, row_index, side, row_share, row_pair, tile_group, tile)
             gemm_tc_grouped_gated(side, w, tile_group, tile, out, ctx.runtime.status, activation)
         return
     if tile not in (16, 64):
@@ -776,7 +779,7 @@ def grouped_linear(a: torch.Tensor, row_index, w: torch.Tensor, tile_group: torc
         if row_index is not None:
             with ctx.ws.scope():
                 side = ctx.ws.alloc((out.shape[0], a.shape[1]), a.dtype)
-                gather_rows(a, row_index, side, row_share, row_pair)
+                gather_rows(a, row_index, side, row_share, row_pair, tile_group, tile)
                 gemm_tc_grouped(side, w, tile_group, tile, out, ctx.runtime.status, activation_name)
         else:
             gemm_tc_grouped(a, w, tile_group, tile, out, ctx.runtime.status, activation_name)
