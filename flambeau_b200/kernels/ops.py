@@ -945,12 +945,13 @@ def paged_attention(ctx, q, out, cache, nh: int, nkv: int, hd: int, window: int,
         short = [G <= 16 and ql * G <= 16 for ql in b.seq_q_len]
         # (a step of single tokens may be replayed from a CUDA graph at any context length: its stretches, and the scratch
         # that goes with them, are sized by the longest context the engine allows, in the eager run as in the captured one)
-        longest = ctx.engine.max_seq_len if b.max_q_len == 1 else b.max_kv_len
+        longest = ctx.engine.max_seq_len if b.max_q_len == 1 and hasattr(ctx, "engine") else b.max_kv_len
+        ws = getattr(ctx, "ws", None)        # (a context without a scratch arena: fresh tensors)
         paged_attention_f32(q, out, cache.k_pool, cache.v_pool, cache.block_table, b.seq_q_start_d, b.seq_q_len_d, b.seq_pos_start_d,
                             b.n_seqs, b.max_q_len, longest, any(short), not all(short), nh, nkv, hd, window, scale,
                             ctx.runtime.status, table_base=cache.table_base, score_slopes=score_slopes, sinks=sinks, vd=vd,
                             keep_first=keep_first, table_head=cache.table_head, softcap=softcap, head_gate=head_gate,
-                            alloc=lambda floats: ctx.ws.alloc((floats,), torch.float32))
+                            alloc=(lambda floats: ws.alloc((floats,), torch.float32)) if ws is not None else None)
     else:
         paged_attention_simt(q, out, cache.k_pool, cache.v_pool, cache.block_table, b.positions, b.row_seq,
                              nh, nkv, hd, window, scale, ctx.runtime.status, table_base=cache.table_base,
