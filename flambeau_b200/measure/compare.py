@@ -58,7 +58,7 @@ def configs(size: dict, layers: int):
     return {"zedivik": z, "mistral": m}
 
 
-ATTENTION = ("paged_attention_mma", "diff_attention_mma", "paged_attention_simt", "diff_attention_simt")
+ATTENTION = ("paged_attention_mma", "diff_attention_mma", "paged_attention_f32", "paged_attention_simt", "diff_attention_simt")
 CLASS_OF = {"paged_attention_mma": "attention", "diff_attention_mma": "attention", "rope_kv_write": "cache_write",
             "qkv_bias_cache_write": "cache_write", "add_rms_norm": "norm", "norm_add_rms_norm": "norm",
             "gate_mul": "gate_mul", "embedding": "embedding", "rope_table": "rope_table", "sample": "sample",

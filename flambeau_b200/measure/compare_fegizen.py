@@ -49,7 +49,7 @@ SIZES = {
     "7b": dict(NODEPEL_SIZES["7b"], dim=128, rot_dim=64, vdim=128, kv_rank=192, q_rank=1536, taps=4, identity=2, tau=16.0),
 }
 
-CLASS_OF = {"paged_attention_mma": "attention", "paged_attention_simt": "attention",
+CLASS_OF = {"paged_attention_mma": "attention", "paged_attention_f32": "attention", "paged_attention_simt": "attention",
             "qk_norm_rope_kv_write": "cache_write", "mla_latents": "cache_write",
             "add_rms_norm": "norm", "add_layer_norm": "norm", "gate_mul": "gate_mul",
             "gdr_prepare": "recurrence_prepare", "gla_prepare": "recurrence_prepare",

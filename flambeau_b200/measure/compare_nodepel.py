@@ -39,8 +39,8 @@ SIZES = {
                r_heads=32, r_qk_heads=8, r_dk=128, r_dv=128, conv=4, experts=64, top=6, expert_ff=1792, shared_ff=3584),
 }
 
-CLASS_OF = {"paged_attention_mma": "attention", "paged_attention_simt": "attention", "rope_kv_write": "cache_write",
-            "qk_norm_rope_kv_write": "cache_write", "add_rms_norm": "norm", "gate_mul": "gate_mul",
+CLASS_OF = {"paged_attention_mma": "attention", "paged_attention_f32": "attention", "paged_attention_simt": "attention",
+            "rope_kv_write": "cache_write", "qk_norm_rope_kv_write": "cache_write", "add_rms_norm": "norm", "gate_mul": "gate_mul",
             "gdr_prepare": "recurrence_prepare", "gdr_recurrent": "recurrence", "gdr_out_norm": "recurrence_out",
             "branch_norm_mix": "branch_mix", "moe_choose": "router", "moe_sort": "expert_order",
             "moe_gather_rows": "expert_gather", "moe_combine": "expert_combine", "activation": "activation",

@@ -159,7 +159,7 @@ def classify(cfg, what: str, note) -> str:
                  (2 * s["I"], s["H"]): "gate_up_proj", (s["H"], s["I"]): "down_proj", (s["V"], s["H"]): "lm_head"}
         return names.get(matrix, what)
     return {"add_rms_norm": "add_norm", "rope_kv_write": "rotary_cache_write", "paged_attention_mma": "attention",
-            "paged_attention_simt": "attention"}.get(what, what)
+            "paged_attention_f32": "attention", "paged_attention_simt": "attention"}.get(what, what)
 
 
 class Sections(dict):

@@ -5,6 +5,10 @@ import pytest
 from flambeau_b200.config.mistral import MistralConfig
 from flambeau_b200.measure import work
 from flambeau_b200.measure.shapes import SHAPES, shape
+from flambeau_b200.measure.compare import ATTENTION
+from flambeau_b200.measure.compare_fegizen import CLASS_OF as fegizen_classes
+from flambeau_b200.measure.compare_nodepel import CLASS_OF as nodepel_classes
+from flambeau_b200.measure.compare_tubepel import CLASS_OF as tubepel_classes
 from flambeau_b200.measure.workloads import classify
 
 
@@ -47,7 +51,10 @@ def test_launcher_calls_fold_into_classes():
     assert classify(cfg, "gemm_tc", (8, 5120, 14336)) == "down_proj"
     assert classify(cfg, "gemm_tc", (8, 131072, 5120)) == "lm_head"
     assert classify(cfg, "add_rms_norm", None) == "add_norm"
-    assert classify(cfg, "paged_attention_mma", None) == "attention"
+    for name in ("paged_attention_mma", "paged_attention_f32", "paged_attention_simt"):
+        assert classify(cfg, name, None) == "attention"
+        assert all(classes[name] == "attention" for classes in (fegizen_classes, nodepel_classes, tubepel_classes))
+        assert name in ATTENTION
     classes = work.kernel_classes(cfg, 8, [4096] * 8)
     assert classes["attention"]["bytes"] >= 8 * 4096 * 2 * 1024 * 2
     portion = work.kernel_classes(cfg, 2048, [2048])
