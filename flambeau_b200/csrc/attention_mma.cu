@@ -441,15 +441,15 @@ int launch_long(const AttnArgs& a, int hd_max, bool tma, int n_seqs, int max_q_l
 
 int g_attention_tc = -1;           // -1: not decided yet (the environment decides), 0: off, 1: on
 
-bool attention_tc_enabled() {
+}  // namespace
+
+bool fb_attention_tc_enabled() {
     if (g_attention_tc < 0) {
         const char* env = getenv("FLAMBEAU_ATTN_TC");
         g_attention_tc = (env && env[0] == '0') ? 0 : 1;
     }
     return g_attention_tc == 1;
 }
-
-}  // namespace
 
 // Into how many equal stretches of at most 16 heads a group of nh / nkv query heads is cut for the split-key
 // arrangement: 1 up to 16 heads, else the smallest divisor of the group that leaves at most 16.
@@ -461,8 +461,8 @@ FB_API int fb_attention_kv_share(int nh, int nkv) {
     return G;
 }
 
-// Portions of prompts run on the tcgen05 kernel where it takes the geometry (1, the default) or always on the
-// mma.sync kernel (0).
+// Portions of prompts (those of differential attention too) and decoded tokens over latents run on the tcgen05 kernel
+// where it takes the geometry (1, the default) or always on the mma.sync kernels (0).
 FB_API void fb_set_attention_tc(int on) { g_attention_tc = on ? 1 : 0; }
 
 // q, out: bfloat16 [rows, heads*hd]; pools bfloat16 [pages][kv heads][page size][hd].
@@ -539,12 +539,12 @@ FB_API int fb_paged_attention_mma(const void* q, long long q_stride, void* out, 
     a.prefetch = fb_make_prefetch(prefetch_base, prefetch_rows, prefetch_row_stride, prefetch_bytes_per_row);
     a.part_o = nullptr; a.part_ml = nullptr; a.part_cnt = nullptr;
     if (any_long) {
-        const int rc = (attention_tc_enabled() && fb_attention_tc_takes(a, tma))
+        const int rc = (fb_attention_tc_enabled() && fb_attention_tc_takes(a, tma))
                            ? fb_launch_attention_tc(a, n_seqs, max_q_len, stream)
                            : launch_long(a, HD_MAX, tma, n_seqs, max_q_len, stream);
         if (rc) return rc;
     }
-    if (any_short && attention_tc_enabled() && fb_attention_tc_split_takes(a, tma)) {
+    if (any_short && fb_attention_tc_enabled() && fb_attention_tc_split_takes(a, tma)) {
         // (the arrival counters at the start of the scratch stay zero)
         const int rc = fb_launch_attention_tc_split(a, n_seqs, scratch + FB_SPLIT_COUNTERS, scratch_floats - FB_SPLIT_COUNTERS, stream);
         if (rc <= 0) return rc;

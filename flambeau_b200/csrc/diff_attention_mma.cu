@@ -6,8 +6,8 @@
 // rows of a CTA share every K/V tile it fetches, so grouped heads cost no second read of the cache.  A warp owns 16
 // rows of ONE map; the warps of map 1 and the warps of map 2 of the same rows sit in one CTA and meet at the end.
 //
-// Portions with maps of 64 over values of 128 run on the tcgen05 kernel (attention_tc.cu).  Else two arrangements of one
-// kernel:
+// Portions with maps of 64 over values of 128 run on the tcgen05 kernel (attention_tc.cu) unless that is switched off.
+// Else two arrangements of one kernel:
 //   portions  (rows of the sequence > short_rows): a CTA owns 64 rows (4 warps per map), walks the 64-key tiles its
 //             rows can see, every warp scoring the whole tile for its 16 rows (32 keys at a time), and ends with the epilogue
 //             (a1 - lambda a2, head norm, gate) through shared memory.
@@ -585,7 +585,7 @@ FB_API int fb_diff_attention_mma(const void* q, long long q_stride, void* out, l
     a.part_o = nullptr; a.part_ml = nullptr;
     a.status = status;
     const int HG = nh / nkv;
-    if (any_long && fb_diff_attention_tc_takes(nh, nkv, kd, vd, page_size, out, (long)out_stride)) {
+    if (any_long && fb_attention_tc_enabled() && fb_diff_attention_tc_takes(nh, nkv, kd, vd, page_size, out, (long)out_stride)) {
         AttnArgs t = {};
         const long pool_rows = (long)n_pages * nkv * page_size;
         int rc = fb_tensor_map_bf16(&t.map_k, k_pool, pool_rows, 2 * kd, 2 * kd, 64, page_size);

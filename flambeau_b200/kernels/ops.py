@@ -853,8 +853,8 @@ def set_gemm_pair(on: bool) -> None:
 
 
 def set_attention_tc(on: bool) -> None:
-    """Portions of prompts on the tcgen05 attention kernel where it takes the geometry (the default), or always on
-    the mma.sync kernel."""
+    """Portions of prompts (those of differential attention too) and decoded tokens over latents on the tcgen05
+    attention kernel where it takes the geometry (the default), or always on the mma.sync kernels."""
     lib().fb_set_attention_tc(1 if on else 0)
 
 

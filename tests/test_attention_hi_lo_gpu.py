@@ -1,11 +1,12 @@
 """Portions of prompts on the tcgen05 attention kernel with softmax weights of two bfloat16 numbers each, and over cache rows
 that are keys and values at once, against a softmax in float64: heads of 64, 128 and 256, one to 64 query heads a key/value
-head, portions around the edges of row tiles and key tiles, decoded tokens whose keys are cut into stretches, windows that cut a page, pages of 8 to 64 keys, sinks, poison in
-every slot that was not written."""
+head, portions around the edges of row tiles and key tiles, decoded tokens whose keys are cut into stretches, windows that
+cut a page, pages of 8 to 64 keys, sinks, poison in every slot that was not written; on the tcgen05 kernel and with it
+switched off."""
 import pytest
 import torch
 
-from test_attention_gpu import Scene
+from test_attention_gpu import Scene, prompt_kernel  # noqa: F401  (a fixture)
 
 pytestmark = pytest.mark.gpu
 
@@ -33,7 +34,7 @@ def softmax_over_pages(sc, sinks, scale):
 @pytest.mark.parametrize("seqs", SEQS, ids=str)
 @pytest.mark.parametrize("window,page", [(0, 16), (50, 16), (0, 8), (97, 64)])
 @pytest.mark.parametrize("geometry", GEOMETRY, ids=str)
-def test_portions_with_weights_in_two_parts(geometry, window, page, seqs):
+def test_portions_with_weights_in_two_parts(prompt_kernel, geometry, window, page, seqs):
     from flambeau_b200.kernels import ops
     nh, nkv, hd, shared = geometry
     sc = Scene(seqs, nh, nkv, hd, window, torch.bfloat16, page_size=page, seed=hd + window, compact=True)

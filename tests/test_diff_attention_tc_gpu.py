@@ -1,5 +1,5 @@
-"""Differential attention over portions with maps of 64 and values of 128, the sizes of the tcgen05 kernel: one to 32 query
-heads a key/value head, portions around the edges of its 128 rows and 64-key tiles, windows, pages of 8 to 64 keys, with and
+"""Differential attention over portions with maps of 64 and values of 128, the sizes of the tcgen05 kernel, on that kernel and
+with it switched off (the mma.sync kernel): one to 32 query heads a key/value head, portions around the edges of its 128 rows and 64-key tiles, windows, pages of 8 to 64 keys, with and
 without a gate per head; planted keys at the windows' edges, poison in every slot that was not written."""
 import pytest
 import torch
@@ -12,22 +12,49 @@ pytestmark = pytest.mark.gpu
 SEQS = [(0, 130), (70, 64), (37, 33), (200, 1), (129, 200), (5, 17)]
 
 
+@pytest.fixture(params=[True, False], ids=["tcgen05", "mma_sync"])
+def portion_kernel(request):
+    from flambeau_b200.kernels import ops
+    ops.set_attention_tc(request.param)
+    yield request.param
+    ops.set_attention_tc(True)
+
+
+def portions(case, gate, out_scale, nh, nkv, window, scale, lam, eps):
+    from flambeau_b200.kernels import ops
+    out = torch.full((case.n, nh * 128), float("nan"), dtype=torch.bfloat16, device="cuda:0")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda:0")
+    ops.diff_attention_mma(case.q_d, out, gate, case.cache, case.seq_q_start, case.seq_q_len, case.seq_pos_start, len(SEQS),
+                           case.max_q_len, case.max_kv_len, case.any_short, case.any_long, nh, nkv, 64, 128, window, scale, lam,
+                           eps, out_scale, status)
+    assert int(status.item()) == 0 and bool(torch.isfinite(out.float()).all())
+    return out
+
+
 @pytest.mark.parametrize("geometry", [(8, 2, 0, 16), (4, 4, 33, 16), (12, 1, 100, 64), (32, 1, 40, 8), (3, 1, 64, 32)], ids=str)
 @pytest.mark.parametrize("gated", [True, False])
-def test_portions_of_two_maps(geometry, gated):
-    from flambeau_b200.kernels import ops
+def test_portions_of_two_maps(portion_kernel, geometry, gated):
     nh, nkv, window, page = geometry
     case = zt.PagedCase(SEQS, nh=nh, nkv=nkv, kd=64, vd=128, window=window, page_size=page, dtype=torch.bfloat16, device="cuda:0",
                         seed=nh + window)
     scale, lam, diff, eps = 0.3, 0.62, 0.35, 1e-5
-    out = torch.full((case.n, nh * 128), float("nan"), dtype=torch.bfloat16, device="cuda:0")
-    status = torch.zeros(1, dtype=torch.int32, device="cuda:0")
-    gate = case.gate_d if gated else None
-    ops.diff_attention_mma(case.q_d, out, gate, case.cache, case.seq_q_start, case.seq_q_len, case.seq_pos_start, len(SEQS),
-                           case.max_q_len, case.max_kv_len, case.any_short, case.any_long, nh, nkv, 64, 128, window, scale, lam,
-                           eps, 1.0 - diff, status)
+    out = portions(case, case.gate_d if gated else None, 1.0 - diff, nh, nkv, window, scale, lam, eps)
     want = case.expected(scale=scale, lam=lam, diff=diff, eps=eps)
     if not gated:
         want = (want.view(case.n, nh, 128) / case.gate_d.double().cpu()[:, :, None]).view(case.n, -1)
-    assert int(status.item()) == 0 and bool(torch.isfinite(out.float()).all())
     assert rel_err(out, want) < 8e-3                   # the tolerance of the other arrangements' tests
+
+
+def test_the_switch_reaches_differential_portions():
+    """The two kernels move their reference points at other keys, so some of 800,000 roundings differ; the same bits would
+    mean that both runs took one kernel."""
+    from flambeau_b200.kernels import ops
+    case = zt.PagedCase(SEQS, nh=16, nkv=4, kd=64, vd=128, window=0, page_size=16, dtype=torch.bfloat16, device="cuda:0", seed=5)
+    outs = []
+    for on in (True, False):
+        ops.set_attention_tc(on)
+        try:
+            outs.append(portions(case, None, 0.65, 16, 4, 0, 0.125, 0.62, 1e-5))
+        finally:
+            ops.set_attention_tc(True)
+    assert not torch.equal(*outs)

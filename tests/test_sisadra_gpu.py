@@ -167,7 +167,7 @@ CHUNKED = [(4, 2, 16, 48, 20, 16), (6, 1, 16, 32, 33, 16), (8, 2, 48, 64, 100, 1
 
 @pytest.mark.parametrize("geometry", CHUNKED, ids=lambda g: "h%d.%d-k%d-v%d-c%d-p%d" % g)
 @pytest.mark.parametrize("window", [0, 23])
-@pytest.mark.parametrize("kernel", ["simt-float32", "simt-bfloat16", "mma-bfloat16"])
+@pytest.mark.parametrize("kernel", ["simt-float32", "simt-bfloat16", "mma-bfloat16", "mma_sync-bfloat16"])
 def test_differential_attention_within_chunks(geometry, window, kernel):
     """First tokens, positions at the ends of chunks, decoded tokens far into a request and at page borders, portions that
     cross a chunk's edge or several, portions of two tokens on either side of it; pages of chunks that were left are given
@@ -206,13 +206,17 @@ def test_differential_attention_within_chunks(geometry, window, kernel):
     lens = [n for _, n in seqs]
     q_d = torch.cat([q.reshape(q.shape[0], -1) for q in qs]).to(dt).to(DEV)
     out, status = torch.full((sum(lens), nh * vd), float("nan"), dtype=dt, device=DEV), i32([0])
-    if which == "mma":
+    if which != "simt":
         if not ops.diff_attention_mma_supported(q_d, nh, nkv, kd, vd):
             pytest.skip("sizes the tensor-core arrangements do not take run on the float32-math kernel")
+        if which == "mma_sync" and (kd, vd) != (64, 128):
+            pytest.skip("sizes the tcgen05 kernel does not take run on the mma.sync kernel anyhow")
+        ops.set_attention_tc(which == "mma")
         short = [n * (nh // nkv) <= 16 for n in lens]
         ops.diff_attention_mma(q_d, out, None, cache, i32([sum(lens[:i]) for i in range(len(lens))]), i32(lens),
                                i32([c for c, _ in seqs]), len(seqs), max(lens), max(c + n for c, n in seqs), any(short),
                                not all(short), nh, nkv, kd, vd, window, scale, lam, eps, 1.0 - diff, status, chunk=chunk)
+        ops.set_attention_tc(True)
     else:
         ops.diff_attention_simt(q_d, out, None, cache, i32([p for c, n in seqs for p in range(c, c + n)]),
                                 i32([s for s, n in enumerate(lens) for _ in range(n)]), nh, nkv, kd, vd, window, scale, lam, eps,
