@@ -10,9 +10,9 @@
 //                  buffers per row tile: the scores run two key tiles ahead of the softmax;
 //   softmax        one thread per row (the row = its tensor-memory lane): the row's 64 scores in one tcgen05.ld
 //                  round trip, base-2 online softmax in float32, P rounded to bfloat16 and stored with tcgen05.st
-//                  over the scores it came from; where the caller wants 16 bits of mantissa, what the rounding left is
-//                  stored behind it as bfloat16 again (two numbers a weight fill the columns that one score had), and
-//                  the product runs over both;
+//                  over the scores it came from; where the caller wants more bits of mantissa, what the rounding left is
+//                  stored as one or two bfloat16 numbers more (two fill the columns that one score had), and the
+//                  product runs over all;
 //   O += P V       tcgen05.mma with P read from tensor memory and V as it lies in the cache ([key][dim], the
 //                  MN-major operand); O in tensor memory.
 //
@@ -54,7 +54,23 @@ constexpr int BN = 64;             // keys per tile
 __host__ __device__ constexpr int tc_threads(int rt) { return 128 + BM * rt; }
 constexpr int NKV = 4;             // K slots and V slots
 constexpr int TMEM_COLS = 512;     // S/P buffer b of row tile t at (2t + b) * 64; O of row tile t at RT * 128 + t * 128
-constexpr float RESCALE_STEP = 8.0f;
+
+// Softmax weights of more than one bfloat16 number (HILO) are three, 24 bits of mantissa, where tensor memory has 32 columns
+// more a buffer: behind everything else, at heads of 64 behind O.  Two row tiles at heads of 128 fill it: there they are two,
+// and the reference point of the exponentials follows a row's maximum at every step, so that the largest weight is 1 and
+// loses nothing in two parts, as on the mma.sync kernels.  (A reference that lags leaves that weight up to 2^8, rounded to 16
+// bits as the others are.  Results that are not the rounding of the exact ones, uneven weights: over latents 0.19 % so, 0.14
+// with three parts, 0.16 on the mma.sync kernel; decoded tokens 0.16, 0.06 and 0.08; two maps 0.22, at every step 0.17, 0.17.
+// The third part costs up to 4 % of a layer, a reference that follows at every step 5 to 40 % over latents, whose O is 256
+// columns, and up to 6 % with two maps.)
+template <int HD, int RT, bool HILO> struct Weights {
+    static constexpr int PARTS = !HILO ? 1 : HD == 128 && RT == 2 ? 2 : 3;
+    static constexpr float RESCALE_STEP = PARTS == 2 ? 0.0f : 8.0f;         // how far (base 2) a maximum may pass the reference
+    __device__ static constexpr int third(int t, int b) {                   // the columns of the third parts
+        return HD == 64 ? RT * 128 + t * 128 + 64 + b * (BN / 2) : RT * 128 + RT * HD + (2 * t + b) * (BN / 2);
+    }
+    static_assert(PARTS < 3 || HD == 64 || RT * 128 + RT * HD + RT * BN <= TMEM_COLS, "tensor memory");
+};
 
 __device__ __forceinline__ float fast_exp2(float x) {
     float y;
@@ -80,7 +96,7 @@ template <int HD, int RT, bool SHARED, bool DIFF> struct TcSmem {
 
 // RT row tiles of 128 rows per CTA: with two, both use every K/V tile that is fetched and the tensor pipe works for
 // one under the softmax of the other; with one, a short portion still spreads over enough CTAs.
-// HILO: the weights enter the product as two bfloat16 numbers each.  SHARED: the key rows are the values as well.
+// HILO: the weights enter the product as two or three bfloat16 numbers each (Weights).  SHARED: the key rows are the values as well.
 // DIFF: differential attention; the row tiles are the two maps of the same rows.  SPLIT: a stretch of the keys of a sequence
 // whose rows fit a row tile.
 template <int HD, int RT, bool HILO, bool SHARED, bool DIFF, bool SPLIT>
@@ -92,6 +108,7 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
     using SM = TcSmem<HD, RT, SHARED, DIFF>;
     constexpr int ROWS = DIFF ? BM : RT * BM;                   // query rows of the CTA
     constexpr int CB = HD / 64;                                 // 64-column blocks of a head
+    using W = Weights<HD, RT, HILO>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
@@ -300,6 +317,7 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
                     const uint64_t db = umma_desc_mn(v_addr + (uint32_t)(kk * 16 * 128), BN * 128, 1024);
                     umma_bf16_ts(d, p_addr + (uint32_t)(kk * 8), db, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
                     if (HILO) umma_bf16_ts(d, p_addr + (uint32_t)(BN / 2 + kk * 8), db, idesc_o, 1u);
+                    if (W::PARTS == 3) umma_bf16_ts(d, tmem_base + (uint32_t)(W::third(t, j & 1) + kk * 8), db, idesc_o, 1u);
                 }
                 if (more) issue_s(j + 2);
                 umma_commit(smem_u32(&pv_done[t]));
@@ -371,7 +389,7 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
             const float m_new = fmaxf(m_ref, fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * a.scale_log2e);
             if (j == 0) {
                 m_ref = m_new;                                  // O is overwritten by the first product
-            } else if (__any_sync(0xffffffffu, m_new > m_ref + RESCALE_STEP || (m_ref == -INFINITY && m_new > m_ref))) {
+            } else if (__any_sync(0xffffffffu, m_new > m_ref + W::RESCALE_STEP || (m_ref == -INFINITY && m_new > m_ref))) {
                 // move the reference point: O *= 2^(old - new), for the whole warp at once.  (The product of tile
                 // j - 2 is complete, that of tile j cannot start before this thread is through: the phase asked
                 // for is the current one or the one just completed.)
@@ -398,7 +416,7 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
             float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
             for (int c = 0; c < BN / 32; ++c) {
-                uint32_t pk[16], rest[16];
+                uint32_t pk[16], rest[16], third[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     // a masked score is -inf: 2^-inf = 0
@@ -406,10 +424,15 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
                     const float p1 = fast_exp2(fmaf(__uint_as_float(v[c][2 * i + 1]), a.scale_log2e, neg_ref));
                     sum4[i & 3] += p0 + p1;
                     pk[i] = pack_bf16(p0, p1);
-                    if (HILO) rest[i] = pack_bf16_remainder(p0, p1);
+                    if (HILO) {
+                        const float r0 = p0 - bf16_low(pk[i]), r1 = p1 - bf16_high(pk[i]);
+                        rest[i] = pack_bf16(r0, r1);
+                        if (W::PARTS == 3) third[i] = pack_bf16(r0 - bf16_low(rest[i]), r1 - bf16_high(rest[i]));
+                    }
                 }
                 tmem_st16(s_addr + (uint32_t)(c * 16), pk);
                 if (HILO) tmem_st16(s_addr + (uint32_t)(BN / 2 + c * 16), rest);
+                if (W::PARTS == 3) tmem_st16(lane_addr + (uint32_t)(W::third(t, j & 1) + c * 16), third);
             }
             l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
             if (t == 0 && has_dead(j)) {                        // (only the first and the last tile can)

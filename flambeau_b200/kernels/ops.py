@@ -878,10 +878,10 @@ def paged_attention_mma(q, out, k_pool, v_pool, block_table, seq_q_start, seq_q_
     these instead of over every sequence.  score_slopes (float32 per query head, optional): slope * (key position -
     query position) is added to every scaled score; portions then run on the mma.sync kernel.  sinks (float32 per
     query head, optional): one more softmax slot per head, its score that number unscaled, without key or value.
-    weights_float32: the softmax weights enter P V as two bfloat16 numbers each (the rounded weight and what the
-    rounding left: 16 bits of mantissa, two MMAs for one) instead of rounded to bfloat16.  keep_first: under a window, the keys at positions below this
-    stay visible to every later query (their tiles are walked ahead of the window's; portions then run on the
-    mma.sync kernel).  softcap > 0: scores are softcap * tanh(scale * q.k / softcap); head_gate (see _head_gate): every
+    weights_float32: the softmax weights enter P V as two or three bfloat16 numbers each (the rounded weight and what the
+    rounding left: 16 bits of mantissa or more, as many MMAs) instead of rounded to bfloat16.  keep_first: under a
+    window, the keys at positions below this stay visible to every later query (their tiles are walked ahead of the
+    window's; portions then run on the mma.sync kernel).  softcap > 0: scores are softcap * tanh(scale * q.k / softcap); head_gate (see _head_gate): every
     head's output is multiplied by sigmoid of its number (portions run on the mma.sync kernel with either)."""
     _cuda(q, out, k_pool, v_pool, block_table, seq_q_start, seq_q_len, seq_pos_start, status, table_base, multi_seqs,
           sinks)

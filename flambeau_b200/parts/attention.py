@@ -37,8 +37,8 @@ class PagedAttention(Mixer):
     num_heads * value_dim columns.
     `sink` (bool): the softmax of every head has one more slot, a learned score per head (`<prefix><names.sink>`,
     [num_heads]) that is not scaled, has no key and no value, and counts once in the denominator.
-    `weights_float32`: the softmax weights keep 16 bits of mantissa through the product with the values when serving
-    in bfloat16 (two bfloat16 numbers a weight, two MMAs for one; the 32-bit mode has them in float32 anyway), for
+    `weights_float32`: the softmax weights keep 16 bits of mantissa or more through the product with the values when serving
+    in bfloat16 (two or three bfloat16 numbers a weight, as many MMAs; the 32-bit mode has them in float32 anyway), for
     designs that say their attention weights are 32-bit numbers; otherwise they are rounded to bfloat16 for that
     product, as flash attention kernels do.
     `keep_first` (with a window): the keys at positions below this stay visible to every later query, each with the

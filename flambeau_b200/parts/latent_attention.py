@@ -31,7 +31,7 @@ class LatentAttention(Mixer):
     The position part turns the rotated part of a head: it hands out its tables (`half`, `prepare`) and says which
     dimensions form a pair (`pairing`: neighbours (2i, 2i + 1) or halves (i, i + half)).
     Rotation angles, both RMS norms, scores and softmax weights are float32 in both engine modes; the weights enter
-    the product with the latents as two bfloat16 numbers each when serving.
+    the product with the latents as two or three bfloat16 numbers each when serving.
 
     Tensors behind the prefix: dq, dq.norm, uq (or q), dkv, dkv.norm, uk, uv, g (with `gate`), sink (with `sink`), o."""
     graph_safe = True

@@ -58,3 +58,41 @@ def test_the_switch_reaches_differential_portions():
         finally:
             ops.set_attention_tc(True)
     assert not torch.equal(*outs)
+
+
+def exact(case, scale, lam, diff, eps):
+    """The difference of the two maps' outputs, normed, in float64 on the GPU; no gate, no window."""
+    rows = []
+    for s, (ctx, n) in enumerate(case.seqs):
+        q, k, v = (t[s].cuda() for t in (case.q, case.k, case.v))
+        seen = torch.arange(ctx + n, device="cuda")[None] <= torch.arange(ctx, ctx + n, device="cuda")[:, None]
+        o = torch.empty(n, case.nh, case.vd, dtype=torch.float64, device="cuda")
+        for h in range(case.nh):
+            g = h // (case.nh // case.nkv)
+            a = [torch.softmax(((q[:, h, m] @ k[:, g, m].T) * scale).masked_fill(~seen, float("-inf")), -1) @ v[:, g] for m in (0, 1)]
+            d = a[0] - lam * a[1]
+            o[:, h] = d / torch.sqrt((d * d).mean(-1, keepdim=True) + eps) * (1.0 - diff)
+        rows.append(o.reshape(n, -1))
+    return torch.cat(rows)
+
+
+def test_weights_lose_no_more_than_on_the_mma_sync_kernel():
+    """Uneven weights: how many results are not the rounding of the exact ones.  Every weight's own error makes some results
+    cross a border between two bfloat16 numbers; the largest weight of a row, which counts most, has none where it is 1."""
+    from flambeau_b200.kernels import ops
+    case = zt.PagedCase([(300, 700)], nh=16, nkv=4, kd=64, vd=128, window=0, page_size=16, dtype=torch.bfloat16, device="cuda:0",
+                        seed=4, plant=False)
+    want, wrong = exact(case, 0.3, 0.62, 0.35, 1e-5).float().bfloat16(), []
+    for on in (True, False):
+        ops.set_attention_tc(on)
+        try:
+            out = torch.empty((case.n, 16 * 128), dtype=torch.bfloat16, device="cuda:0")
+            status = torch.zeros(1, dtype=torch.int32, device="cuda:0")
+            ops.diff_attention_mma(case.q_d, out, None, case.cache, case.seq_q_start, case.seq_q_len, case.seq_pos_start, 1,
+                                   case.max_q_len, case.max_kv_len, False, True, 16, 4, 64, 128, 0, 0.3, 0.62, 1e-5, 0.65, status)
+            assert int(status.item()) == 0
+            wrong.append(int((out != want).sum()))
+        finally:
+            ops.set_attention_tc(True)
+    # (counts of rare events: three standard deviations of their difference)
+    assert wrong[0] <= wrong[1] + 3.0 * sum(wrong) ** 0.5, wrong
