@@ -159,7 +159,7 @@ bool fb_attention_tc_takes(const fb_attn::AttnArgs& a, bool tma);
 int fb_launch_attention_tc(const fb_attn::AttnArgs& a, int n_seqs, int max_q_len, cudaStream_t stream);
 // Decoded tokens on the tcgen05 kernel: whether it takes this geometry (a.short_rows set), and its launch (1: too little room).
 bool fb_attention_tc_split_takes(const fb_attn::AttnArgs& a, bool tma);
-int fb_launch_attention_tc_split(fb_attn::AttnArgs& a, int n_seqs, float* part, long long floats, cudaStream_t stream);
+int fb_launch_attention_tc_split(fb_attn::AttnArgs& a, int n_seqs, int max_kv_len, float* part, long long floats, cudaStream_t stream);
 // The same for differential attention over portions (fills in nothing: a.hd is the width of a key row, 128).
 bool fb_diff_attention_tc_takes(int nh, int nkv, int kd, int vd, int page_size, const void* out, long out_stride);
 int fb_launch_diff_attention_tc(const fb_attn::AttnArgs& a, int n_seqs, int max_q_len, cudaStream_t stream);

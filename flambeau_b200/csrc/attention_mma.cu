@@ -546,7 +546,8 @@ FB_API int fb_paged_attention_mma(const void* q, long long q_stride, void* out, 
     }
     if (any_short && fb_attention_tc_enabled() && fb_attention_tc_split_takes(a, tma)) {
         // (the arrival counters at the start of the scratch stay zero)
-        const int rc = fb_launch_attention_tc_split(a, n_seqs, scratch + FB_SPLIT_COUNTERS, scratch_floats - FB_SPLIT_COUNTERS, stream);
+        const int rc = fb_launch_attention_tc_split(a, n_seqs, max_kv_len, scratch + FB_SPLIT_COUNTERS,
+                                                    scratch_floats - FB_SPLIT_COUNTERS, stream);
         if (rc <= 0) return rc;
     }
     if (any_short) {

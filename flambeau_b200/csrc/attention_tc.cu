@@ -650,19 +650,35 @@ int fb_launch_diff_attention_tc(const AttnArgs& a, int n_seqs, int max_q_len, cu
 
 // Decoded tokens (rows up to 16 a stretch of heads, short_rows in all) over rows of 256 that are keys and values at once.
 // Measured with 8 sequences of 8,172 rows and 32 heads: 54 us on the split-key kernel, which fetches a row four times (as key
-// and as value, for two stretches of 16 heads), 25 here with the merge.
+// and as value, for two stretches of 16 heads), 25 here with the merge.  A layer of 1 to 64 sequences of 60 to 8,000 rows takes
+// 0.58 to 0.99 of the time with 32 heads and 0.71 to 1.00 with 16; no size was found where the split-key kernel is faster.
 bool fb_attention_tc_split_takes(const AttnArgs& a, bool tma) { return a.hd == 256 && fb_attention_tc_takes(a, tma) && a.short_rows <= BM; }
 
+// Into how many stretches the keys of a sequence are cut, at most `most`: the count whose rounds of CTAs (one a
+// multiprocessor) times the tiles of a stretch are fewest, three tiles counted for a CTA's set-up and end; at least three
+// stretches where there are tiles for them, so that sequences of different lengths spread.  38 sequences of 8,000 rows, 16
+// heads, a layer: four stretches are 152 CTAs and a second round for four of them, 158 us; seven take 125, the
+// split-key kernel 136.
+FB_API int fb_attention_tc_stretches(long long pairs, int tiles, int most, int sms) {
+    int best = 0;
+    long long best_cost = 0;
+    for (int s = 1; s <= most && s <= 64; ++s) {
+        const int per = split_tiles(tiles, s), there = (tiles + per - 1) / per;
+        if (there < s) continue;                       // (more stretches than the tiles make)
+        if (s < 3 && s < most && split_tiles(tiles, s + 1) < per) continue;
+        const long long cost = (pairs * s + sms - 1) / sms * (per + 3);
+        if (best == 0 || cost < best_cost) { best = s; best_cost = cost; }
+    }
+    return best > 0 ? best : most >= 1 ? 1 : 0;
+}
+
 // part: room for partial results, `floats` of them; 1 where it does not do (nothing was launched).
-int fb_launch_attention_tc_split(AttnArgs& a, int n_seqs, float* part, long long floats, cudaStream_t stream) {
+int fb_launch_attention_tc_split(AttnArgs& a, int n_seqs, int max_kv_len, float* part, long long floats, cudaStream_t stream) {
     const long pairs = (long)n_seqs * a.nkv;
     a.split_rows = a.short_rows;
-    const long long each = pairs * a.split_rows * (a.hd + 2);
-    // One CTA a multiprocessor while the pairs leave room for more than four stretches each; else four, so that sequences of
-    // different lengths spread.
-    long splits = fb_sm_count() / pairs;
-    if (splits < 4) splits = 4;
-    if (splits > floats / each) splits = (long)(floats / each);
+    const long long each = pairs * a.split_rows * (a.hd + 2), most = floats / each;
+    const int keys = a.window > 0 ? min(max_kv_len, a.window + BM) : max_kv_len;
+    const long splits = fb_attention_tc_stretches(pairs, (keys + BN - 1) / BN, (int)(most < 64 ? most : 64), fb_sm_count());
     if (splits < 1) return 1;
     a.k_splits = (int)splits;
     a.part_o = part;

@@ -56,6 +56,8 @@ _SIGNATURES = {
     "fb_gemm_tc_gated": (I, [P, L, P, L, P, I, L, I, I, I, I, F, F, P, L, P, I, P, STREAM]),
     # attention_simt.cu
     "fb_paged_attention_simt": (I, [P, L, P, L, I, P, P, I, I, P, I, P, I, P, P, I, I, I, I, I, I, I, F, F, P, P, P, L, I, L, P, STREAM]),
+    # attention_tc.cu
+    "fb_attention_tc_stretches": (I, [L, I, I, I]),
     # attention_f32.cu
     "fb_attention_f32_splits": (I, [I, I, I, I, I]),
     "fb_paged_attention_f32": (I, [P, L, P, L, P, P, I, I, P, I, P, I, P, P, P, I, I, I, I, I, I, I, I, I, I, I, F, F, P, P, P, L, I, L, I, P,
