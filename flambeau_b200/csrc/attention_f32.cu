@@ -165,6 +165,7 @@ attention_f32_kernel(const F32Args a) {
         const int t0 = tile_start(it) + tx, t1 = t0 + 16;
         const bool there0 = has_page[(it & 1) * KEYS + tx], there1 = has_page[(it & 1) * KEYS + tx + 16];
         float p[RPT][2];
+        bool see[RPT][2];
         bool whole_tile = there0 && there1;                      // every row of this warp sees every key of the tile
 #pragma unroll
         for (int i = 0; i < RPT; ++i) {
@@ -176,17 +177,17 @@ attention_f32_kernel(const F32Args a) {
             }
             x += slope[i] * (float)(t0 - p_row[i]);
             y += slope[i] * (float)(t1 - p_row[i]);
-            const bool see0 = there0 && t0 <= p_row[i] && (t0 >= t0_row[i] || t0 < keep);
-            const bool see1 = there1 && t1 <= p_row[i] && (t1 >= t0_row[i] || t1 < keep);
-            x = see0 ? x : -INFINITY;
-            y = see1 ? y : -INFINITY;
+            see[i][0] = there0 && t0 <= p_row[i] && (t0 >= t0_row[i] || t0 < keep);
+            see[i][1] = there1 && t1 <= p_row[i] && (t1 >= t0_row[i] || t1 < keep);
+            x = see[i][0] ? x : -INFINITY;
+            y = see[i][1] ? y : -INFINITY;
             float top = fmaxf(x, y);
 #pragma unroll
             for (int off = 8; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
             const float m_new = fmaxf(m[i], top), m_use = m_new == -INFINITY ? 0.0f : m_new;
             const float corr = m[i] == -INFINITY ? 0.0f : expf(m[i] - m_use);
-            p[i][0] = see0 ? expf(x - m_use) : 0.0f;
-            p[i][1] = see1 ? expf(y - m_use) : 0.0f;
+            p[i][0] = see[i][0] ? expf(x - m_use) : 0.0f;
+            p[i][1] = see[i][1] ? expf(y - m_use) : 0.0f;
             l[i] = l[i] * corr + (p[i][0] + p[i][1]);            // (this lane's keys; the lanes' sums meet at the end)
             m[i] = m_new;
 #pragma unroll
@@ -195,8 +196,8 @@ attention_f32_kernel(const F32Args a) {
         whole_tile = __all_sync(0xffffffffu, whole_tile);
 #pragma unroll
         for (int i = 0; i < RPT; ++i) {
-            Ps[tx * (BM + 4) + ty * RPT + i] = p[i][0];
-            Ps[(tx + 16) * (BM + 4) + ty * RPT + i] = p[i][1];
+            Ps[tx * (BM + 4) + ty * RPT + i] = see[i][0] ? p[i][0] : -1.0f;     // (below zero: a key that the row does not see)
+            Ps[(tx + 16) * (BM + 4) + ty * RPT + i] = see[i][1] ? p[i][1] : -1.0f;
         }
         __syncthreads();                                         // the weights are there, K is free
         if (it < last_tile) fetch_k(it + 1, next_page);
@@ -223,7 +224,8 @@ attention_f32_kernel(const F32Args a) {
                 const float4 v = *reinterpret_cast<const float4*>(vr + k * VDP + 64 * c);
 #pragma unroll
                 for (int i = 0; i < RPT; ++i) {
-                    if (!whole && w[i] == 0.0f) continue;        // (what a row does not see must not reach it as 0 * NaN)
+                    if (!whole && w[i] < 0.0f) continue;         // (what a row does not see must not reach it as 0 * NaN; what it
+                                                                 // sees does, also with a weight that has become 0)
                     o[i][4 * c] = fmaf(w[i], v.x, o[i][4 * c]);
                     o[i][4 * c + 1] = fmaf(w[i], v.y, o[i][4 * c + 1]);
                     o[i][4 * c + 2] = fmaf(w[i], v.z, o[i][4 * c + 2]);

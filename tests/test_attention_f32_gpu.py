@@ -13,7 +13,7 @@ SIZES = [(32, 8, 128, 128), (4, 2, 24, 24), (6, 3, 40, 72), (32, 1, 64, 64), (2,
 SEQS = {"mixed": [(0, 1), (500, 1), (37, 70), (129, 200), (5, 4), (63, 65)], "decoding": [(900, 1), (31, 1), (32, 1)], "portion": [(0, 33)]}
 
 
-def both(sc, vd, options, poison=None, drop_page=None):
+def both(sc, vd, options, poison=None, drop_page=None, slope=None):
     from flambeau_b200.kernels import ops
     g = torch.Generator().manual_seed(3)
     v_pool = torch.randn(*sc.k_pool.shape[:3], vd, generator=g)
@@ -31,6 +31,8 @@ def both(sc, vd, options, poison=None, drop_page=None):
         gate = torch.randn(2, n, sc.nh + 3, generator=g).to(DEV)
         kw.update(softcap=20.0, sinks=torch.randn(sc.nh, generator=g).to(DEV), head_gate=(gate[0][:, :sc.nh], 2, gate.stride(0)),
                   score_slopes=(-torch.rand(sc.nh, generator=g) * 0.05).to(DEV))
+    if slope is not None:
+        kw.update(score_slopes=torch.full((sc.nh,), slope, device=DEV))
     window, scale = 50 if "window" in options else 0, 2.0 * sc.hd ** -0.5
     outs, flags = [], []
     lens = [m for _, m in sc.seqs]
@@ -68,3 +70,11 @@ def test_a_later_value_that_is_no_number_and_a_missing_page():
     assert torch.equal(torch.isnan(a), torch.isnan(b)) and bool(torch.isfinite(b[:57]).all()) and bool(torch.isnan(b[57:]).all())
     (a, b), flags = both(sc, 64, "plain", drop_page=(0, 2))
     assert flags[0] == flags[1] != 0 and float((a - b).abs().max() / a.abs().max()) < 5e-6
+
+
+def test_a_seen_value_that_is_no_number_reaches_every_row_that_sees_it():
+    """Scores fall by 20 a position, so most rows weigh the key at position 10 by exactly 0; it is seen all the same, in tiles
+    that a row sees whole and in those it does not."""
+    sc = Scene([(3, 90)], 8, 2, 64, 0, torch.float32, seed=2)
+    (a, b), _ = both(sc, 64, "plain", poison=10, slope=-20.0)
+    assert torch.equal(torch.isnan(a), torch.isnan(b)) and bool(torch.isfinite(b[:7]).all()) and bool(torch.isnan(b[7:]).all())
