@@ -36,6 +36,7 @@ struct F32Args {
     float scale, softcap;
     const float* score_slopes; const float* sinks;
     const float* head_gate; long gate_stride; int gate_partials; long gate_partial_stride;
+    int token_tiles;                    // CTAs that the tokens of a (sequence, key/value head) are laid over
     int short_rows;                     // sequences with at most this many rows (tokens x G) run with BM 16
     int n_splits;
     float* part_o; float* part_ml;      // [split][row][head] x vd, and x (maximum, sum)
@@ -56,11 +57,12 @@ attention_f32_kernel(const F32Args a) {
     constexpr int RPT = BM / 8, NC = VDP / 64;                   // rows and groups of four columns a thread
     extern __shared__ __align__(16) float sh[];
     const int G = a.nh / a.nkv, hd = a.hd, vd = a.vd;
-    const int seq = blockIdx.y / a.nkv, kvh = blockIdx.y - seq * a.nkv;
+    const int pair = blockIdx.x / a.token_tiles, tile = blockIdx.x - pair * a.token_tiles;
+    const int seq = pair / a.nkv, kvh = pair - seq * a.nkv;
     const int q_len = a.seq_q_len[seq];
     if ((q_len * G <= a.short_rows) != (BM == 16)) return;
     const int TQ = BM / G;
-    const int tok0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * TQ;      // later tokens see more keys: start them first
+    const int tok0 = (a.token_tiles - 1 - tile) * TQ;      // later tokens see more keys: start them first
     if (tok0 >= q_len) return;
     const int ntok = min(TQ, q_len - tok0), rows = ntok * G;
     const int q_start = a.seq_q_start[seq] + tok0, pos0 = a.seq_pos_start[seq] + tok0;
@@ -317,7 +319,7 @@ size_t smem_bytes(int bm, int hd, int vdp) {
 }
 
 template <int BM, int VDP>
-int launch(const F32Args& a, int max_q_len, cudaStream_t stream) {
+int launch(F32Args a, int max_q_len, cudaStream_t stream) {
     auto kern = attention_f32_kernel<BM, VDP>;
     static bool configured[FB_MAX_DEVICES] = {};
     if (fb_needs_setup(configured)) {
@@ -328,7 +330,8 @@ int launch(const F32Args& a, int max_q_len, cudaStream_t stream) {
     }
     const int TQ = BM / (a.nh / a.nkv);
     const int longest = BM == 16 ? min(max_q_len, TQ) : max_q_len;     // (a sequence with BM 16 is one tile)
-    fb_launch(kern, dim3((longest + TQ - 1) / TQ, a.n_seqs * a.nkv, a.n_splits), dim3(THREADS), smem_bytes(BM, a.hd, VDP), stream, a);
+    a.token_tiles = (longest + TQ - 1) / TQ;
+    fb_launch(kern, dim3((unsigned)((long)a.token_tiles * a.n_seqs * a.nkv), 1, a.n_splits), dim3(THREADS), smem_bytes(BM, a.hd, VDP), stream, a);
     return fb_check_launch("attention_f32");
 }
 
@@ -370,7 +373,7 @@ FB_API int fb_paged_attention_f32(const float* q, long long q_stride, float* out
                (uintptr_t)k_pool % 16 == 0 && (uintptr_t)v_pool % 16 == 0, "attention_f32: unaligned operands");
     FB_REQUIRE(page_size > 0 && n_pages > 0 && window >= 0 && keep_first >= 0, "attention_f32: bad cache geometry");
     FB_REQUIRE(softcap >= 0.0f && (!head_gate || gate_stride >= nh), "attention_f32: bad cap or gate");
-    FB_REQUIRE((long long)n_seqs * nkv <= 65535, "attention_f32: too many sequences or heads for one grid");
+    FB_REQUIRE((long long)n_seqs * nkv * max_q_len < (1LL << 31), "attention_f32: too many sequences and tokens for one grid");
     if (n == 0 || n_seqs == 0) return 0;
     if (n_splits < 1) n_splits = 1;
     if (n_splits > MAX_SPLITS) n_splits = MAX_SPLITS;

@@ -940,7 +940,7 @@ def paged_attention(ctx, q, out, cache, nh: int, nkv: int, hd: int, window: int,
                             score_slopes=score_slopes, sinks=sinks, weights_float32=weights_float32,
                             keep_first=keep_first, table_head=cache.table_head, softcap=softcap,
                             head_gate=head_gate)
-    elif f32_attention_supported(q, out, cache.k_pool, cache.v_pool, nh, nkv, hd, vd):
+    elif f32_attention_supported(q, out, cache.k_pool, cache.v_pool, nh, nkv, hd, vd) and b.n_seqs * nkv * b.max_q_len < 1 << 31:
         G = nh // nkv
         short = [G <= 16 and ql * G <= 16 for ql in b.seq_q_len]
         # (a step of single tokens may be replayed from a CUDA graph at any context length: its stretches, and the scratch

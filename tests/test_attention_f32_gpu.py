@@ -78,3 +78,15 @@ def test_a_seen_value_that_is_no_number_reaches_every_row_that_sees_it():
     sc = Scene([(3, 90)], 8, 2, 64, 0, torch.float32, seed=2)
     (a, b), _ = both(sc, 64, "plain", poison=10, slope=-20.0)
     assert torch.equal(torch.isnan(a), torch.isnan(b)) and bool(torch.isfinite(b[:7]).all()) and bool(torch.isnan(b[7:]).all())
+
+
+def test_more_sequences_times_heads_than_a_grid_has_rows():
+    """33,000 decoded tokens of two key/value heads (three sequences over and over); the row-wise kernel takes them in one
+    launch."""
+    sc, n = Scene([(0, 1), (5, 1), (2, 1)], 2, 2, 4, 0, torch.float32, seed=3, page_size=4), 33000
+    sc.seqs, sc.table = sc.seqs * (n // 3), sc.table.repeat(n // 3, 1)
+    sc.positions, sc.seq_pos_start, sc.seq_q_len = (t.repeat(n // 3) for t in (sc.positions, sc.seq_pos_start, sc.seq_q_len))
+    sc.row_seq = sc.seq_q_start = torch.arange(n, dtype=torch.int32)
+    sc.q_flat = torch.randn(n, sc.nh * sc.hd, generator=torch.Generator().manual_seed(4))
+    (a, b), flags = both(sc, 4, "plain")
+    assert flags == [0, 0] and float((a - b).abs().max() / a.abs().max()) < 5e-6
