@@ -1,14 +1,17 @@
 // Paged causal (sliding-window) attention in float32 on the CUDA cores, in tiles: the attention of the true 32-bit path for
 // head sizes that are multiples of 4 up to 256 (attention_simt.cu takes every other size and the bfloat16 forms).
 //
-// A CTA of 128 threads owns one key/value head, BM query rows = (BM / G) tokens x the G query heads that share the head, and a
-// stretch of the 32-key tiles that its rows see.  K and V tiles come through the block table by 16-byte asynchronous copies, V
+// A CTA of 128 threads owns one key/value head, BM query rows = (BM / G) tokens x the G query heads that share the head, and
+// some of the 32-key tiles that its rows see.  K and V tiles come through the block table by 16-byte asynchronous copies, V
 // under the scores and the next K under the product.  Thread (ty, tx) of 8 x 16 holds rows ty * BM / 8 and following: their
 // scores of keys tx and tx + 16, then their output columns 4 tx + 64 c; so a row's maximum and sum are agreed on by 16 lanes
 // and its rescaling needs no memory.  Rows up to 16 (decoded tokens) run with BM 16, others with BM 64, in two launches.
 //
-// Where that gives too few CTAs the tiles are cut into stretches: every CTA leaves its rows' maximum, sum and unnormalised
-// output, and a warp per (row, head) merges them.
+// A row's bits depend on its position and its keys alone, not on the rows that share its step, on how its prompt was cut, or on
+// how the work was laid over CTAs: tiles begin at multiples of 32 positions, stretches of tiles at multiples of 256, a stretch
+// is summed on its own, and the stretches are joined in their order by one rule (join).  A CTA that takes all stretches of its
+// rows joins them in its output rows; where that gives too few CTAs each takes some, leaves every stretch's maximum, sum and
+// unnormalised output, and a warp per row joins them.
 //
 // What bounds it: multiply-adds over portions (2 x 128 x 128 a row and tile of 32 keys at heads of 128; the scores read 24
 // cycles of shared memory for 64 multiply-adds of a warp), the stream of keys and values for decoded tokens.  301 tokens
@@ -23,7 +26,9 @@ namespace {
 
 constexpr int THREADS = 128;
 constexpr int KEYS = 32;                // keys of a tile
-constexpr int MAX_SPLITS = 32;
+constexpr int STRETCH = 256;            // keys of a stretch: joined on their own, whoever takes them
+constexpr int TPS = STRETCH / KEYS;
+constexpr long long SCRATCH_FLOATS = 1LL << 25;      // most that stretches of one launch may leave for joining
 
 struct F32Args {
     const float* q; long q_stride;
@@ -38,10 +43,44 @@ struct F32Args {
     const float* head_gate; long gate_stride; int gate_partials; long gate_partial_stride;
     int token_tiles;                    // CTAs that the tokens of a (sequence, key/value head) are laid over
     int short_rows;                     // sequences with at most this many rows (tokens x G) run with BM 16
-    int n_splits;
-    float* part_o; float* part_ml;      // [split][row][head] x vd, and x (maximum, sum)
+    int slots, per;                     // stretches that a row's keys have at most, and that a CTA takes
+    int part_rows;                      // rows of a pair in the parts of BM 16
+    float* part_o; float* part_ml;      // per stretch and row: output x vd, and (maximum, sum); nullptr: a CTA takes all
     int* status;
 };
+
+// What a stretch (maximum m, sum l) adds to the stretches before it (M, L): the factors of the output so far and of its own.
+struct Join { float before, own; };
+__device__ __forceinline__ Join join(float& M, float& L, float m, float l) {
+    const float top = fmaxf(M, m);
+    Join j;
+    j.before = M == -INFINITY ? 0.0f : expf(M - top);
+    j.own = m == -INFINITY ? 0.0f : expf(m - top);
+    L = fmaf(L, j.before, __fmul_rn(l, j.own));
+    M = top;
+    return j;
+}
+__device__ __forceinline__ float joined(const Join& j, float before, float own) { return fmaf(before, j.before, __fmul_rn(own, j.own)); }
+
+// What a row's joined output is multiplied with in the end.
+__device__ __forceinline__ float finish(const F32Args& a, int row, int head, float M, float L) {
+    float f = 1.0f, sum = L;
+    if (a.sinks) {                                               // the slot without key and value
+        const float sk = a.sinks[head], top = fmaxf(M, sk);
+        f = M == -INFINITY ? 0.0f : expf(M - top);
+        sum = fmaf(sum, f, expf(sk - top));
+    }
+    f = sum > 0.0f ? f / sum : 0.0f;
+    if (a.head_gate)
+        f /= 1.0f + expf(-fb_slab_sum(a.head_gate + (size_t)row * a.gate_stride, head, a.gate_partials, a.gate_partial_stride));
+    return f;
+}
+
+// Row r of a CTA, in the parts of a stretch.
+template <int BM>
+__device__ __forceinline__ size_t part_at(const F32Args& a, int slot, int pair, int row, int head, int r) {
+    return BM == 16 ? ((size_t)slot * a.n_seqs * a.nkv + pair) * a.part_rows + r : ((size_t)slot * a.n + row) * a.nh + head;
+}
 
 __device__ __forceinline__ void copy16(float* dst, const float* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
@@ -50,7 +89,7 @@ __device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_
 template <int LEFT> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
 
 template <int BM, int VDP>
-__global__ void __launch_bounds__(THREADS, VDP <= 128 ? 3 : 1)
+__global__ void __launch_bounds__(THREADS, VDP == 64 ? 3 : VDP == 128 ? 2 : 1)
 attention_f32_kernel(const F32Args a) {
     fb_pdl_launch_dependents();
     fb_pdl_wait();
@@ -72,15 +111,26 @@ attention_f32_kernel(const F32Args a) {
     float* Ks = Qs + BM * LQ;                                    // [KEYS][LQ]
     float* Vs = Ks + KEYS * LQ;                                  // [KEYS][VDP]
     float* Ps = Vs + KEYS * VDP;                                 // [KEYS][BM + 4]: the weights, key by key
-    int* has_page = reinterpret_cast<int*>(Ps + KEYS * (BM + 4));      // [2][KEYS]
+    float* run = Ps + KEYS * (BM + 4);                           // [2][2][BM]: maxima and sums of the stretches joined so far,
+                                                                 // read from one half and left in the other
+    int* has_page = reinterpret_cast<int*>(run + 4 * BM);        // [2][KEYS]
 
     // ---- the tiles: those that hold kept first keys and lie before the window's first, then the window's ----
     const int t_hi = pos0 + ntok - 1, t_lo = fb_first_key(pos0, a.window, 0);
     const int keep = a.window > 0 ? a.keep_first : 0;
     const int tile_lo = t_lo / KEYS * KEYS, head_tiles = min((keep + KEYS - 1) / KEYS, t_lo / KEYS);
     const int n_tiles = head_tiles + (t_hi - tile_lo) / KEYS + 1;
-    const int per = (n_tiles + a.n_splits - 1) / a.n_splits;
-    const int first_tile = blockIdx.z * per, last_tile = min(first_tile + per, n_tiles) - 1;
+    // ---- its stretches, numbered from the first that holds a tile ----
+    const int head_last = (head_tiles - 1) / TPS, window_first = tile_lo / STRETCH;
+    const int shift = (head_tiles > 0 ? head_last + (window_first > head_last) : 0) - window_first;
+    auto tile_of = [&](int s) {                                  // the first tile of stretch s
+        if (s >= a.slots) return n_tiles;
+        if (head_tiles > 0 && s <= head_last) return s * TPS;
+        return min(n_tiles, head_tiles + max(0, (s - shift) * TPS - tile_lo / KEYS));
+    };
+    const int slot_end = min((int)(blockIdx.z + 1) * a.per, a.slots);
+    int slot = blockIdx.z * a.per, stretch_end = tile_of(slot + 1);
+    const int first_tile = tile_of(slot), last_tile = tile_of(slot_end) - 1;
     auto tile_start = [&](int i) { return i < head_tiles ? i * KEYS : tile_lo + (i - head_tiles) * KEYS; };
 
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
@@ -167,7 +217,6 @@ attention_f32_kernel(const F32Args a) {
         const int t0 = tile_start(it) + tx, t1 = t0 + 16;
         const bool there0 = has_page[(it & 1) * KEYS + tx], there1 = has_page[(it & 1) * KEYS + tx + 16];
         float p[RPT][2];
-        bool see[RPT][2];
         bool whole_tile = there0 && there1;                      // every row of this warp sees every key of the tile
 #pragma unroll
         for (int i = 0; i < RPT; ++i) {
@@ -179,18 +228,19 @@ attention_f32_kernel(const F32Args a) {
             }
             x += slope[i] * (float)(t0 - p_row[i]);
             y += slope[i] * (float)(t1 - p_row[i]);
-            see[i][0] = there0 && t0 <= p_row[i] && (t0 >= t0_row[i] || t0 < keep);
-            see[i][1] = there1 && t1 <= p_row[i] && (t1 >= t0_row[i] || t1 < keep);
-            x = see[i][0] ? x : -INFINITY;
-            y = see[i][1] ? y : -INFINITY;
+            const bool see0 = there0 && t0 <= p_row[i] && (t0 >= t0_row[i] || t0 < keep);
+            const bool see1 = there1 && t1 <= p_row[i] && (t1 >= t0_row[i] || t1 < keep);
+            x = see0 ? x : -INFINITY;
+            y = see1 ? y : -INFINITY;
             float top = fmaxf(x, y);
 #pragma unroll
             for (int off = 8; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
             const float m_new = fmaxf(m[i], top), m_use = m_new == -INFINITY ? 0.0f : m_new;
             const float corr = m[i] == -INFINITY ? 0.0f : expf(m[i] - m_use);
-            p[i][0] = see[i][0] ? expf(x - m_use) : 0.0f;
-            p[i][1] = see[i][1] ? expf(y - m_use) : 0.0f;
-            l[i] = l[i] * corr + (p[i][0] + p[i][1]);            // (this lane's keys; the lanes' sums meet at the end)
+            const float px = see0 ? expf(x - m_use) : 0.0f, py = see1 ? expf(y - m_use) : 0.0f;
+            l[i] = l[i] * corr + (px + py);                      // (this lane's keys; the lanes' sums meet at the end)
+            p[i][0] = see0 ? px : -1.0f;                         // (below zero: a key that the row does not see)
+            p[i][1] = see1 ? py : -1.0f;
             m[i] = m_new;
 #pragma unroll
             for (int c = 0; c < 4 * NC; ++c) o[i][c] *= corr;
@@ -198,8 +248,8 @@ attention_f32_kernel(const F32Args a) {
         whole_tile = __all_sync(0xffffffffu, whole_tile);
 #pragma unroll
         for (int i = 0; i < RPT; ++i) {
-            Ps[tx * (BM + 4) + ty * RPT + i] = see[i][0] ? p[i][0] : -1.0f;     // (below zero: a key that the row does not see)
-            Ps[(tx + 16) * (BM + 4) + ty * RPT + i] = see[i][1] ? p[i][1] : -1.0f;
+            Ps[tx * (BM + 4) + ty * RPT + i] = p[i][0];
+            Ps[(tx + 16) * (BM + 4) + ty * RPT + i] = p[i][1];
         }
         __syncthreads();                                         // the weights are there, K is free
         if (it < last_tile) fetch_k(it + 1, next_page);
@@ -243,79 +293,99 @@ attention_f32_kernel(const F32Args a) {
             for (int k = 0; k < KEYS; ++k) weigh(std::false_type(), k);
         page = next_page;
         next_page = page2;
-        __syncthreads();                                         // V and the weights are free
-    }
+        if (it + 1 == stretch_end || it == last_tile) {          // the stretch is complete
+            const bool first = slot == 0;
+            const float* run_in = run + (slot & 1) * 2 * BM;
+            float* run_out = run + (~slot & 1) * 2 * BM;
 #pragma unroll
-    for (int i = 0; i < RPT; ++i) {
+            for (int i = 0; i < RPT; ++i) {
 #pragma unroll
-        for (int off = 8; off > 0; off >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], off);
-        const int r = ty * RPT + i;
-        if (r >= rows) continue;
-        const int row = q_start + r / G, head = kvh * G + r % G;
-        if (a.n_splits > 1) {
-            const size_t at = ((size_t)blockIdx.z * a.n + row) * a.nh + head;
-            if (tx == 0) {
-                a.part_ml[2 * at] = m[i];
-                a.part_ml[2 * at + 1] = l[i];
+                for (int off = 8; off > 0; off >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], off);
+                const int r = ty * RPT + i;
+                if (r >= rows) continue;
+                const int row = q_start + r / G, head = kvh * G + r % G;
+                if (a.part_o) {
+                    const size_t at = part_at<BM>(a, slot, pair, row, head, r);
+                    if (tx == 0) *reinterpret_cast<float2*>(a.part_ml + 2 * at) = make_float2(m[i], l[i]);
+#pragma unroll
+                    for (int c = 0; c < NC; ++c)
+                        if (4 * tx + 64 * c < vd)
+                            *reinterpret_cast<float4*>(a.part_o + at * vd + 4 * tx + 64 * c) = make_float4(o[i][4 * c], o[i][4 * c + 1], o[i][4 * c + 2], o[i][4 * c + 3]);
+                    continue;
+                }
+                float M = first ? -INFINITY : run_in[r], L = first ? 0.0f : run_in[BM + r];
+                const Join j = join(M, L, m[i], l[i]);
+                const float f = it == last_tile ? finish(a, row, head, M, L) : 1.0f;
+                if (tx == 0) {
+                    run_out[r] = M;
+                    run_out[BM + r] = L;
+                }
+                float* op = a.out + (size_t)row * a.out_stride + (size_t)head * vd + 4 * tx;     // (read by the thread that wrote it)
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+                    if (4 * tx + 64 * c < vd) {
+                        const float4 b = first ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(op + 64 * c);
+                        *reinterpret_cast<float4*>(op + 64 * c) = make_float4(joined(j, b.x, o[i][4 * c]) * f, joined(j, b.y, o[i][4 * c + 1]) * f,
+                                                                              joined(j, b.z, o[i][4 * c + 2]) * f, joined(j, b.w, o[i][4 * c + 3]) * f);
+                    }
             }
 #pragma unroll
-            for (int c = 0; c < NC; ++c)
-                if (4 * tx + 64 * c < vd)
-                    *reinterpret_cast<float4*>(a.part_o + at * vd + 4 * tx + 64 * c) = make_float4(o[i][4 * c], o[i][4 * c + 1], o[i][4 * c + 2], o[i][4 * c + 3]);
-            continue;
-        }
-        float f = 1.0f, sum = l[i];
-        if (a.sinks) {                                           // the slot without key and value
-            const float sk = a.sinks[head], m_new = fmaxf(m[i], sk);
-            f = m[i] == -INFINITY ? 0.0f : expf(m[i] - m_new);
-            sum = sum * f + expf(sk - m_new);
-        }
-        f = sum > 0.0f ? f / sum : 0.0f;
-        if (a.head_gate)
-            f /= 1.0f + expf(-fb_slab_sum(a.head_gate + (size_t)row * a.gate_stride, head, a.gate_partials, a.gate_partial_stride));
-        float* op = a.out + (size_t)row * a.out_stride + (size_t)head * vd;
+            for (int i = 0; i < RPT; ++i) {
+                m[i] = -INFINITY;
+                l[i] = 0.0f;
 #pragma unroll
-        for (int c = 0; c < NC; ++c)
-            if (4 * tx + 64 * c < vd)
-                *reinterpret_cast<float4*>(op + 4 * tx + 64 * c) = make_float4(o[i][4 * c] * f, o[i][4 * c + 1] * f, o[i][4 * c + 2] * f, o[i][4 * c + 3] * f);
+                for (int c = 0; c < 4 * NC; ++c) o[i][c] = 0.0f;
+            }
+            stretch_end = tile_of(++slot + 1);
+        }
+        __syncthreads();                                         // V and the weights are free
     }
+    if (a.part_o && tx == 0)                                     // stretches that these rows do not have
+        for (; slot < slot_end; ++slot)
+            for (int r = ty * RPT; r < min((ty + 1) * RPT, rows); ++r)
+                *reinterpret_cast<float2*>(a.part_ml + 2 * part_at<BM>(a, slot, pair, q_start + r / G, kvh * G + r % G, r)) = make_float2(-INFINITY, 0.0f);
 }
 
-// One warp a (row, head): the stretches' results made one.
+// One warp a row of the CTAs above (blockIdx.y: four rows each): its stretches joined.
+template <int BM>
 __global__ void __launch_bounds__(128)
-attention_f32_merge_kernel(const F32Args a) {
+attention_f32_join_kernel(const F32Args a) {
     fb_pdl_launch_dependents();
     fb_pdl_wait();
-    const long item = (long)blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (item >= (long)a.n * a.nh) return;
-    const int lane = threadIdx.x & 31, row = (int)(item / a.nh), head = (int)(item - (long)row * a.nh);
-    const size_t stride = (size_t)a.n * a.nh;
-    float ms = -INFINITY, ls = 0.0f;                             // stretch `lane`
-    if (lane < a.n_splits) {
-        ms = a.part_ml[2 * (item + lane * stride)];
-        ls = a.part_ml[2 * (item + lane * stride) + 1];
-    }
-    float top = fb_warp_max(ms);
-    if (a.sinks) top = fmaxf(top, a.sinks[head]);
-    const float w = ms == -INFINITY ? 0.0f : expf(ms - top);
-    float sum = fb_warp_sum(w * ls);
-    if (a.sinks) sum += expf(a.sinks[head] - top);
-    float f = sum > 0.0f ? 1.0f / sum : 0.0f;
-    if (a.head_gate)
-        f /= 1.0f + expf(-fb_slab_sum(a.head_gate + (size_t)row * a.gate_stride, head, a.gate_partials, a.gate_partial_stride));
-    float* op = a.out + (size_t)row * a.out_stride + (size_t)head * a.vd;
-    for (int d = lane; d < (a.vd + 31) / 32 * 32; d += 32) {
-        float acc = 0.0f;
-        for (int s = 0; s < a.n_splits; ++s) {
-            const float ws = __shfl_sync(0xffffffffu, w, s);
-            if (d < a.vd && ws > 0.0f) acc = fmaf(ws, a.part_o[(item + s * stride) * a.vd + d], acc);
+    const int G = a.nh / a.nkv, lane = threadIdx.x & 31, r = blockIdx.y * 4 + (threadIdx.x >> 5);
+    const int pair = blockIdx.x / a.token_tiles, tile = blockIdx.x - pair * a.token_tiles;
+    const int seq = pair / a.nkv, kvh = pair - seq * a.nkv, q_len = a.seq_q_len[seq];
+    if ((q_len * G <= a.short_rows) != (BM == 16)) return;
+    const int TQ = BM / G, tok0 = (a.token_tiles - 1 - tile) * TQ;
+    if (tok0 >= q_len || r >= min(TQ, q_len - tok0) * G) return;
+    const int row = a.seq_q_start[seq] + tok0 + r / G, head = kvh * G + r % G;
+    float M = -INFINITY, L = 0.0f;
+    float4 acc[2] = {};
+#pragma unroll 4
+    for (int s = 0; s < a.slots; ++s) {
+        const size_t at = part_at<BM>(a, s, pair, row, head, r);
+        const float2 ml = *reinterpret_cast<const float2*>(a.part_ml + 2 * at);
+        if (ml.x == -INFINITY && ml.y == 0.0f) continue;         // nothing was seen there (and nothing left)
+        const Join j = join(M, L, ml.x, ml.y);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int d = 4 * lane + 128 * c;
+            if (d >= a.vd) continue;
+            const float4 x = *reinterpret_cast<const float4*>(a.part_o + at * a.vd + d);
+            acc[c] = make_float4(joined(j, acc[c].x, x.x), joined(j, acc[c].y, x.y), joined(j, acc[c].z, x.z), joined(j, acc[c].w, x.w));
         }
-        if (d < a.vd) op[d] = acc * f;
+    }
+    const float f = finish(a, row, head, M, L);
+    float* op = a.out + (size_t)row * a.out_stride + (size_t)head * a.vd;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const int d = 4 * lane + 128 * c;
+        if (d < a.vd) *reinterpret_cast<float4*>(op + d) = make_float4(acc[c].x * f, acc[c].y * f, acc[c].z * f, acc[c].w * f);
     }
 }
 
 size_t smem_bytes(int bm, int hd, int vdp) {
-    return ((size_t)(bm + KEYS) * (hd + 4) + (size_t)KEYS * vdp + (size_t)KEYS * (bm + 4) + 2 * KEYS) * sizeof(float);
+    return ((size_t)(bm + KEYS) * (hd + 4) + (size_t)KEYS * vdp + (size_t)KEYS * (bm + 4) + 4 * bm + 2 * KEYS) * sizeof(float);
 }
 
 template <int BM, int VDP>
@@ -331,8 +401,12 @@ int launch(F32Args a, int max_q_len, cudaStream_t stream) {
     const int TQ = BM / (a.nh / a.nkv);
     const int longest = BM == 16 ? min(max_q_len, TQ) : max_q_len;     // (a sequence with BM 16 is one tile)
     a.token_tiles = (longest + TQ - 1) / TQ;
-    fb_launch(kern, dim3((unsigned)((long)a.token_tiles * a.n_seqs * a.nkv), 1, a.n_splits), dim3(THREADS), smem_bytes(BM, a.hd, VDP), stream, a);
-    return fb_check_launch("attention_f32");
+    const unsigned ctas = (unsigned)((long)a.token_tiles * a.n_seqs * a.nkv);
+    fb_launch(kern, dim3(ctas, 1, (a.slots + a.per - 1) / a.per), dim3(THREADS), smem_bytes(BM, a.hd, VDP), stream, a);
+    const int rc = fb_check_launch("attention_f32");
+    if (rc || !a.part_o) return rc;
+    fb_launch((attention_f32_join_kernel<BM>), dim3(ctas, BM / 4), dim3(128), 0, stream, a);
+    return fb_check_launch("attention_f32_join");
 }
 
 template <int BM>
@@ -342,29 +416,62 @@ int launch(const F32Args& a, int max_q_len, cudaStream_t stream) {
     return launch<BM, 256>(a, max_q_len, stream);
 }
 
-}  // namespace
+// (vd + 2 floats a row are no multiple of 16 bytes, the outputs are read by 16)
+long long border4(long long floats) { return (floats + 3) / 4 * 4; }
 
-// Into how many stretches the tiles of a step are cut: as many as make four CTAs a multiprocessor, at least two tiles each,
-// at most 32.  (One CTA a multiprocessor leaves its four warps waiting on each other's loads, and CTAs that start while the
-// kernel ahead still runs then share the SMs that are free first: 301 tokens behind 500 took 560 us so.)
-FB_API int fb_attention_f32_splits(int n_seqs, int nkv, int G, int max_q_len, int max_keys) {
-    const long rows = (long)max_q_len * G;
-    const long ctas = (long)n_seqs * nkv * (rows <= 16 ? 1 : (max_q_len + 64 / G - 1) / (64 / G));
-    long s = ctas > 0 ? 4L * fb_sm_count() / ctas : 1;
-    const long most = max_keys / (2 * KEYS);
-    if (s > most) s = most;
-    if (s > MAX_SPLITS) s = MAX_SPLITS;
-    return s < 1 ? 1 : (int)s;
+// How a step's stretches are laid over CTAs.
+struct Plan {
+    int slots, per_short, per_long;     // stretches of a row at most; those a CTA takes, with BM 16 and BM 64
+    long long short_floats, long_floats;                         // scratch (0: every CTA takes all stretches)
+};
+
+// short_tiles, long_tiles: CTAs a key/value head of the sequences that run with BM 16 and BM 64.  Stretches are spread until
+// there are about four CTAs a multiprocessor.  (One leaves its four warps waiting on each other's loads, and CTAs that start
+// while the kernel ahead still runs then share the SMs that are free first: 301 tokens behind 500 took 560 us so.)  A row's
+// stretches: those of its window's keys, which begin anywhere in one and end anywhere in another, and of the kept first keys.
+Plan plan_of(int n_seqs, int n, int nh, int nkv, int vd, int max_q_len, int max_kv_len, int window, int keep_first, long long short_tiles,
+             long long long_tiles) {
+    Plan p = {};
+    long long slots = (max_kv_len + STRETCH - 1) / STRETCH;
+    if (window > 0) {
+        const long long most = (keep_first + (long long)STRETCH - 1) / STRETCH + (window + 62LL) / STRETCH + 2;
+        if (most < slots) slots = most;
+    }
+    p.slots = (int)(slots < 1 ? 1 : slots);
+    const int G = nh / nkv;
+    auto spread = [&](long long ctas, long long floats_a_slot, int& per, long long& floats) {
+        per = p.slots;
+        floats = 0;
+        if (ctas <= 0 || p.slots == 1) return;
+        const long long want = 4LL * fb_sm_count(), each = (p.slots * ctas + want / 2) / want;
+        if (each >= p.slots || p.slots * floats_a_slot > SCRATCH_FLOATS) return;
+        per = each < 1 ? 1 : (int)each;
+        floats = p.slots * floats_a_slot;                        // (slots x rows x (vd + 2))
+    };
+    spread(short_tiles * nkv, (long long)n_seqs * nkv * (max_q_len == 1 ? G : 16) * (vd + 2), p.per_short, p.short_floats);
+    spread(long_tiles * nkv, (long long)n * nh * (vd + 2), p.per_long, p.long_floats);
+    return p;
 }
 
-// q, out: float32 [rows, nh * hd] / [rows, nh * vd]; pools float32.  part: n_splits * n * nh * (vd + 2) floats (n_splits > 1).
+}  // namespace
+
+// Floats of scratch that fb_paged_attention_f32 wants for the same numbers.
+FB_API long long fb_attention_f32_scratch_floats(int n_seqs, int n, int nh, int nkv, int vd, int max_q_len, int max_kv_len, int window,
+                                                 int keep_first, long long short_tiles, long long long_tiles) {
+    if (n_seqs <= 0 || n <= 0 || nkv <= 0 || nh % nkv != 0) return 0;
+    const Plan p = plan_of(n_seqs, n, nh, nkv, vd, max_q_len, max_kv_len, window, keep_first, short_tiles, long_tiles);
+    return p.short_floats + border4(p.long_floats);
+}
+
+// q, out: float32 [rows, nh * hd] / [rows, nh * vd]; pools float32.  short_tiles: sequences with at most 16 rows (tokens x query
+// heads a key/value head; none where that is more than 16 heads); long_tiles: over the others, 64-row tiles of their tokens.
 FB_API int fb_paged_attention_f32(const float* q, long long q_stride, float* out, long long out_stride, const float* k_pool,
                                   const float* v_pool, int page_size, int n_pages, const int* block_table, int table_stride,
                                   const int* table_base, int table_head, const int* seq_q_start, const int* seq_q_len,
-                                  const int* seq_pos_start, int n_seqs, int max_q_len, int any_short, int any_long, int n, int nh,
-                                  int nkv, int hd, int vd, int window, int keep_first, float scale, float softcap,
-                                  const float* score_slopes, const float* sinks, const float* head_gate, long long gate_stride,
-                                  int gate_partials, long long gate_partial_stride, int n_splits, float* part,
+                                  const int* seq_pos_start, int n_seqs, int max_q_len, int max_kv_len, long long short_tiles,
+                                  long long long_tiles, int n, int nh, int nkv, int hd, int vd, int window, int keep_first, float scale,
+                                  float softcap, const float* score_slopes, const float* sinks, const float* head_gate,
+                                  long long gate_stride, int gate_partials, long long gate_partial_stride, float* part,
                                   long long part_floats, int* status, cudaStream_t stream) {
     FB_REQUIRE(n >= 0 && n_seqs >= 0 && nh > 0 && nkv > 0 && nh % nkv == 0, "attention_f32: bad head counts");
     FB_REQUIRE(hd % 4 == 0 && hd >= 4 && hd <= 256 && vd % 4 == 0 && vd >= 4 && vd <= 256 && nh / nkv <= 64,
@@ -375,10 +482,10 @@ FB_API int fb_paged_attention_f32(const float* q, long long q_stride, float* out
     FB_REQUIRE(softcap >= 0.0f && (!head_gate || gate_stride >= nh), "attention_f32: bad cap or gate");
     FB_REQUIRE((long long)n_seqs * nkv * max_q_len < (1LL << 31), "attention_f32: too many sequences and tokens for one grid");
     if (n == 0 || n_seqs == 0) return 0;
-    if (n_splits < 1) n_splits = 1;
-    if (n_splits > MAX_SPLITS) n_splits = MAX_SPLITS;
-    const long long items = (long long)n * nh;
-    FB_REQUIRE(n_splits == 1 || (part && part_floats >= n_splits * items * (vd + 2)), "attention_f32: too little scratch");
+    const Plan p = plan_of(n_seqs, n, nh, nkv, vd, max_q_len, max_kv_len, window, keep_first, short_tiles, long_tiles);
+    const long long wanted = p.short_floats + border4(p.long_floats);
+    FB_REQUIRE(wanted == 0 || (part && (uintptr_t)part % 16 == 0 && part_floats >= wanted),
+               "attention_f32: too little scratch");
     F32Args a;
     a.q = q; a.q_stride = (long)q_stride; a.out = out; a.out_stride = (long)out_stride;
     a.k_pool = k_pool; a.v_pool = v_pool; a.page_size = page_size; a.n_pages = n_pages;
@@ -390,20 +497,22 @@ FB_API int fb_paged_attention_f32(const float* q, long long q_stride, float* out
     a.head_gate = head_gate; a.gate_stride = (long)gate_stride;
     a.gate_partials = gate_partials < 1 ? 1 : gate_partials; a.gate_partial_stride = (long)gate_partial_stride;
     a.short_rows = nh / nkv <= 16 ? 16 : 0;                      // (a token of more than 16 heads takes BM 64)
-    a.n_splits = n_splits;
-    a.part_o = part; a.part_ml = part ? part + n_splits * items * vd : nullptr;
+    a.slots = p.slots;
+    a.part_rows = max_q_len == 1 ? nh / nkv : 16;
     a.status = status;
-    if (any_long) {
+    auto parts = [&](float* at, long long floats, int per) {     // (outputs first: they are read four at a time)
+        a.per = per;
+        a.part_o = floats ? at : nullptr;
+        a.part_ml = floats ? at + floats / (vd + 2) * vd : nullptr;
+    };
+    if (long_tiles > 0) {
+        parts(part, p.long_floats, p.per_long);
         const int rc = launch<64>(a, max_q_len, stream);
         if (rc) return rc;
     }
-    if (any_short && a.short_rows > 0) {
-        const int rc = launch<16>(a, max_q_len, stream);
-        if (rc) return rc;
-    }
-    if (n_splits > 1) {
-        fb_launch(attention_f32_merge_kernel, dim3((unsigned)((items + 3) / 4)), dim3(128), 0, stream, a);
-        return fb_check_launch("attention_f32_merge");
+    if (short_tiles > 0 && a.short_rows > 0) {
+        parts(part + border4(p.long_floats), p.short_floats, p.per_short);
+        return launch<16>(a, max_q_len, stream);
     }
     return 0;
 }

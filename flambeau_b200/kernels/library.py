@@ -59,9 +59,9 @@ _SIGNATURES = {
     # attention_tc.cu
     "fb_attention_tc_stretches": (I, [L, I, I, I]),
     # attention_f32.cu
-    "fb_attention_f32_splits": (I, [I, I, I, I, I]),
-    "fb_paged_attention_f32": (I, [P, L, P, L, P, P, I, I, P, I, P, I, P, P, P, I, I, I, I, I, I, I, I, I, I, I, F, F, P, P, P, L, I, L, I, P,
-                                   L, P, STREAM]),
+    "fb_attention_f32_scratch_floats": (L, [I, I, I, I, I, I, I, I, I, L, L]),
+    "fb_paged_attention_f32": (I, [P, L, P, L, P, P, I, I, P, I, P, I, P, P, P, I, I, I, L, L, I, I, I, I, I, I, I, F, F, P, P, P, L, I, L,
+                                   P, L, P, STREAM]),
     # qk_norm_rope.cu
     "fb_qk_norm_rope_kv_write": (I, [P, L, I, L, P, P, P, I, I, F, F, P, P, I, P, L, I, P, P, P, I, P, I, P, P, I, I, I, I,
                                      I, I, I, I, I, I, P, STREAM]),

@@ -497,11 +497,12 @@ def f32_attention_supported(q: torch.Tensor, out: torch.Tensor, k_pool: torch.Te
 def paged_attention_f32(q, out, k_pool, v_pool, block_table, seq_q_start, seq_q_len, seq_pos_start, n_seqs: int, max_q_len: int,
                         max_kv_len: int, any_short: bool, any_long: bool, nh: int, nkv: int, hd: int, window: int, scale: float,
                         status, table_base=None, score_slopes=None, sinks=None, vd: int = 0, keep_first: int = 0,
-                        table_head: int = 0, softcap: float = 0.0, head_gate=None, alloc=None) -> None:
+                        table_head: int = 0, softcap: float = 0.0, head_gate=None, alloc=None, seq_lens=None) -> None:
     """paged_attention_simt's result in float32, tile by tile (csrc/attention_f32.cu); sequences are described per entry of
     the step (first row, rows, first position).  any_short / any_long: whether the step holds sequences with rows * (nh / nkv)
-    <= 16 / > 16 (groups of more than 16 heads count as long).  `alloc(n)` returns n float32 of scratch for the results of
-    stretches of keys (default: a fresh tensor)."""
+    <= 16 / > 16 (groups of more than 16 heads count as long).  seq_lens (rows of every sequence, on the host) says how many
+    CTAs there will be, else all are taken for as long as the longest; a row's bits do not depend on it, nor on max_kv_len.
+    `alloc(n)` returns n float32 of scratch for the results of stretches of keys (default: a fresh tensor)."""
     _cuda(q, out, k_pool, v_pool, block_table, seq_q_start, seq_q_len, seq_pos_start, status, table_base, sinks)
     _i32(table_base, "table_base")
     n = q.shape[0]
@@ -516,18 +517,23 @@ def paged_attention_f32(q, out, k_pool, v_pool, block_table, seq_q_start, seq_q_
         raise KernelError("attention_f32: float32 operands with sizes that are multiples of 4 up to 256")
     if not k_pool.is_contiguous() or not v_pool.is_contiguous():
         raise KernelError("attention: cache pools must be contiguous")
-    max_keys = max_kv_len if not window else min(max_kv_len, window + int(keep_first) + max_q_len)
-    splits = lib().fb_attention_f32_splits(n_seqs, nkv, nh // nkv, max_q_len, int(max_keys))
-    part, floats = None, 0
-    if splits > 1:
-        floats = splits * n * nh * (vd + 2)
+    G = nh // nkv
+    lens = [int(m) for m in seq_lens] if seq_lens is not None else [max_q_len] * n_seqs
+    short = [G <= 16 and m * G <= 16 for m in lens] if seq_lens is not None else [not any_long] * n_seqs
+    tokens = 64 // G
+    short_tiles = sum(short) if seq_lens is not None else n_seqs if any_short else 0
+    long_tiles = sum(-(-m // tokens) for m, is_short in zip(lens, short) if not is_short)
+    floats = lib().fb_attention_f32_scratch_floats(n_seqs, n, nh, nkv, vd, max_q_len, int(max_kv_len), int(window), int(keep_first),
+                                                   short_tiles, long_tiles)
+    part = None
+    if floats > 0:
         part = alloc(floats) if alloc is not None else torch.empty(floats, dtype=torch.float32, device=q.device)
     check(lib().fb_paged_attention_f32(
         q.data_ptr(), _rows(q), out.data_ptr(), _rows(out), k_pool.data_ptr(), v_pool.data_ptr(), page_size, n_pages,
         block_table.data_ptr(), block_table.stride(0), _ptr(table_base), int(table_head), seq_q_start.data_ptr(),
-        seq_q_len.data_ptr(), seq_pos_start.data_ptr(), n_seqs, max_q_len, 1 if any_short else 0, 1 if any_long else 0, n, nh, nkv,
+        seq_q_len.data_ptr(), seq_pos_start.data_ptr(), n_seqs, max_q_len, int(max_kv_len), short_tiles, long_tiles, n, nh, nkv,
         hd, vd, int(window), int(keep_first), float(scale), float(softcap), _slopes(score_slopes, nh), _ptr(sinks),
-        *_head_gate(head_gate, n, nh), splits, _ptr(part), floats, status.data_ptr(), _stream()), "paged_attention_f32")
+        *_head_gate(head_gate, n, nh), _ptr(part), floats, status.data_ptr(), _stream()), "paged_attention_f32")
 
 
 def apply_penalties(logits, rows, tokens, counts, repetition, presence, frequency) -> None:
@@ -951,7 +957,8 @@ def paged_attention(ctx, q, out, cache, nh: int, nkv: int, hd: int, window: int,
                             b.n_seqs, b.max_q_len, longest, any(short), not all(short), nh, nkv, hd, window, scale,
                             ctx.runtime.status, table_base=cache.table_base, score_slopes=score_slopes, sinks=sinks, vd=vd,
                             keep_first=keep_first, table_head=cache.table_head, softcap=softcap, head_gate=head_gate,
-                            alloc=(lambda floats: ws.alloc((floats,), torch.float32)) if ws is not None else None)
+                            alloc=(lambda floats: ws.alloc((floats,), torch.float32)) if ws is not None else None,
+                            seq_lens=b.seq_q_len)
     else:
         paged_attention_simt(q, out, cache.k_pool, cache.v_pool, cache.block_table, b.positions, b.row_seq,
                              nh, nkv, hd, window, scale, ctx.runtime.status, table_base=cache.table_base,

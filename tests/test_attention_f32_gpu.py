@@ -90,3 +90,49 @@ def test_more_sequences_times_heads_than_a_grid_has_rows():
     sc.q_flat = torch.randn(n, sc.nh * sc.hd, generator=torch.Generator().manual_seed(4))
     (a, b), flags = both(sc, 4, "plain")
     assert flags == [0, 0] and float((a - b).abs().max() / a.abs().max()) < 5e-6
+
+
+def rows_of(sc, keep, longest, seq_lens=True, cut=None, window=0, vd=None):
+    """The tiled kernel's output for the sequences `keep` of a scene, alone in a step; cut: (sequence, rows) whose portion is only
+    its rows from there on."""
+    from flambeau_b200.kernels import ops
+    vd = vd or sc.hd
+    g = torch.Generator().manual_seed(7)
+    v = torch.randn(*sc.k_pool.shape[:3], vd, generator=g).to(DEV)
+    lens, starts = sc.seq_q_len[keep].clone(), [int(sc.seq_q_start[s]) for s in keep]
+    pos = sc.seq_pos_start[keep].clone()
+    if cut is not None:
+        lens[0], starts[0], pos[0] = lens[0] - cut, starts[0] + cut, pos[0] + cut
+    rows = torch.cat([torch.arange(a, a + int(m)) for a, m in zip(starts, lens)])
+    q_start = torch.cumsum(lens, 0, dtype=torch.int32) - lens
+    q = sc.q_flat[rows].to(DEV)
+    out, status = torch.full((len(rows), sc.nh * vd), float("nan"), device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    G = sc.nh // sc.nkv
+    short = [G <= 16 and m * G <= 16 for m in lens.tolist()]
+    sinks = torch.randn(sc.nh, generator=g).to(DEV)
+    ops.paged_attention_f32(q, out, sc.k_pool.nan_to_num(0.0).to(DEV), v, sc.table[keep].to(DEV), q_start.to(DEV), lens.to(DEV), pos.to(DEV),
+                            len(keep), int(lens.max()), longest, any(short), not all(short), sc.nh, sc.nkv, sc.hd, window, sc.hd ** -0.5,
+                            status, vd=vd, sinks=sinks, keep_first=40 if window else 0, seq_lens=lens.tolist() if seq_lens else None)
+    assert int(status.item()) == 0 and bool(torch.isfinite(out).all())
+    return out, q_start.tolist(), lens.tolist()
+
+
+@pytest.mark.parametrize("window", [0, 700, 90])
+@pytest.mark.parametrize("sizes", [(8, 2, 64, 64), (32, 8, 128, 128), (16, 1, 256, 256), (20, 1, 20, 12), (3, 3, 40, 72)], ids=str)
+def test_a_row_has_the_same_bits_whatever_shares_its_step(sizes, window):
+    """Decoded tokens and portions alone, together, beside many others, with other bounds on the longest context (which decide
+    over how many CTAs the keys are cut), and the last row of a portion as a token of its own."""
+    nh, nkv, hd, vd = sizes
+    seqs = [(2600, 1), (511, 1), (256, 300), (1000, 71), (37, 5), (0, 1)]      # (an odd number of rows, heads and stretches once)
+    sc = Scene(seqs, nh, nkv, hd, 0, torch.float32, seed=hd)
+    everyone = list(range(len(seqs)))
+    whole, start, lens = rows_of(sc, everyone, 2601, window=window, vd=vd)
+    for s in everyone:
+        mine = whole[start[s]:start[s] + lens[s]]
+        for keep, longest in (([s], sum(seqs[s])), ([s], 32768), ([s] + everyone[::2] + everyone, 4000)):
+            got, at, _ = rows_of(sc, keep, max(longest, max(sum(seqs[k]) for k in keep)), seq_lens=longest != 4000, window=window, vd=vd)
+            assert torch.equal(got[at[0]:at[0] + lens[s]], mine), (s, keep, longest)
+        if lens[s] > 1:
+            for cut in (lens[s] - 1, lens[s] // 3):
+                got, _, _ = rows_of(sc, [s], 2601, cut=cut, window=window, vd=vd)
+                assert torch.equal(got, mine[cut:]), (s, cut)
