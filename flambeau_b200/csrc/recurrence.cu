@@ -108,6 +108,22 @@ template <int R, int LPC, int NC, int THREADS, bool SPLIT> struct Cut {
     __host__ __device__ static constexpr int floats(int ch) { return STAGES * stage_floats(ch); }
 };
 
+// A lane's share of a column's sum S^T x, x in groups of four channels: pairs of channels in float32x2.  Sixteen channels a lane
+// are two chains of eight, so that 8 lanes of sixteen and 16 lanes of eight add in one order: what a step's launch gives a lane
+// does not show in the result.
+template <int R> __device__ __forceinline__ float lane_sum(const f2* s, const ulonglong2* x) {
+    constexpr int CHAINS = R == 16 ? 2 : 1;
+    float part[CHAINS];
+#pragma unroll
+    for (int h = 0; h < CHAINS; ++h) {
+        f2 y = fma2(s[2 * h + 1], x[h].y, mul2(s[2 * h], x[h].x));
+#pragma unroll
+        for (int r = h + CHAINS; r < R / 4; r += CHAINS) y = fma2(s[2 * r + 1], x[r].y, fma2(s[2 * r], x[r].x, y));
+        part[h] = sum2(y);
+    }
+    return CHAINS == 2 ? part[0] + part[CHAINS - 1] : part[0];
+}
+
 // Named barriers of a CTA: `count` threads meet, or come by.
 __device__ __forceinline__ void meet(int id, int count) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory"); }
 __device__ __forceinline__ void come_by(int id, int count) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory"); }
@@ -324,18 +340,8 @@ recurrent_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, 
         for (int j = 0; j < N; ++j)
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
-                f2 y = mul2(s[c][0], x.q[j][0].x);
-                y = fma2(s[c][1], x.q[j][0].y, y);
-#pragma unroll
-                for (int r = 1; r < R / 4; ++r) y = fma2(s[c][2 * r + 1], x.q[j][r].y, fma2(s[c][2 * r], x.q[j][r].x, y));
-                b[c * N + j] = sum2(y);
-                if constexpr (DELTA) {
-                    y = mul2(s[c][0], x.k[j][0].x);
-                    y = fma2(s[c][1], x.k[j][0].y, y);
-#pragma unroll
-                    for (int r = 1; r < R / 4; ++r) y = fma2(s[c][2 * r + 1], x.k[j][r].y, fma2(s[c][2 * r], x.k[j][r].x, y));
-                    a[c * N + j] = sum2(y);
-                }
+                b[c * N + j] = lane_sum<R>(s[c], x.q[j]);
+                if constexpr (DELTA) a[c * N + j] = lane_sum<R>(s[c], x.k[j]);
             }
         float D[DOTS];
 #pragma unroll

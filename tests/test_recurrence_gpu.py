@@ -9,7 +9,7 @@ from test_fegizen_gpu import fake_batch
 pytestmark = pytest.mark.gpu
 DEV, F64 = "cuda:0", torch.float64
 
-LENGTHS = [[1, 1, 1], [2, 5], [4, 1, 3], [31, 64], [33, 7, 66], [100]]
+LENGTHS = [[1, 1, 1], [3, 2, 1], [2, 5], [4, 1, 3], [31, 64], [33, 7, 66], [100]]
 # (key size, value size, heads, query/key heads)
 SIZES = [(4, 3, 2, 1), (16, 40, 2, 2), (18, 70, 2, 1), (32, 33, 4, 2), (64, 17, 2, 1), (100, 40, 2, 2), (128, 128, 4, 2), (128, 33, 20, 20),
          (128, 100, 30, 10), (127, 16, 2, 2), (200, 20, 2, 1), (256, 31, 1, 1), (500, 9, 1, 1), (600, 5, 1, 1), (1024, 6, 1, 1)]
@@ -64,3 +64,39 @@ def test_recurrence_equals_its_formula(rule, sizes, lengths):
     scale_o, scale_s = float(want_o.abs().max()), float(want_s.abs().max())
     assert float((o.double().cpu().view(n, H, dv) - want_o).abs().max()) < 4e-6 * scale_o
     assert float((sd.double().cpu() - want_s).abs().max()) < 4e-6 * scale_s
+
+
+def run(rule, qkv, beta, decay, state, lengths, slots, sizes):
+    from flambeau_b200.kernels import ops
+    dk, dv, H, G = sizes
+    batch, st, o = fake_batch(lengths, slots), state.clone(), torch.empty(sum(lengths), H * dv, device=DEV)
+    if rule == "linear":
+        ops.gla_recurrent(qkv, decay, st, batch, o, H, dk, dv)
+    else:
+        (ops.gdr_recurrent if rule == "head" else ops.gdr_channel_recurrent)(qkv, beta, decay, st, batch, o, G, H, dk, dv)
+    return o, st
+
+
+@pytest.mark.parametrize("sizes", [(128, 128, 16, 4), (128, 40, 8, 8), (64, 64, 4, 2), (96, 33, 4, 4), (127, 20, 4, 4), (200, 24, 2, 2),
+                                   (256, 64, 3, 3), (512, 16, 4, 4), (700, 8, 2, 2)], ids=str)
+@pytest.mark.parametrize("rule", ["head", "channel", "linear"])
+def test_a_request_has_the_same_bits_whatever_shares_its_step(rule, sizes):
+    """Every request alone, with one other and with all others: a decoded token in a step of such tokens and beside portions,
+    a portion that has the device to itself and one that shares it."""
+    dk, dv, H, G = sizes
+    G = H if rule == "linear" else G
+    sizes = (dk, dv, H, G)
+    lengths = [1, 90, 2, 343, 1, 3, 64, 7]
+    gen = torch.Generator(device=DEV).manual_seed(dk + dv)
+    n, starts = sum(lengths), [sum(lengths[:i]) for i in range(len(lengths))]
+    qkv = torch.randn(n, 2 * G * dk + H * dv, generator=gen, device=DEV) * dk ** -0.5
+    beta, decay = (torch.rand(n, w, generator=gen, device=DEV) ** 0.25 for w in (H, H * dk if rule != "head" else H))
+    state = torch.randn(len(lengths), H * dv * dk, generator=gen, device=DEV)
+    whole, st_whole = run(rule, qkv, beta, decay, state, lengths, list(range(len(lengths))), sizes)
+    for i, length in enumerate(lengths):
+        for others in ([], [0], [3], [4, 0]):
+            who = [i] + [x for x in others if x != i]
+            rows = torch.cat([torch.arange(starts[x], starts[x] + lengths[x], device=DEV) for x in who])
+            o, st = run(rule, qkv[rows], beta[rows], decay[rows], state, [lengths[x] for x in who], who, sizes)
+            assert torch.equal(o[:length], whole[starts[i]:starts[i] + length]), (i, who)
+            assert torch.equal(st[i], st_whole[i]), (i, who)
