@@ -714,6 +714,8 @@ def gather_rows(h: torch.Tensor, place_token: torch.Tensor, out: torch.Tensor, s
     rows, D = out.shape
     if h.dtype != out.dtype or h.shape[1] != D or not out.is_contiguous() or place_token.numel() < rows:
         raise KernelError("gather_rows: shapes or dtypes do not agree")
+    if tile_group is not None and (tile <= 0 or tile_group.numel() * int(tile) < rows):
+        raise KernelError("gather_rows: fewer tiles than rows")
     check(lib().fb_moe_gather_rows(h.data_ptr(), _rows(h), dtype_code(h), place_token.data_ptr(), out.data_ptr(), rows,
                                    D, _ptr(share), _ptr(place_pair), _ptr(tile_group), int(tile), _stream()), "moe_gather_rows")
 

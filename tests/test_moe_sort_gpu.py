@@ -30,3 +30,33 @@ def test_every_pair_has_its_place(n, K, E, tile, load):
     count = torch.bincount(flat[has].long(), minlength=E)
     want = torch.repeat_interleave(torch.arange(E), -(-count // tile)).int()
     assert torch.equal(expert[:want.numel()], want) and bool((expert[want.numel():] == -1).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=str)
+@pytest.mark.parametrize("width", [64, 2048, 100])
+@pytest.mark.parametrize("shared", [False, True])
+def test_rows_of_tiles_that_have_a_group(dtype, width, shared):
+    """Fetched rows of used tiles, with and without shares and places without a token; a skipped tile keeps what it held in the
+    form that moves eight numbers at a time (100 is no multiple: one number at a time writes it).  Tables that do not reach over
+    all rows are refused before anything is launched."""
+    from flambeau_b200.kernels import ops
+    from flambeau_b200.kernels.library import KernelError
+    g = torch.Generator().manual_seed(width)
+    n, tile, tiles = 40, 16, 5
+    rows = tiles * tile
+    h = torch.randn(n, width, generator=g).to("cuda", dtype)
+    token = torch.randint(0, n, (rows,), generator=g).int()
+    token[torch.rand(rows, generator=g) < 0.2] = -1
+    group = torch.tensor([3, -1, 0, 3, -1], dtype=torch.int32)
+    share, pair = torch.rand(2 * n, generator=g), torch.randint(0, 2 * n, (rows,), generator=g).int()
+    more = dict(share=share.cuda(), place_pair=pair.cuda()) if shared else {}
+    out = torch.full((rows, width), 7.0, dtype=dtype, device="cuda")
+    ops.gather_rows(h, token.cuda(), out, tile_group=group.cuda(), tile=tile, **more)
+    want = torch.where(token[:, None] >= 0, h.cpu().float()[token.clamp_min(0).long()] * (share[pair.long()][:, None] if shared else 1.0), 0.0)
+    used = (group >= 0).repeat_interleave(tile)
+    assert torch.equal(out.cpu()[used], want.to(dtype)[used])
+    if width % 8 == 0:
+        assert bool((out.cpu()[~used] == 7.0).all())
+    for bad in (dict(tile_group=group[:4].cuda(), tile=tile), dict(tile_group=group.cuda(), tile=0), dict(tile_group=group.cuda(), tile=15)):
+        with pytest.raises(KernelError):
+            ops.gather_rows(h, token.cuda(), out, **bad)
