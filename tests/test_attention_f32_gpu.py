@@ -136,3 +136,31 @@ def test_a_row_has_the_same_bits_whatever_shares_its_step(sizes, window):
             for cut in (lens[s] - 1, lens[s] // 3):
                 got, _, _ = rows_of(sc, [s], 2601, cut=cut, window=window, vd=vd)
                 assert torch.equal(got, mine[cut:]), (s, cut)
+
+
+def test_replayed_decode_steps_across_the_ends_of_stretches(tmp_path):
+    """Two requests decode past positions 256 and 512 from one captured graph, whose stretches were laid out for the longest
+    context that the engine allows: the same bits as step by step without graphs and in another company."""
+    import tiny
+    from flambeau_b200.engine.batch import Entry
+    from flambeau_b200.engine.step import Engine, EngineOptions
+    cfg = dict(tiny.CONFIGS["A"], sliding_window=None)
+    folder = tiny.make_folder(tmp_path / "m", cfg, seed=3, dtype="float32")
+    toks = tiny.random_requests(cfg, [262, 518], seed=5)
+    got = {}
+    for graphs, longest in ((True, 3000), (False, 3000), (False, 600)):
+        engine = Engine.from_folder(folder, EngineOptions(dtype="float32", cache_tokens=6400, max_requests=2, max_step_tokens=1024,
+                                                          max_seq_len=longest, cuda_graphs=graphs))
+        engine.step([Entry("a", toks["r0"][:250], [249]), Entry("b", toks["r1"][:506], [505])])
+        got[graphs, longest] = [engine.step([Entry("a", [toks["r0"][250 + t]], [0]), Entry("b", [toks["r1"][506 + t]], [0])]).clone()
+                                for t in range(12)]
+        engine.runtime.check_status("decode")
+    for steps in list(got.values())[1:]:
+        for x, y in zip(got[True, 3000], steps):
+            assert torch.equal(x, y)
+    alone = Engine.from_folder(folder, EngineOptions(dtype="float32", cache_tokens=6400, max_requests=2, max_step_tokens=1024,
+                                                     max_seq_len=3000, cuda_graphs=False))
+    alone.step([Entry("b", toks["r1"][:100], [])])
+    alone.step([Entry("b", toks["r1"][100:506], [405])])
+    for t in range(12):
+        assert torch.equal(alone.step([Entry("b", [toks["r1"][506 + t]], [0])])[0], got[True, 3000][t][1])
