@@ -1,4 +1,4 @@
-// mbarrier and bulk-copy (TMA) primitives shared by the kernels that stage
+// mbarrier, bulk-copy (TMA) and cp.async primitives shared by the kernels that stage
 // their operands asynchronously.  Every wait is bounded in time: when it runs
 // out, FB_STATUS_WAIT_TIMEOUT is set in the status word and the caller leaves
 // its loop, so a fault in the pipeline logic shows as an error, never as a hang.
@@ -52,6 +52,17 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* st
         }
     }
 }
+
+// 4 or 16 bytes from global to shared memory (both aligned to as many) by a thread's own asynchronous copies, which are
+// counted in groups: cp_async_wait<LEFT> waits until all but the thread's LEFT newest groups have landed.
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
 
 // `bytes` contiguous bytes from global to shared memory (both 16-byte aligned, bytes a multiple of 16);
 // completion is counted on the mbarrier.

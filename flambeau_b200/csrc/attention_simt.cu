@@ -10,8 +10,9 @@
 //
 // The same kernel serves prompt portions and decoded tokens in one launch: a
 // row only needs its position and the block table of its sequence (whose row starts
-// at logical page table_base[sequence], or at page 0 without table_base).  It is the
-// attention of the true 32-bit path and the reference for the faster kernels.
+// at logical page table_base[sequence], or at page 0 without table_base).  It takes what
+// the faster kernels do not (in the true 32-bit path sizes that are no multiple of 4 or
+// above 256, and rows off 16-byte borders) and is their reference.
 //
 // Value rows may be narrower or wider than key rows (vd against hd).  With `sinks` (one float32 per query head) the
 // softmax has one more slot whose score is that number as it stands (not scaled) and which carries no value: it

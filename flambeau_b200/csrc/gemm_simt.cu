@@ -8,7 +8,7 @@
 // on how many rows the call has.
 // Weight layout as in the reference: rows = outputs, columns = inputs
 // (crates/kernels-hip/src/kernels/mmq_f16_tile.cu:34-39).
-#include "common.cuh"
+#include "async_copy.cuh"
 
 template <typename TA, typename TW, typename TO, int BM, int BN, int BK, int TM, int TN>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
@@ -76,10 +76,6 @@ gemm_simt_kernel(const TA* __restrict__ A, long lda, const TW* __restrict__ W, l
 // 48 cycles of shared memory stand beside 256 multiply-adds of a warp at 8 x 8 a thread; the two overlap to about 30 TFLOP/s
 // of the 74 that the multiply-adds alone would give.  Measured (us, before / here): 301 x 6,144 x 4,096 961 / 571, 301 x 4,096
 // x 4,096 903 / 557, 64 x 28,672 x 4,096 954 / 601, 8 x 4,096 x 4,096 188 / 53.
-__device__ __forceinline__ void f32_copy16(float* dst, const float* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-
 template <int BM, int BN, int BK, int STAGES, int TM, int TN>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 gemm_f32_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W, long ldw, float* __restrict__ out, long ldo,
@@ -99,11 +95,11 @@ gemm_f32_kernel(const float* __restrict__ A, long lda, const float* __restrict__
                 const int r = e / (BK / 4), k = 4 * (e - r * (BK / 4));
                 const bool in = k0 + k < K && (r < BM ? m0 + r < M : n0 + r - BM < N);      // (K is a multiple of 4)
                 float* dst = st + r * LD + k;
-                if (in) f32_copy16(dst, (r < BM ? A + (size_t)(m0 + r) * lda : W + (size_t)(n0 + r - BM) * ldw) + k0 + k);
+                if (in) cp_async16(dst, (r < BM ? A + (size_t)(m0 + r) * lda : W + (size_t)(n0 + r - BM) * ldw) + k0 + k);
                 else *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        cp_async_commit();
     };
     unsigned long long acc[TM][TN];                    // (sum over even k, sum over odd k)
 #pragma unroll
@@ -113,7 +109,7 @@ gemm_f32_kernel(const float* __restrict__ A, long lda, const float* __restrict__
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) fetch(s);
     for (int step = 0; step < n_steps; ++step) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        cp_async_wait<STAGES - 2>();
         __syncthreads();                               // this step's stage is there; the one before it is free
         fetch(step + STAGES - 1);
         const float* as = sh + step % STAGES * STAGE + ty * TM * LD;
