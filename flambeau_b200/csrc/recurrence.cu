@@ -17,8 +17,15 @@
 //
 // LPC lanes share NC neighbouring columns, R key channels a lane: vectors leave shared memory as 16-byte loads that feed NC
 // columns (the lanes that load the same vector are neighbours: measured, a warp's 16-byte load takes two cycles of shared
-// memory where neighbouring lanes agree and four however else they agree), products run on pairs of channels (fma.rn.f32x2), and the lanes' sums are exchanged by halves.  Tokens arrive by
-// asynchronous copies, a stage of some blocks at a time.
+// memory where neighbouring lanes agree and four however else they agree), products run on pairs of channels
+// (fma.rn.f32x2), and the lanes' sums are exchanged by halves.  Tokens arrive by asynchronous copies, a stage of some blocks
+// at a time.
+//
+// Requests with fewer than four tokens in a step (decoded tokens) go token by token, fetched straight into registers: in a
+// kernel of their own where a step has one token a request, beside the portions else.
+//
+// What a request's bits depend on: its tokens, its state and where its prompt was cut (blocks count from a portion's first
+// token), not the requests that share its step or how many columns and channels a launch gives a lane.
 //
 // What bounds it: 13 multiply-adds a channel and column for four tokens are 97 us of 2,048 tokens on 32 heads of 128 x 128;
 // with the exchange, the loads and the stages a warp issues 700 instructions for those 208, most of them depending on the one
@@ -29,6 +36,7 @@
 // [q: G*dk | k: G*dk | v: H*dv]; head h of H reads q/k head h / (H / G).
 #include <type_traits>
 
+#include "async_copy.cuh"
 #include "rows.cuh"
 
 namespace {
@@ -39,15 +47,6 @@ constexpr int TB = 4;                  // tokens of a block
 constexpr int DOTS = 16;               // products between the tokens of a block: k_i k_j (i < j), then k_i q_j (i <= j)
 __device__ constexpr int kk_at(int i, int j) { return i * 3 - i * (i - 1) / 2 + j - i - 1; }
 __device__ constexpr int kq_at(int i, int j) { return 6 + i * 4 - i * (i - 1) / 2 + j - i; }
-
-__device__ __forceinline__ void copy4(float* dst, const float* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copy16(float* dst, const float* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int LEFT> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
 
 // Two float32 in one 64-bit register.
 typedef unsigned long long f2;
@@ -128,15 +127,150 @@ template <int R> __device__ __forceinline__ float lane_sum(const f2* s, const ul
 __device__ __forceinline__ void meet(int id, int count) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory"); }
 __device__ __forceinline__ void come_by(int id, int count) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory"); }
 
+// The first channel of lane li's r-th group of four, LPC lanes a column.
+template <int LPC> __device__ __forceinline__ int channel_of(int r, int li) { return r * (4 * LPC) + 4 * li; }
+
+// Four channels of a row from d on, zeros beyond dk.
+template <bool BY4> __device__ __forceinline__ ulonglong2 load_group(const float* row, int d, int dk) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (BY4) {
+        if (d < dk) v = Vec4<float>::load(row + d);
+    } else {
+        if (d < dk) v.x = row[d];
+        if (d + 1 < dk) v.y = row[d + 1];
+        if (d + 2 < dk) v.z = row[d + 2];
+        if (d + 3 < dk) v.w = row[d + 3];
+    }
+    return make_ulonglong2(pack2(v.x, v.y), pack2(v.z, v.w));
+}
+template <bool BY4> __device__ __forceinline__ void store_group(float* row, int d, int dk, f2 lo, f2 hi) {
+    float x[4];
+    unpack2(lo, x[0], x[1]);
+    unpack2(hi, x[2], x[3]);
+    if constexpr (BY4) {
+        if (d < dk) Vec4<float>::store(row + d, make_float4(x[0], x[1], x[2], x[3]));
+    } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (d + u < dk) row[d + u] = x[u];
+    }
+}
+
+// Where the tokens, states and results of a launch lie.
+struct Rows {
+    const float* qkv; const float* beta; const float* decay;
+    float* state; long state_stride;
+    const int* seq_q_start; const int* seq_q_len; const int* seq_slot;
+    float* o;
+    int G, H, dk, dv;
+};
+
+// A request's tokens one by one, for a decoded token or a few (fewer than a block's): a lane fetches its channels of the
+// token's vectors and of its columns' state from global memory, and nothing passes through shared memory.
+template <int RULE, int R, int LPC, int NC, bool BY4>
+__device__ __forceinline__ void few_tokens(const Rows& a, int seq, int head, int li, int col0, int L) {
+    constexpr bool DELTA = RULE != LINEAR;
+    constexpr int PW = 32 / LPC;
+    const int dk = a.dk, dv = a.dv, qk = a.G * dk, C = 2 * qk + a.H * dv, g = head / (a.H / a.G);
+    float* S = a.state + (size_t)a.seq_slot[seq] * a.state_stride + (size_t)head * dv * dk;
+    f2 s[NC][R / 2];
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+        for (int r = 0; r < R / 4; ++r) {
+            const ulonglong2 v = load_group<BY4>(S + (size_t)(col0 + c) * dk, channel_of<LPC>(r, li), col0 + c < dv ? dk : 0);
+            s[c][2 * r] = v.x;
+            s[c][2 * r + 1] = v.y;
+        }
+#pragma unroll 1
+    for (int t = 0; t < L; ++t) {
+        const size_t row = (size_t)a.seq_q_start[seq] + t;
+        const float* qp = a.qkv + row * C + (size_t)g * dk;
+        ulonglong2 q[R / 4], k[R / 4], w[R / 4];
+#pragma unroll
+        for (int r = 0; r < R / 4; ++r) {
+            const int d = channel_of<LPC>(r, li);
+            q[r] = load_group<BY4>(qp, d, dk);
+            k[r] = load_group<BY4>(qp + qk, d, dk);
+            if constexpr (RULE == DELTA_HEAD) {
+                const float x = a.decay[row * a.H + head];
+                w[r].x = w[r].y = pack2(x, x);
+            } else w[r] = load_group<BY4>(a.decay + (row * a.H + head) * dk, d, dk);
+        }
+        float v[NC], bt = 1.0f;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) v[c] = col0 + c < dv ? a.qkv[row * C + 2 * qk + (size_t)head * dv + col0 + c] : 0.0f;
+        if constexpr (DELTA) bt = a.beta[row * a.H + head];
+        constexpr int SUMS = 1 + NC * (DELTA ? 2 : 1);           // k.q, then S^T q and S^T k of every column
+        float sum[SUMS];
+        f2 kf[R / 2];
+#pragma unroll
+        for (int r = 0; r < R / 4; ++r) {
+            kf[2 * r] = k[r].x;
+            kf[2 * r + 1] = k[r].y;
+        }
+        sum[0] = lane_sum<R>(kf, q);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+#pragma unroll
+            for (int r = 0; r < R / 4; ++r) {
+                s[c][2 * r] = mul2(s[c][2 * r], w[r].x);
+                s[c][2 * r + 1] = mul2(s[c][2 * r + 1], w[r].y);
+            }
+            sum[1 + c] = lane_sum<R>(s[c], q);
+            if constexpr (DELTA) sum[1 + NC + c] = lane_sum<R>(s[c], k);
+        }
+#pragma unroll
+        for (int off = LPC / 2; off > 0; off >>= 1)
+#pragma unroll
+            for (int i = 0; i < SUMS; ++i) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], off * PW);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            float u = v[c];
+            if constexpr (DELTA) u = bt * (v[c] - sum[1 + NC + c]);
+            const f2 uu = pack2(u, u);
+#pragma unroll
+            for (int r = 0; r < R / 4; ++r) {
+                s[c][2 * r] = fma2(k[r].x, uu, s[c][2 * r]);
+                s[c][2 * r + 1] = fma2(k[r].y, uu, s[c][2 * r + 1]);
+            }
+            if (li == 0 && col0 + c < dv) a.o[row * a.H * dv + (size_t)head * dv + col0 + c] = fmaf(u, sum[0], sum[1 + c]);
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+        for (int r = 0; r < R / 4; ++r)
+            if (col0 + c < dv) store_group<BY4>(S + (size_t)(col0 + c) * dk, channel_of<LPC>(r, li), dk, s[c][2 * r], s[c][2 * r + 1]);
+}
+
+// Steps of one token a request (decoding).
+template <int RULE, int R, int LPC, int NC, bool BY4>
+__global__ void __launch_bounds__(128)
+one_token_kernel(const Rows a) {
+    fb_pdl_wait();
+    fb_pdl_launch_dependents();                                  // (not ahead of the wait: see recurrent_kernel)
+    constexpr int PW = 32 / LPC, COLS = 128 / LPC * NC;
+    const int seq = blockIdx.x / a.H, head = blockIdx.x - seq * a.H;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int L = a.seq_q_len[seq];
+    if (L > 0) few_tokens<RULE, R, LPC, NC, BY4>(a, seq, head, lane / PW, blockIdx.y * COLS + (warp * PW + lane % PW) * NC, L);
+}
+
 // BY4: rows of q, k, decay and the state start on 16-byte borders and dk is a multiple of 4.
 template <int RULE, int R, int LPC, int NC, int THREADS, bool BY4, bool SPLIT>
 __global__ void __launch_bounds__(SPLIT ? 2 * THREADS : THREADS)
-recurrent_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, const float* __restrict__ decay,
-                 float* __restrict__ state, long state_stride, const int* __restrict__ seq_q_start,
-                 const int* __restrict__ seq_q_len, const int* __restrict__ seq_slot, float* __restrict__ o, int G, int H, int dk,
-                 int dv, int ch) {
-    fb_pdl_launch_dependents();
+recurrent_kernel(const Rows a_, int ch) {
+    // The kernels behind are let in when the one ahead has ended, not before: CTAs of the output product, which hold an SM's
+    // shared memory for their weights, else take the SMs that this kernel has not filled (three decoded tokens, a decay per
+    // channel, 16 heads: a layer 37.7 us so, 35.2 in this order; 17 tokens 49.1 and 45.5).
+    const float* __restrict__ qkv = a_.qkv;
+    const float* __restrict__ beta = a_.beta;
+    const float* __restrict__ decay = a_.decay;
+    float* __restrict__ o = a_.o;
+    const int G = a_.G, H = a_.H, dk = a_.dk, dv = a_.dv;
     fb_pdl_wait();
+    fb_pdl_launch_dependents();
     using C_ = Cut<R, LPC, NC, THREADS, SPLIT>;
     constexpr int DKP = C_::DKP, COLS = C_::COLS, WARPS = THREADS / 32;
     constexpr bool DELTA = RULE != LINEAR;
@@ -147,8 +281,12 @@ recurrent_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, 
     constexpr int PW = 32 / LPC;                                 // groups of columns a warp; their lanes alternate
     const int li = lane / PW, group = warp * PW + lane % PW, col0 = blockIdx.y * COLS + group * NC;
     const int qk = G * dk, C = 2 * qk + H * dv;
-    const int start = seq_q_start[seq], L = seq_q_len[seq];
-    float* S = state + (size_t)seq_slot[seq] * state_stride + (size_t)head * dv * dk;
+    const int start = a_.seq_q_start[seq], L = a_.seq_q_len[seq];
+    if (L < TB) {                                                // a decoded token beside portions
+        if (L > 0 && threadIdx.x < THREADS) few_tokens<RULE, R, LPC, NC, BY4>(a_, seq, head, li, col0, L);
+        return;
+    }
+    float* S = a_.state + (size_t)a_.seq_slot[seq] * a_.state_stride + (size_t)head * dv * dk;
     auto stage = [&](int i) { return sh + i % C_::STAGES * C_::stage_floats(ch); };
     auto ends_of = [&](float* st) { return st + ch * (3 * DKP + COLS + 2); };                 // [block rows][DKP]
     auto dots_of = [&](float* st) { return ends_of(st) + C_::block_rows(ch) * DKP; };         // [block rows][DOTS]
@@ -169,13 +307,13 @@ recurrent_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, 
                 const float* rowp = qkv + row * C + (size_t)g * dk + d;
                 const float* gp = decay + (row * H + head) * dk + d;
                 if constexpr (BY4) {
-                    copy16(qs + e, rowp);
-                    copy16(ks + e, rowp + qk);
-                    if constexpr (RULE != DELTA_HEAD) copy16(gs + e, gp);
+                    cp_async16(qs + e, rowp);
+                    cp_async16(ks + e, rowp + qk);
+                    if constexpr (RULE != DELTA_HEAD) cp_async16(gs + e, gp);
                 } else {
-                    copy4(qs + e, rowp);
-                    copy4(ks + e, rowp + qk);
-                    if constexpr (RULE != DELTA_HEAD) copy4(gs + e, gp);
+                    cp_async4(qs + e, rowp);
+                    cp_async4(ks + e, rowp + qk);
+                    if constexpr (RULE != DELTA_HEAD) cp_async4(gs + e, gp);
                 }
             } else {
 #pragma unroll
@@ -184,17 +322,15 @@ recurrent_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, 
         }
         for (int e = tid; e < cnt * COLS; e += THREADS) {
             const int t = e / COLS, c2 = blockIdx.y * COLS + (e - t * COLS);
-            if (c2 < dv) copy4(vs + e, qkv + (size_t)(start + t0 + t) * C + 2 * qk + (size_t)head * dv + c2);
+            if (c2 < dv) cp_async4(vs + e, qkv + (size_t)(start + t0 + t) * C + 2 * qk + (size_t)head * dv + c2);
             else vs[e] = 0.0f;
         }
         if (DELTA && tid < cnt) {
-            copy4(vs + ch * COLS + tid, beta + (size_t)(start + t0 + tid) * H + head);
-            if constexpr (RULE == DELTA_HEAD) copy4(vs + ch * (COLS + 1) + tid, decay + (size_t)(start + t0 + tid) * H + head);
+            cp_async4(vs + ch * COLS + tid, beta + (size_t)(start + t0 + tid) * H + head);
+            if constexpr (RULE == DELTA_HEAD) cp_async4(vs + ch * (COLS + 1) + tid, decay + (size_t)(start + t0 + tid) * H + head);
         }
-        copies_commit();
+        cp_async_commit();
     };
-    // The first channel of this lane's r-th group of four.
-    auto channel = [&](int r4) { return r4 * (4 * LPC) + 4 * li; };
 
     // The vectors of the N tokens from `t` on made what the columns want of them, in place (q: G(1..j) q_j; k: G(1..j) k_j;
     // decay: G(j+1..N) k_j), the block's decay, and the products between its tokens, by one warp.
@@ -281,8 +417,8 @@ recurrent_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, 
             if (i + 1 < n_stages) {
                 if (i + 1 >= C_::STAGES) meet(1 + C_::STAGES + (i + 1) % C_::STAGES, 2 * THREADS);
                 fetch((i + 1) * ch, stage(i + 1));
-                copies_wait<1>();
-            } else copies_wait<0>();
+                cp_async_wait<1>();
+            } else cp_async_wait<0>();
             meet(1 + 2 * C_::STAGES, THREADS);           // every fetching thread's copies are there
             prepare_stage(i);
             come_by(1 + i % C_::STAGES, 2 * THREADS);
@@ -292,24 +428,13 @@ recurrent_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, 
 
     f2 s[NC][R / 2];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-        const bool live = col0 + c < dv;
-        const float* Sc = S + (size_t)(live ? col0 + c : 0) * dk;
+    for (int c = 0; c < NC; ++c)
 #pragma unroll
         for (int r = 0; r < R / 4; ++r) {
-            const int d = channel(r);
-            float x[4];
-            if constexpr (BY4) {
-                const float4 v = live && d < dk ? Vec4<float>::load(Sc + d) : make_float4(0.f, 0.f, 0.f, 0.f);
-                x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
-            } else {
-#pragma unroll
-                for (int u = 0; u < 4; ++u) x[u] = live && d + u < dk ? Sc[d + u] : 0.0f;
-            }
-            s[c][2 * r] = pack2(x[0], x[1]);
-            s[c][2 * r + 1] = pack2(x[2], x[3]);
+            const ulonglong2 v = load_group<BY4>(S + (size_t)(col0 + c) * dk, channel_of<LPC>(r, li), col0 + c < dv ? dk : 0);
+            s[c][2 * r] = v.x;
+            s[c][2 * r + 1] = v.y;
         }
-    }
 
     // The vectors of N tokens that the state is multiplied with, in registers.
     struct Vectors { ulonglong2 q[TB][R / 4], k[DELTA ? TB : 1][R / 4]; };
@@ -426,8 +551,8 @@ recurrent_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, 
         } else {
             if (i + 1 < n_stages) {                      // (its last readers passed the barrier below)
                 fetch(t0 + ch, stage(i + 1));
-                copies_wait<1>();
-            } else copies_wait<0>();
+                cp_async_wait<1>();
+            } else cp_async_wait<0>();
             __syncthreads();
             prepare_stage(i);
             __syncthreads();
@@ -442,30 +567,14 @@ recurrent_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, 
         } else __syncthreads();                          // the stage may be overwritten by the fetch after next
     }
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-        if (col0 + c >= dv) continue;
-        float* Sc = S + (size_t)(col0 + c) * dk;
+    for (int c = 0; c < NC; ++c)
 #pragma unroll
-        for (int r = 0; r < R / 4; ++r) {
-            const int d = channel(r);
-            float x[4];
-            unpack2(s[c][2 * r], x[0], x[1]);
-            unpack2(s[c][2 * r + 1], x[2], x[3]);
-            if constexpr (BY4) {
-                if (d < dk) Vec4<float>::store(Sc + d, make_float4(x[0], x[1], x[2], x[3]));
-            } else {
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (d + u < dk) Sc[d + u] = x[u];
-            }
-        }
-    }
+        for (int r = 0; r < R / 4; ++r)
+            if (col0 + c < dv) store_group<BY4>(S + (size_t)(col0 + c) * dk, channel_of<LPC>(r, li), dk, s[c][2 * r], s[c][2 * r + 1]);
 }
 
 template <int RULE, int R, int LPC, int NC, int THREADS, bool BY4, bool SPLIT>
-int launch(const float* qkv, const float* beta, const float* decay, float* state, long state_stride, const int* seq_q_start,
-           const int* seq_q_len, const int* seq_slot, int n_seqs, int rows, float* o, int G, int H, int dk, int dv,
-           cudaStream_t stream) {
+int launch(const Rows& a, int n_seqs, int rows, cudaStream_t stream) {
     using C_ = Cut<R, LPC, NC, THREADS, SPLIT>;
     auto kernel = recurrent_kernel<RULE, R, LPC, NC, THREADS, BY4, SPLIT>;
     constexpr int whole = C_::floats(C_::CH) * (int)sizeof(float), alone = 120 * 1024, most = whole > alone ? whole : alone;
@@ -475,80 +584,116 @@ int launch(const float* qkv, const float* beta, const float* decay, float* state
         if (e != cudaSuccess) return fb_fail(-2, "recurrence: cannot reserve %d bytes of shared memory: %s", most, cudaGetErrorString(e));
         fb_setup_done(configured);
     }
-    const dim3 grid(n_seqs * H, (dv + C_::COLS - 1) / C_::COLS);
-    // One token a request (decoding): a stage of one block, so that many CTAs share an SM and the states stream.  A portion
-    // that gives no SM two CTAs asks for more shared memory than two can have: launched while the kernel ahead still runs,
-    // they would else fill the SMs that are free first with two each (measured: 830 us instead of 480).
-    const int ch = rows <= n_seqs ? TB : C_::CH;
-    const bool spread = rows > n_seqs && (long)grid.x * grid.y <= fb_sm_count();
-    const size_t smem = spread ? most : C_::floats(ch) * sizeof(float);
-    fb_launch(kernel, grid, dim3(C_::ALL), smem, stream, qkv, beta, decay, state, state_stride, seq_q_start, seq_q_len, seq_slot,
-              o, G, H, dk, dv, ch);
+    const dim3 grid(n_seqs * a.H, (a.dv + C_::COLS - 1) / C_::COLS);
+    const bool round = (long)grid.x * grid.y <= fb_sm_count();
+    // A few tokens a request: stages of one block, so that many CTAs share an SM.  A portion that gives no SM two CTAs asks for
+    // more shared memory than two can have: launched while the kernel ahead still runs, they would else fill the SMs that are
+    // free first with two each (measured: 830 us instead of 480 when this kernel took 480).
+    const int ch = rows <= 4L * n_seqs ? TB : C_::CH;
+    const size_t smem = round && rows > 4L * n_seqs ? most : C_::floats(ch) * sizeof(float);
+    fb_launch(kernel, grid, dim3(C_::ALL), smem, stream, a, ch);
     return fb_check_launch("recurrence");
 }
 
+template <int RULE, int R, int LPC, int NC, bool BY4>
+int launch_one(const Rows& a, int n_seqs, cudaStream_t stream) {
+    constexpr int COLS = 128 / LPC * NC, spread = 100 * 1024;
+    auto kernel = one_token_kernel<RULE, R, LPC, NC, BY4>;
+    static bool configured[FB_MAX_DEVICES] = {};
+    if (fb_needs_setup(configured)) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, spread);
+        if (e != cudaSuccess) return fb_fail(-2, "recurrence: cannot reserve %d bytes of shared memory: %s", spread, cudaGetErrorString(e));
+        fb_setup_done(configured);
+    }
+    // Where two CTAs an SM hold them all, they ask for the shared memory that lets two in, so that they spread over the SMs
+    // (one request, linear, 16 heads: a layer 26.6 us without, 25.3 with it; eight requests 29.8 and 32.8).
+    const dim3 grid(n_seqs * a.H, (a.dv + COLS - 1) / COLS);
+    fb_launch(kernel, grid, dim3(128), (long)grid.x * grid.y <= 2L * fb_sm_count() ? spread : 0, stream, a);
+    return fb_check_launch("recurrence");
+}
+
+// What a launch gives a lane must not show in the result: for one key size, lane_sum and the exchange between lanes add in one
+// order in every instance below.
 template <int RULE>
 int run(const float* qkv, const float* beta, const float* decay, float* state, long state_stride, const int* seq_q_start,
-        const int* seq_q_len, const int* seq_slot, int n_seqs, int rows, float* o, int G, int H, int dk, int dv,
+        const int* seq_q_len, const int* seq_slot, int n_seqs, int rows, int longest, float* o, int G, int H, int dk, int dv,
         cudaStream_t stream) {
     const long C = 2L * G * dk + (long)H * dv;
     const bool by4 = dk % 4 == 0 && C % 4 == 0 && state_stride % 4 == 0 && (uintptr_t)qkv % 16 == 0 &&
                      (uintptr_t)state % 16 == 0 && (RULE == DELTA_HEAD || (uintptr_t)decay % 16 == 0);
-#define FB_RECURRENCE(R, LPC, NC, THREADS, BY4, SPLIT)                                                                     \
-    return launch<RULE, R, LPC, NC, THREADS, BY4, SPLIT>(qkv, beta, decay, state, state_stride, seq_q_start, seq_q_len, seq_slot, \
-                                                  n_seqs, rows, o, G, H, dk, dv, stream)
-#define FB_RECURRENCE_BY(R, LPC, NC)                       \
-    do {                                                   \
-        if (by4) FB_RECURRENCE(R, LPC, NC, 128, true, false); \
-        FB_RECURRENCE(R, LPC, NC, 128, false, false);      \
+    const Rows a = {qkv, beta, decay, state, state_stride, seq_q_start, seq_q_len, seq_slot, o, G, H, dk, dv};
+#define FB_ONE(R, LPC, NC) return by4 ? launch_one<RULE, R, LPC, NC, true>(a, n_seqs, stream) : launch_one<RULE, R, LPC, NC, false>(a, n_seqs, stream)
+    if (rows <= n_seqs || longest < TB) {
+        if (dk <= 16) FB_ONE(4, 4, 2);
+        if (dk <= 32) FB_ONE(4, 8, 2);
+        if (dk <= 64) FB_ONE(4, 16, 2);
+        if (dk <= 128) FB_ONE(8, 16, 2);
+        if (dk <= 256) FB_ONE(8, 32, 2);
+        if (dk <= 512) FB_ONE(16, 32, 1);
+        FB_ONE(32, 32, 1);
+    }
+#undef FB_ONE
+#define FB_RECURRENCE_OF(R, LPC, NC, THREADS, BY4, SPLIT) return launch<RULE, R, LPC, NC, THREADS, BY4, SPLIT>(a, n_seqs, rows, stream)
+#define FB_RECURRENCE(R, LPC, NC, BY4, SPLIT) FB_RECURRENCE_OF(R, LPC, NC, 128, BY4, SPLIT)
+#define FB_RECURRENCE_BY(R, LPC, NC)                  \
+    do {                                              \
+        if (by4) FB_RECURRENCE(R, LPC, NC, true, false); \
+        FB_RECURRENCE(R, LPC, NC, false, false);      \
     } while (0)
     if (dk <= 16) FB_RECURRENCE_BY(4, 4, 2);
     if (dk <= 32) FB_RECURRENCE_BY(4, 8, 2);
     if (dk <= 64) FB_RECURRENCE_BY(4, 16, 2);
-    if (dk <= 128 && by4 && rows > n_seqs) {
-        // Portions: with a decay per channel, 2,048 tokens of 32 heads of 128 x 128 take 376 us on 32 columns a CTA and 450
-        // on 16 (391 without threads of their own for the stages); 16 heads, which 32 columns spread over 64 SMs only, 373 and 288.
-        if ((long)n_seqs * H * ((dv + 15) / 16) <= fb_sm_count()) FB_RECURRENCE(8, 16, 2, 128, true, true);
-        FB_RECURRENCE(16, 8, 2, 128, true, true);
+    if (dk <= 128 && by4) {
+        // With a decay per channel, 2,048 tokens of 32 heads of 128 x 128 take 376 us on 32 columns a CTA and 450 on 16 (391
+        // without threads of their own for the stages); 16 heads, which 32 columns spread over 64 SMs only, 373 and 288.
+        // Few tokens are over before 32 columns pay: a layer of 64 takes 75.6 us on 16, 79.5 on 32 (linear, 32 heads), 17 take 80 and 84.
+        if (rows <= 128 || (long)n_seqs * H * ((dv + 15) / 16) <= fb_sm_count()) FB_RECURRENCE(8, 16, 2, true, true);
+        FB_RECURRENCE(16, 8, 2, true, true);
     }
-    if (dk <= 128) FB_RECURRENCE_BY(16, 8, 2);
+    if (dk <= 128) FB_RECURRENCE(16, 8, 2, false, false);
     if (dk <= 256) FB_RECURRENCE_BY(16, 16, 2);
-    if (dk <= 512) FB_RECURRENCE_BY(16, 32, 2);
+    if (dk <= 512) {
+        // (a stage fills more than half of an SM's shared memory: more CTAs than SMs are better off with twice the columns each;
+        // 1,024 tokens of 32 heads of 512 x 64, a decay per channel: 507 us, 807 on 8 columns)
+        if (by4 && (long)n_seqs * H * ((dv + 7) / 8) > fb_sm_count()) FB_RECURRENCE_OF(16, 32, 2, 256, true, false);
+        FB_RECURRENCE_BY(16, 32, 2);
+    }
     FB_RECURRENCE_BY(32, 32, 1);
 #undef FB_RECURRENCE_BY
 #undef FB_RECURRENCE
+#undef FB_RECURRENCE_OF
 }
 
 }  // namespace
 
-// rows: tokens of the step over all requests.
+// rows: tokens of the step over all requests; longest: of the request that has most (rows where that is not known).
 FB_API int fb_gdr_recurrent(const float* qkv, const float* beta, const float* decay, float* state, long long state_stride,
-                            const int* seq_q_start, const int* seq_q_len, const int* seq_slot, int n_seqs, int rows, float* o,
-                            int G, int H, int dk, int dv, cudaStream_t stream) {
+                            const int* seq_q_start, const int* seq_q_len, const int* seq_slot, int n_seqs, int rows, int longest,
+                            float* o, int G, int H, int dk, int dv, cudaStream_t stream) {
     FB_REQUIRE(n_seqs >= 0 && rows >= 0 && G > 0 && H > 0 && H % G == 0 && dk > 0 && dv > 0, "gated delta: bad sizes");
     FB_REQUIRE(dk <= 1024, "gated delta: key size %d is larger than 1024", dk);
     if (n_seqs == 0) return 0;
-    return run<DELTA_HEAD>(qkv, beta, decay, state, (long)state_stride, seq_q_start, seq_q_len, seq_slot, n_seqs, rows, o, G, H,
+    return run<DELTA_HEAD>(qkv, beta, decay, state, (long)state_stride, seq_q_start, seq_q_len, seq_slot, n_seqs, rows, longest, o, G, H,
                            dk, dv, stream);
 }
 
 // decay: float32 [rows][H][dk], one factor per head and key channel; the rest as in fb_gdr_recurrent.
 FB_API int fb_gdr_channel_recurrent(const float* qkv, const float* beta, const float* decay, float* state,
                                     long long state_stride, const int* seq_q_start, const int* seq_q_len, const int* seq_slot,
-                                    int n_seqs, int rows, float* o, int G, int H, int dk, int dv, cudaStream_t stream) {
+                                    int n_seqs, int rows, int longest, float* o, int G, int H, int dk, int dv, cudaStream_t stream) {
     FB_REQUIRE(n_seqs >= 0 && rows >= 0 && G > 0 && H > 0 && H % G == 0 && dk > 0 && dv > 0, "gated delta: bad sizes");
     FB_REQUIRE(dk <= 1024, "gated delta: key size %d is larger than 1024", dk);
     if (n_seqs == 0) return 0;
-    return run<DELTA_CHANNEL>(qkv, beta, decay, state, (long)state_stride, seq_q_start, seq_q_len, seq_slot, n_seqs, rows, o, G,
+    return run<DELTA_CHANNEL>(qkv, beta, decay, state, (long)state_stride, seq_q_start, seq_q_len, seq_slot, n_seqs, rows, longest, o, G,
                               H, dk, dv, stream);
 }
 
 FB_API int fb_gla_recurrent(const float* qkv, const float* decay, float* state, long long state_stride, const int* seq_q_start,
-                            const int* seq_q_len, const int* seq_slot, int n_seqs, int rows, float* o, int H, int dk, int dv,
-                            cudaStream_t stream) {
+                            const int* seq_q_len, const int* seq_slot, int n_seqs, int rows, int longest, float* o, int H, int dk,
+                            int dv, cudaStream_t stream) {
     FB_REQUIRE(n_seqs >= 0 && rows >= 0 && H > 0 && dk > 0 && dv > 0, "linear attention: bad sizes");
     FB_REQUIRE(dk <= 1024, "linear attention: key size %d is larger than 1024", dk);
     if (n_seqs == 0) return 0;
-    return run<LINEAR>(qkv, nullptr, decay, state, (long)state_stride, seq_q_start, seq_q_len, seq_slot, n_seqs, rows, o, H, H,
+    return run<LINEAR>(qkv, nullptr, decay, state, (long)state_stride, seq_q_start, seq_q_len, seq_slot, n_seqs, rows, longest, o, H, H,
                        dk, dv, stream);
 }

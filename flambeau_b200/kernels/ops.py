@@ -1121,6 +1121,11 @@ def gdr_prepare(proj, conv_w, taps: int, a_log, dt_bias, state, tail_off: int, b
                                float(unit_eps), _stream()), "gdr_prepare")
 
 
+def _longest(batch, qkv) -> int:
+    """Tokens of the request that brings most of them (all of the step's where the batch does not say)."""
+    return int(getattr(batch, "max_q_len", qkv.shape[0]))
+
+
 def gdr_recurrent(qkv, beta, decay, state, batch, o, G: int, H: int, dk: int, dv: int) -> None:
     """S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q over the step's tokens of every request, the state
     [H][dk][dv] at the start of the request's slot."""
@@ -1129,8 +1134,8 @@ def gdr_recurrent(qkv, beta, decay, state, batch, o, G: int, H: int, dk: int, dv
         raise KernelError("gated delta: bad output or state")
     check(lib().fb_gdr_recurrent(qkv.data_ptr(), beta.data_ptr(), decay.data_ptr(), state.data_ptr(), state.stride(0),
                                  batch.seq_q_start_d.data_ptr(), batch.seq_q_len_d.data_ptr(),
-                                 batch.seq_slot_d.data_ptr(), batch.n_seqs, int(qkv.shape[0]), o.data_ptr(),
-                                 G, H, dk, dv, _stream()), "gdr_recurrent")
+                                 batch.seq_slot_d.data_ptr(), batch.n_seqs, int(qkv.shape[0]), _longest(batch, qkv),
+                                 o.data_ptr(), G, H, dk, dv, _stream()), "gdr_recurrent")
 
 
 def gdr_channel_recurrent(qkv, beta, decay, state, batch, o, G: int, H: int, dk: int, dv: int) -> None:
@@ -1144,8 +1149,8 @@ def gdr_channel_recurrent(qkv, beta, decay, state, batch, o, G: int, H: int, dk:
         raise KernelError("gated delta: bad output, decay or state")
     check(lib().fb_gdr_channel_recurrent(qkv.data_ptr(), beta.data_ptr(), decay.data_ptr(), state.data_ptr(),
                                          state.stride(0), batch.seq_q_start_d.data_ptr(), batch.seq_q_len_d.data_ptr(),
-                                         batch.seq_slot_d.data_ptr(), batch.n_seqs, int(n), o.data_ptr(),
-                                         G, H, dk, dv, _stream()), "gdr_channel_recurrent")
+                                         batch.seq_slot_d.data_ptr(), batch.n_seqs, int(n), _longest(batch, qkv),
+                                         o.data_ptr(), G, H, dk, dv, _stream()), "gdr_channel_recurrent")
 
 
 LOW_RANK_FUNCTIONS = {"plain": 0, "sigmoid": 1, "decay": 2}
@@ -1378,9 +1383,8 @@ def gla_recurrent(qkv, decay, state, batch, o, H: int, dk: int, dv: int) -> None
         raise KernelError("linear attention: bad output or state")
     check(lib().fb_gla_recurrent(qkv.data_ptr(), decay.data_ptr(), state.data_ptr(), state.stride(0),
                                  batch.seq_q_start_d.data_ptr(), batch.seq_q_len_d.data_ptr(),
-                                 batch.seq_slot_d.data_ptr(), batch.n_seqs, int(qkv.shape[0]), o.data_ptr(), H, dk, dv,
-                                 _stream()),
-          "gla_recurrent")
+                                 batch.seq_slot_d.data_ptr(), batch.n_seqs, int(qkv.shape[0]), _longest(batch, qkv),
+                                 o.data_ptr(), H, dk, dv, _stream()), "gla_recurrent")
 
 
 # ---------------------------------------------------------------------------

@@ -70,6 +70,7 @@ def run(rule, qkv, beta, decay, state, lengths, slots, sizes):
     from flambeau_b200.kernels import ops
     dk, dv, H, G = sizes
     batch, st, o = fake_batch(lengths, slots), state.clone(), torch.empty(sum(lengths), H * dv, device=DEV)
+    batch.max_q_len = max(lengths)
     if rule == "linear":
         ops.gla_recurrent(qkv, decay, st, batch, o, H, dk, dv)
     else:
@@ -94,7 +95,7 @@ def test_a_request_has_the_same_bits_whatever_shares_its_step(rule, sizes):
     state = torch.randn(len(lengths), H * dv * dk, generator=gen, device=DEV)
     whole, st_whole = run(rule, qkv, beta, decay, state, lengths, list(range(len(lengths))), sizes)
     for i, length in enumerate(lengths):
-        for others in ([], [0], [3], [4, 0]):
+        for others in ([], [0], [3], [4, 0], [2, 5]):
             who = [i] + [x for x in others if x != i]
             rows = torch.cat([torch.arange(starts[x], starts[x] + lengths[x], device=DEV) for x in who])
             o, st = run(rule, qkv[rows], beta[rows], decay[rows], state, [lengths[x] for x in who], who, sizes)
