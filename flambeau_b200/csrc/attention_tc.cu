@@ -28,8 +28,9 @@
 //
 // Heads of 256 (one row tile: O takes 256 columns): a tile is fetched once and serves as K and as V, its slot is free when
 // its product is through.  An MMA of 64 columns takes as long as one of 128 (62 to 72 cycles), so a key tile costs 16 x 65 for
-// the scores and 2 x 4 x 130 for the product with both parts of the weights, which bounds it.  2,048 tokens of 32 heads of
-// 256 over one latent row: 570 us on the mma.sync kernel (7 % of the tensor pipes' rate), 153 here.
+// the scores and 3 x 4 x 130 for the product with the three parts of the weights: 75 us of 2,048 tokens of 32 heads of 256 over
+// one latent row, which take about 170 (570 on the mma.sync kernel, 153 with two parts).  The softmax bounds it, one thread a
+// row: a quarter more MMAs, the third part's, cost a layer 1 to 4 %.
 //
 // Decoded tokens over latents (SPLIT): the rows of a sequence are fewer than a row tile, which costs a key tile no more; a CTA
 // takes a stretch of a sequence's key tiles and leaves its rows' maximum, sum and unnormalised O, and a warp per row merges them.
@@ -37,7 +38,8 @@
 // Differential attention (two score maps of 64 a head over values of 128): the row tiles are the two maps of the same 128
 // rows, each with its column block of Q and K and both on one V tile.  At the end the threads of both take half of the
 // columns each, read both maps' O from tensor memory and form the difference, its norm and the gate.  A key tile costs 8 x 65
-// for the scores and 16 x 65 for the products.  2,048 tokens of 32 heads: 373 us on the mma.sync kernel, 141 here.
+// for the scores and 16 x 65 for the products, 45 us of 2,048 tokens of 32 heads, which take about 153 (373 on the mma.sync
+// kernel, 141 with a reference that lags): the softmax threads again.
 //
 // Formulas: crates/kernels-hip/src/kernels/attention_prefill_flash_tile_f16.cu:73-213 (tile + online softmax).
 #include "attention_common.cuh"
