@@ -248,8 +248,11 @@ __device__ __forceinline__ void few_tokens(const Rows& a, int seq, int head, int
 template <int RULE, int R, int LPC, int NC, bool BY4>
 __global__ void __launch_bounds__(128)
 one_token_kernel(const Rows a) {
+    // The kernels behind are let in when the one ahead has ended, not before: CTAs of the output product, which hold an SM's
+    // shared memory for their weights, else take the SMs that this kernel has not filled (three decoded tokens, a decay per
+    // channel, 16 heads: a layer 37.7 us so, 35.2 in this order).  Portions are slower with it (linear, 700 tokens 279 and 332).
     fb_pdl_wait();
-    fb_pdl_launch_dependents();                                  // (not ahead of the wait: see recurrent_kernel)
+    fb_pdl_launch_dependents();
     constexpr int PW = 32 / LPC, COLS = 128 / LPC * NC;
     const int seq = blockIdx.x / a.H, head = blockIdx.x - seq * a.H;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -261,16 +264,13 @@ one_token_kernel(const Rows a) {
 template <int RULE, int R, int LPC, int NC, int THREADS, bool BY4, bool SPLIT>
 __global__ void __launch_bounds__(SPLIT ? 2 * THREADS : THREADS)
 recurrent_kernel(const Rows a_, int ch) {
-    // The kernels behind are let in when the one ahead has ended, not before: CTAs of the output product, which hold an SM's
-    // shared memory for their weights, else take the SMs that this kernel has not filled (three decoded tokens, a decay per
-    // channel, 16 heads: a layer 37.7 us so, 35.2 in this order; 17 tokens 49.1 and 45.5).
     const float* __restrict__ qkv = a_.qkv;
     const float* __restrict__ beta = a_.beta;
     const float* __restrict__ decay = a_.decay;
     float* __restrict__ o = a_.o;
     const int G = a_.G, H = a_.H, dk = a_.dk, dv = a_.dv;
-    fb_pdl_wait();
     fb_pdl_launch_dependents();
+    fb_pdl_wait();
     using C_ = Cut<R, LPC, NC, THREADS, SPLIT>;
     constexpr int DKP = C_::DKP, COLS = C_::COLS, WARPS = THREADS / 32;
     constexpr bool DELTA = RULE != LINEAR;
