@@ -13,9 +13,10 @@
 // rows joins them in its output rows; where that gives too few CTAs each takes some, leaves every stretch's maximum, sum and
 // unnormalised output, and a warp per row joins them.
 //
-// What bounds it: multiply-adds over portions (2 x 128 x 128 a row and tile of 32 keys at heads of 128; the scores read 24
+// What bounds it: multiply-adds over portions (2 x 32 x 128 a row and tile of 32 keys at heads of 128; the scores read 24
 // cycles of shared memory for 64 multiply-adds of a warp), the stream of keys and values for decoded tokens.  301 tokens
-// behind 500 (32 heads of 128 on 8): 3,340 us with a warp a (row, head), about 140 here.
+// behind 500 (32 heads of 128 on 8), launched behind itself: 3,330 us with a warp a (row, head), 195 here; 8 decoded tokens
+// of 8,000 keys 7,700 and 312.  (Stretches cut by the step's rows took 192 and 215: the latter in one round of CTAs.)
 //
 // Sums run in float32 throughout; sinks, caps, gates, slopes and kept first keys as in attention_simt.cu.
 #include <type_traits>
