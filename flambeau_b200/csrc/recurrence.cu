@@ -606,7 +606,8 @@ int launch_one(const Rows& a, int n_seqs, cudaStream_t stream) {
         fb_setup_done(configured);
     }
     // Where two CTAs an SM hold them all, they ask for the shared memory that lets two in, so that they spread over the SMs
-    // (one request, linear, 16 heads: a layer 26.6 us without, 25.3 with it; eight requests 29.8 and 32.8).
+    // (one request, a decay per channel, 32 heads: a layer 62.4 us without, 58.0 with it, 59.2 with the kernels behind held back
+    // as well; eight requests 68.4 and 77.5).
     const dim3 grid(n_seqs * a.H, (a.dv + COLS - 1) / COLS);
     fb_launch(kernel, grid, dim3(128), (long)grid.x * grid.y <= 2L * fb_sm_count() ? spread : 0, stream, a);
     return fb_check_launch("recurrence");
