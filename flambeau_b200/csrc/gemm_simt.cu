@@ -1,8 +1,9 @@
 // out[M,N] = A[M,K] * W[N,K]^T with float32 FMA accumulation on the CUDA cores.
 //
-// This is the matrix product of the true 32-bit path (no tensor cores: the
-// tensor pipes have no float32 x float32 mode) and the fallback of the
-// bfloat16 path for shapes the tensor-core kernel refuses.  Each output
+// This is the matrix product of the true 32-bit path for the shapes that
+// gemm_f32_tc.cu does not take (fewer than 64 outputs or 512 inputs, weight
+// rows off 16-byte borders) and the fallback of the bfloat16 path for shapes
+// the tensor-core kernel refuses.  Each output
 // element is summed in one thread in ascending k (even and odd k on their own
 // where 16-byte copies fetch the rows), so the result of a row does not depend
 // on how many rows the call has.

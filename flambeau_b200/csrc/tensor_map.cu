@@ -28,10 +28,10 @@ EncodeTiledFn encode_fn() {
 }
 
 struct MapKey {
-    const void* ptr; long rows, cols, ld; int box_cols, box_rows;
+    const void* ptr; long rows, cols, ld; int box_cols, box_rows, elem_bytes;
     bool operator==(const MapKey& o) const {
         return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_cols == o.box_cols &&
-               box_rows == o.box_rows;
+               box_rows == o.box_rows && elem_bytes == o.elem_bytes;
     }
 };
 struct MapKeyHash {
@@ -41,34 +41,43 @@ struct MapKeyHash {
         h = h * 1000003u ^ (size_t)k.cols;
         h = h * 1000003u ^ (size_t)k.ld;
         h = h * 1000003u ^ (size_t)k.box_cols;
+        h = h * 1000003u ^ (size_t)k.elem_bytes;
         return h * 1000003u ^ (size_t)k.box_rows;
     }
 };
 
 }  // namespace
 
-int fb_tensor_map_bf16(CUtensorMap* out, const void* ptr, long rows, long cols, long ld, int box_cols, int box_rows) {
+int fb_tensor_map_rows(CUtensorMap* out, const void* ptr, int elem_bytes, long rows, long cols, long ld, int box_cols,
+                       int box_rows) {
     static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
     static std::mutex mu;
-    const MapKey key{ptr, rows, cols, ld, box_cols, box_rows};
+    const MapKey key{ptr, rows, cols, ld, box_cols, box_rows, elem_bytes};
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find(key);
     if (it != cache.end()) { *out = it->second; return 0; }
     EncodeTiledFn fn = encode_fn();
     if (!fn) return fb_fail(-3, "tensor map: the driver does not provide cuTensorMapEncodeTiled");
-    if (box_cols * 2 != 128 || box_rows < 1 || box_rows > 256)
+    const int row_bytes = box_cols * elem_bytes;
+    if ((elem_bytes != 2 && elem_bytes != 4) || (row_bytes != 128 && row_bytes != 64) || box_rows < 1 || box_rows > 256)
         return fb_fail(-3, "tensor map: box of %d x %d elements is not supported", box_rows, box_cols);
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+    const cuuint64_t strides[1] = {(cuuint64_t)ld * elem_bytes};
     const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
     const cuuint32_t elem[2] = {1, 1};
-    CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, elem,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    CUresult r = fn(out, elem_bytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+                    const_cast<void*>(ptr), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    row_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fb_fail(-3, "tensor map: cuTensorMapEncodeTiled failed with code %d", (int)r);
     if (cache.size() > 8192) cache.clear();
     cache.emplace(key, *out);
     return 0;
+}
+
+int fb_tensor_map_bf16(CUtensorMap* out, const void* ptr, long rows, long cols, long ld, int box_cols, int box_rows) {
+    if (box_cols * 2 != 128) return fb_fail(-3, "tensor map: box of %d x %d elements is not supported", box_rows, box_cols);
+    return fb_tensor_map_rows(out, ptr, 2, rows, cols, ld, box_cols, box_rows);
 }
 
 // The same encoding without the cache: nothing is kept and no host memory is taken, for callers that must not

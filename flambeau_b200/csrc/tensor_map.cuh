@@ -7,7 +7,12 @@
 // with the 128-byte swizzle (box_cols * 2 bytes must be 128).  Returns 0, or a negative code after fb_fail().
 int fb_tensor_map_bf16(CUtensorMap* out, const void* ptr, long rows, long cols, long ld, int box_cols, int box_rows);
 
-// As above, but nothing is cached and no host memory is taken.
+// The same for float32 (elem_bytes 4) or bfloat16 (2) rows in boxes whose rows are 128 bytes (128-byte swizzle) or 64 bytes
+// (64-byte swizzle) long.
+int fb_tensor_map_rows(CUtensorMap* out, const void* ptr, int elem_bytes, long rows, long cols, long ld, int box_cols,
+                       int box_rows);
+
+// As fb_tensor_map_bf16, but nothing is cached and no host memory is taken.
 int fb_tensor_map_bf16_uncached(CUtensorMap* out, const void* ptr, long rows, long cols, long ld, int box_cols,
                                 int box_rows);
 

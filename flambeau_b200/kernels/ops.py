@@ -620,6 +620,34 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: torch.T
     return _SPLITS_USED.value if slabs is not None else 1
 
 
+def f32_tc_supported(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
+    """Whether the tcgen05 product of float32 operands takes these: enough features and depth to fill its tiles, weight
+    rows that start on 16-byte borders.  The rule looks at the weights and the depth alone, never at the number of rows:
+    which kernel multiplies a row must not depend on its company."""
+    return (a.dtype == w.dtype == out.dtype == torch.float32 and a.dim() == 2 and w.dim() == 2 and out.dim() == 2
+            and a.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1 and w.shape[0] >= 64 and w.shape[1] >= 512
+            and w.shape[1] % 4 == 0 and w.stride(0) % 4 == 0 and w.data_ptr() % 16 == 0)
+
+
+def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: torch.Tensor, ws) -> None:
+    """out[M,N] = a[M,K] @ w[N,K]^T in float32 on the tensor cores: every float32 as three bfloat16 numbers (see
+    csrc/gemm_f32_tc.cu).  `ws` is the step's arena, which holds the parts of `a` meanwhile."""
+    _cuda(a, w, out, status)
+    M, K = a.shape
+    N = w.shape[0]
+    if w.shape[1] != K or out.shape[0] != M or out.shape[1] != N:
+        raise KernelError(f"gemm: shapes a{tuple(a.shape)} w{tuple(w.shape)} out{tuple(out.shape)} do not agree")
+    if not (a.dtype == w.dtype == out.dtype == torch.float32):
+        raise KernelError("gemm_f32_tc: operands must be float32")
+    partials, counters = _SplitScratch.get(a.device)
+    with ws.scope():
+        parts = ws.alloc((3 * M * ((K + 31) // 32 * 32),), torch.bfloat16)
+        check(lib().fb_gemm_f32_tc(a.data_ptr(), _rows(a), w.data_ptr(), _rows(w), out.data_ptr(), _rows(out), M, N, K,
+                                   parts.data_ptr(), parts.numel(), partials.data_ptr(), partials.numel(),
+                                   counters.data_ptr(), counters.numel(), status.data_ptr(), _stream()),
+              "gemm_f32_tc", (M, N, K))
+
+
 def gemm_tc_add(a: torch.Tensor, w: torch.Tensor, acc: torch.Tensor, status: torch.Tensor, max_slabs: int = 1) -> bool:
     """acc[M,N] += a[M,K] @ w[N,K]^T in float32, where the product is one the two-SM tensor-core kernel takes in
     whole tiles (hundreds of rows, and no split of K would be chosen although `max_slabs` slabs could be had): each
@@ -806,10 +834,12 @@ def grouped_linear(a: torch.Tensor, row_index, w: torch.Tensor, tile_group: torc
 
 
 def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, ctx=None) -> None:
-    """out = a @ w^T with the kernel that fits the dtypes and the shape: the tcgen05 kernel for bfloat16
-    operands it can fetch by TMA, the float32-FMA kernel for everything else (all of the 32-bit mode)."""
+    """out = a @ w^T with the kernel that fits the dtypes and the shape: the tcgen05 kernels for bfloat16 and for
+    float32 operands they can fetch by TMA, the float32-FMA kernel for everything else."""
     if ctx is not None and tc_supported(a, w, out):
         gemm_tc(a, w, out, ctx.runtime.status)
+    elif ctx is not None and f32_tc_supported(a, w, out):
+        gemm_f32_tc(a, w, out, ctx.runtime.status, ctx.ws)
     else:
         gemm_simt(a, w, out)
 
