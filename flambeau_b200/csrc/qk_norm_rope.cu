@@ -25,6 +25,16 @@ __device__ __forceinline__ float qkr_slab_sum(const float* row, int c, int n_par
     return v;
 }
 
+// Which multiplications join an addition is written out, so that the kernels of few rows and of portions give the same bits.
+__device__ __forceinline__ float qkr_squares(float4 v) {
+    return __fmaf_rn(v.w, v.w, __fmaf_rn(v.z, v.z, __fmaf_rn(v.y, v.y, __fmul_rn(v.x, v.x))));
+}
+// v turned with its partner o by the angle's (cosine, signed sine).
+__device__ __forceinline__ float4 qkr_turn(float4 v, float4 o, float4 cs, float4 sn) {
+    return make_float4(__fmaf_rn(v.x, cs.x, __fmul_rn(o.x, sn.x)), __fmaf_rn(v.y, cs.y, __fmul_rn(o.y, sn.y)),
+                       __fmaf_rn(v.z, cs.z, __fmul_rn(o.z, sn.z)), __fmaf_rn(v.w, cs.w, __fmul_rn(o.w, sn.w)));
+}
+
 template <typename TW, typename T>
 __global__ void __launch_bounds__(1024)
 qk_norm_rope_kv_write_kernel(const float* __restrict__ proj, long proj_stride, int n_partials, long partial_stride,
@@ -257,7 +267,7 @@ qk_norm_rope_heads_kernel(const float* __restrict__ proj, long proj_stride, int 
             float s = 0.0f;
 #pragma unroll
             for (int i = 0; i < NV; ++i)
-                s += x[j][i].x * x[j][i].x + x[j][i].y * x[j][i].y + x[j][i].z * x[j][i].z + x[j][i].w * x[j][i].w;
+                s += qkr_squares(x[j][i]);
             const float f = 1.0f / sqrtf(fb_warp_sum(s) / (float)hd + eps);
 #pragma unroll
             for (int i = 0; i < NV; ++i) {
@@ -271,10 +281,7 @@ qk_norm_rope_heads_kernel(const float* __restrict__ proj, long proj_stride, int 
                 float4 o;
                 o.x = __shfl_sync(0xffffffffu, x[j][0].x, mate); o.y = __shfl_sync(0xffffffffu, x[j][0].y, mate);
                 o.z = __shfl_sync(0xffffffffu, x[j][0].z, mate); o.w = __shfl_sync(0xffffffffu, x[j][0].w, mate);
-                if (turns) {
-                    x[j][0].x = x[j][0].x * cs.x + o.x * sn.x; x[j][0].y = x[j][0].y * cs.y + o.y * sn.y;
-                    x[j][0].z = x[j][0].z * cs.z + o.z * sn.z; x[j][0].w = x[j][0].w * cs.w + o.w * sn.w;
-                }
+                if (turns) x[j][0] = qkr_turn(x[j][0], o, cs, sn);
             }
         } else if (half > 0) {
             float* mine = sh + (size_t)warp * hd;
@@ -305,6 +312,118 @@ qk_norm_rope_heads_kernel(const float* __restrict__ proj, long proj_stride, int 
         for (int i = 0; i < NV; ++i) {
             const int c = lane + 32 * i;
             if (c < nvec) Vec4<T>::store(dst + 4 * c, x[j][i]);
+        }
+    }
+}
+
+// Portions with heads of 32, 64 or 128: one CTA a row, whose q and k (and v) columns lie flat over the warps, U groups of four
+// columns a thread, so LANES = hd / 4 neighbouring lanes hold a head and no lane is idle whatever the head's size.  A thread's
+// columns lie 128 apart: they have one place within their heads, hence one weight and one angle.  The arithmetic
+// (and the order of the norm's sums) is the kernel's above, whose heads of a warp each cost it the index arithmetic of a head,
+// in 64 bits: at 2,048 rows of 64 + 16 maps of 64 and 8 values of 128 it issued 118 instructions per number and took 69 us,
+// this one 45 and 38 us (75 MB, 11 at the copy rate; the factors' square roots and divisions are the largest part).  A few
+// rows stay with a warp a head: there one CTA a row leaves SMs idle (a layer of 70 rows: 39.8 us by heads, 35.0 by rows).
+template <typename TW, typename T, int LANES, int U>
+__global__ void __launch_bounds__(384, 2)
+qk_norm_rope_rows_kernel(const float* __restrict__ proj, long proj_stride, int n_partials, long partial_stride,
+                         const TW* __restrict__ bias, const TW* __restrict__ q_weight,
+                         const TW* __restrict__ k_weight, float eps, float weight_offset, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                         int half, T* __restrict__ q_out, long q_out_stride, const int* __restrict__ positions,
+                         const int* __restrict__ row_seq, const int* __restrict__ block_table, int table_stride,
+                         const int* __restrict__ table_base, int table_head, T* __restrict__ k_pool,
+                         T* __restrict__ v_pool, int page_size, int n_pages, int nh, int nkv, int maps,
+                         int vd, int v_off, int v_is_k, int write_kv, int* status) {
+    fb_pdl_launch_dependents();
+    constexpr int hd = 4 * LANES;
+    const int row = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
+    const int nv = nkv / maps, qw = nh * hd, kw = write_kv ? nkv * hd : 0, vw = write_kv && !v_is_k ? nv * vd : 0;
+    const int d = 4 * (tid % LANES);                   // place within a head of q or k
+    float4 wq, wk;
+    if (q_weight) {
+        wq = Vec4<TW>::load(q_weight + d);
+        wk = Vec4<TW>::load(k_weight + d);
+        wq.x += weight_offset; wq.y += weight_offset; wq.z += weight_offset; wq.w += weight_offset;
+        wk.x += weight_offset; wk.y += weight_offset; wk.z += weight_offset; wk.w += weight_offset;
+    }
+    fb_pdl_wait();
+    const float* pr = proj + (size_t)row * proj_stride;
+    const int p = write_kv ? positions[row] : 0, seq = write_kv ? row_seq[row] : 0;
+    const bool turns = d < 2 * half, second = d >= half;
+    float4 cs = make_float4(0.f, 0.f, 0.f, 0.f), sn = cs;
+    if (turns) {
+        const size_t at = (size_t)row * half + d - (second ? half : 0);
+        cs = Vec4<float>::load(cos_t + at);
+        sn = Vec4<float>::load(sin_t + at);
+        if (!second) { sn.x = -sn.x; sn.y = -sn.y; sn.z = -sn.z; sn.w = -sn.w; }
+    }
+    const int mate = ((tid & 31) + (second ? -(half >> 2) : half >> 2)) & 31;
+    size_t cache_row = 0;                              // + head * page_size: the token's row in a pool
+    bool cached = false;
+    // columns of q and k, then of v; a warp takes U stretches of 128 side by side, so that the warps of queries do not wait for
+    // the way to the token's page (the same number of steps for every thread: warps meet in the norm's sums)
+    const int all = qw + kw + vw, per_step = 128, per_pass = 4 * U * nt;
+    for (int c0 = 128 * U * (tid >> 5) + 4 * (tid & 31); c0 - 4 * (tid & 31) < all; c0 += per_pass) {
+        float4 x[U];
+        int at[U];                                     // the column within the projection's row
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = c0 + u * per_step;
+            at[u] = c < qw + kw ? c : v_off + c - (qw + kw);
+            x[u] = c < all ? Vec4<float>::load(pr + at[u]) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if (write_kv && c0 - 4 * (tid & 31) + U * per_step > qw) {          // (warp-uniform)
+            const int entry = fb_table_column(p / page_size, table_base ? table_base[seq] : 0, table_head);
+            const int page = (entry >= 0 && entry < table_stride) ? block_table[(size_t)seq * table_stride + entry] : -1;
+            cached = page >= 0 && page < n_pages;
+            if (!cached && (tid & 31) == 0) atomicOr(status, FB_STATUS_BAD_PAGE);
+            cache_row = (size_t)page * nv * page_size + (p % page_size);
+        }
+        if (bias) {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (c0 + u * per_step < all) {
+                    const float4 b = Vec4<TW>::load(bias + at[u]);
+                    x[u].x += b.x; x[u].y += b.y; x[u].z += b.z; x[u].w += b.w;
+                }
+        }
+        for (int s = 1; s < n_partials; ++s)
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (c0 + u * per_step < all) {
+                    const float4 m = Vec4<float>::load(pr + (size_t)s * partial_stride + at[u]);
+                    x[u].x += m.x; x[u].y += m.y; x[u].z += m.z; x[u].w += m.w;
+                }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = c0 + u * per_step;
+            if (c - 4 * (tid & 31) >= all) break;      // (a warp's columns: 128 from here on)
+            float4 v = x[u];
+            const bool is_q = c < qw, is_v = c >= qw + kw;
+            if (is_v || (v_is_k && !is_q)) {
+                const int e = is_v ? c - (qw + kw) : c - qw, g = e / vd;
+                if (cached && c < all) Vec4<T>::store(v_pool + (cache_row + (size_t)g * page_size) * vd + e - g * vd, v);
+            }
+            if (c - 4 * (tid & 31) >= qw + kw) continue;                 // values alone in this warp
+            if (q_weight) {
+                float s = qkr_squares(v);
+#pragma unroll
+                for (int o = LANES / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                const float f = 1.0f / sqrtf(s / (float)hd + eps);
+                const float4 w = is_q ? wq : wk;
+                v.x *= f * w.x; v.y *= f * w.y; v.z *= f * w.z; v.w *= f * w.w;
+            }
+            if (half > 0) {
+                float4 o;
+                o.x = __shfl_sync(0xffffffffu, v.x, mate); o.y = __shfl_sync(0xffffffffu, v.y, mate);
+                o.z = __shfl_sync(0xffffffffu, v.z, mate); o.w = __shfl_sync(0xffffffffu, v.w, mate);
+                if (turns) v = qkr_turn(v, o, cs, sn);
+            }
+            if (is_q) {
+                Vec4<T>::store(q_out + (size_t)row * q_out_stride + c, v);
+            } else if (!is_v && cached) {
+                const int h = (c - qw) / hd, g = maps == 1 ? h : h / maps;
+                Vec4<T>::store(k_pool + ((cache_row + (size_t)g * page_size) * maps + (h - g * maps)) * hd + d, v);
+            }
         }
     }
 }
@@ -344,6 +463,17 @@ FB_API int fb_qk_norm_rope_kv_write(const float* proj, long long proj_stride, in
         aligned(q_weight, 4 * wsize) && aligned(k_weight, 4 * wsize) && aligned(bias, 4 * wsize)) {
         if (scope == FB_QK_NORM_NONE) q_weight = k_weight = nullptr;
         const int v_is_k = v_off == k_off ? 1 : 0;
+        if (n > 64 && half % 4 == 0 && (hd == 32 || hd == 64 || hd == 128)) {
+            // (threads: the row's columns in steps of four groups of four a thread, so that a common row is one step)
+            const long cols = (long)nh * hd + (write_kv ? (long)nkv * hd + (v_is_k ? 0 : (long)nv * vd) : 0);
+            const long steps = (cols + 6143) / 6144, threads = ((cols + 16 * steps - 1) / (16 * steps) + 31) / 32 * 32;
+#define FB_QKR_ROWS(LANES_)                                                                                                       FB_DISPATCH_DTYPE(w_dtype, TW, FB_DISPATCH_DTYPE(out_dtype, T,                                                            (fb_launch((qk_norm_rope_rows_kernel<TW, T, LANES_, 4>), dim3(n), dim3((unsigned)threads), 0, stream,                            proj, (long)proj_stride, n_partials, (long)partial_stride, (const TW*)bias, (const TW*)q_weight, (const TW*)k_weight,                            eps, weight_offset, cos_t, sin_t, half, (T*)q_out, (long)q_out_stride, positions, row_seq, block_table,                            table_stride, table_base, table_head, (T*)k_pool, (T*)v_pool, page_size, n_pages, nh, nkv, maps, vd,                            v_off, v_is_k, write_kv, status))))
+            if (hd == 32) FB_QKR_ROWS(8);
+            else if (hd == 64) FB_QKR_ROWS(16);
+            else FB_QKR_ROWS(32);
+#undef FB_QKR_ROWS
+            return fb_check_launch("qk_norm_rope_kv_write");
+        }
         // (a few rows: one head a warp, so that the heads spread over the device; a portion: four, for loads in flight)
         const int hpw = n <= 64 ? 1 : 4;
         const int per_row = nh + (write_kv ? (v_is_k ? nkv : nkv + nv) : 0);
