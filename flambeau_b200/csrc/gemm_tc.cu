@@ -474,6 +474,11 @@ static int gemm_tc_grouped(const void* X, long long lda, const void* W, long lon
     else FB_REQUIRE(ldo >= N, "gemm_tc_grouped: a row stride is shorter than its row");
     FB_REQUIRE((long long)groups * N < 2147483647LL, "gemm_tc_grouped: too many weight rows");
     if (M == 0) return 0;
+    if (tile == 32 && (o_dtype == FB_F32 || o_dtype == FB_BF16)) {
+        const int rc = fb_launch_gemm_pair_grouped(X, (long)lda, W, (long)ldw, groups, tile_group, out, o_dtype, (long)ldo, M, N, K, gated, act,
+                                                   status, stream);
+        if (rc <= 0) return rc;
+    }
     CUtensorMap mw, mx;
     int rc = fb_tensor_map_bf16(&mw, W, (long long)groups * N, K, (long)ldw, BK, BM);
     if (rc) return rc;

@@ -35,6 +35,10 @@ constexpr int P_TMEM_COLS = 2 * PBN;
 constexpr int P_OUT_TOKENS = 16;
 constexpr int P_OUT_BYTES = P_OUT_TOKENS * PBM * 4;
 constexpr int P_SMEM_BYTES = P_STAGES * P_STAGE_BYTES + 1024 + 256 + 4 * P_OUT_BYTES;
+constexpr int P_GROUP_TILE = 32;       // rows of a tile of the grouped form
+constexpr int P_GROUP_BOX = 16;        // rows a copy of its tokens brings (half a tile: each CTA takes half of every tile's rows)
+constexpr int P_LIST = 440;            // its units of tokens that are kept in shared memory
+static_assert(P_SMEM_BYTES + 4 * P_LIST <= 227 * 1024, "shared memory");
 // Pairs that run at a time: one per two SMs of the current device.
 inline int pair_slots() { return fb_sm_count() / 2 > 0 ? fb_sm_count() / 2 : 1; }
 
@@ -110,12 +114,59 @@ __device__ __forceinline__ PairUnit pair_unit(int u, int tiles_m, int tiles, int
     return w;
 }
 
-template <typename TO, bool ACT>     // ACT: the epilogue applies the plain activation `plain_act`
+// The grouped form (routed experts): its weights come from HBM once, and a CTA's share of a tile's tokens from L2 is half of what
+// the one-SM kernel of 128 x 128 wants, whose 128 bytes a cycle and SM were its bound.  2,048 / 1,024 / 180 tokens on 6 of 64
+// experts of 1,792 x 4,096, both products: 491 -> 413, 396 -> 360, 327 -> 315 us, of which 287 are the weights at the copy rate;
+// 512 tokens 326 -> 335 (48 rows an expert fit tiles of 64 well, and this kernel is not launched ahead of the one before it ends).
+// Rows come in tiles of 32 that belong to one group (an expert) each, negative groups are skipped.  A unit of
+// tokens is up to eight neighbouring tiles of one group, multiplied at their own width with that group's weight rows.  Every CTA
+// lists the units when it starts: one warp walks the tiles 32 at a time.  A unit is its first tile and, from bit 24 on, its tiles.
+__device__ __forceinline__ uint32_t group_unit_at(const int* tile_group, int n_tiles, int t) {
+    const int g = tile_group[t];
+    int c = 1;
+    while (c < PBN / P_GROUP_TILE && t + c < n_tiles && tile_group[t + c] == g) ++c;
+    return (uint32_t)t | (uint32_t)c << 24;
+}
+// All 32 lanes.  Writes the first P_LIST units and returns how many there are.
+__device__ __forceinline__ int group_units(const int* tile_group, int n_tiles, uint32_t* list) {
+    constexpr int MOST = PBN / P_GROUP_TILE;
+    const int lane = threadIdx.x & 31;
+    int found = 0, run = 0, before = -1;                 // run: where the run that reaches into this stretch began
+    for (int t0 = 0; t0 < n_tiles; t0 += 32) {
+        const int t = t0 + lane, g = t < n_tiles ? tile_group[t] : -1;
+        const int left = __shfl_up_sync(0xffffffffu, g, 1);
+        const uint32_t begins = __ballot_sync(0xffffffffu, g != (lane ? left : before));
+        const uint32_t mine = begins & (0xffffffffu >> (31 - lane));
+        const int from = mine ? t0 + 31 - __clz(mine) : run;
+        const uint32_t units = __ballot_sync(0xffffffffu, g >= 0 && (t - from) % MOST == 0);
+        const int at = found + __popc(units & ((1u << lane) - 1u));
+        if ((units >> lane & 1u) && at < P_LIST) list[at] = group_unit_at(tile_group, n_tiles, t);
+        found += __popc(units);
+        run = __shfl_sync(0xffffffffu, from, 31);
+        before = __shfl_sync(0xffffffffu, g, 31);
+    }
+    return found;
+}
+// Unit i, counted on from the last listed one where the list is too short for it (more units than any sort of rows by group
+// makes of up to 3,000 tiles).
+__device__ __forceinline__ uint32_t group_unit(const int* tile_group, int n_tiles, const uint32_t* list, int i) {
+    if (i < P_LIST) return list[i];
+    uint32_t unit = list[P_LIST - 1];
+    for (int k = P_LIST; k <= i; ++k) {
+        int t = (int)(unit & 0xffffffu) + (int)(unit >> 24);
+        while (tile_group[t] < 0) ++t;
+        unit = group_unit_at(tile_group, n_tiles, t);
+    }
+    return unit;
+}
+
+template <typename TO, bool ACT, bool GROUPED>     // ACT: the epilogue applies the plain activation `plain_act`
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                     const __grid_constant__ CUtensorMap map_o, int boxed_out,
                     TO* __restrict__ out, long ldo, long slab_stride, int M, int N, int K, int tiles_m, int tiles,
-                    int splits, int n_units, FbGate gated, int plain_act, int accumulate, int* status) {
+                    int splits, int n_units, FbGate gated, int plain_act, int accumulate, int* status,
+                    const int* __restrict__ tile_group, int n_tiles) {
     constexpr int S = P_STAGES;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -124,12 +175,16 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     // [2S+2..2S+4): accumulator empty (even CTA's are used)
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * S + 4);
     int* bail = (int*)(tmem_slot + 1);
+    int* group_count = bail + 1;
     uint8_t* out_stage = smem + S * P_STAGE_BYTES + 256;     // [2 groups of warps][2 buffers][16 tokens][128 features]
+
+    uint32_t* list = (uint32_t*)(out_stage + 4 * P_OUT_BYTES);
 
     fb_pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
-    const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+    const int pair = blockIdx.x >> 1;
+    int n_pairs = gridDim.x >> 1, first_unit = pair;
     const int kb_total = (K + PBK - 1) / PBK;
 
     if (threadIdx.x == 0) {
@@ -149,23 +204,54 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                      ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)P_TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
+    if (GROUPED && warp == 2) {
+        fb_pdl_wait();                           // which weights a tile wants is the work of the kernels before this one
+        const int found = group_units(tile_group, n_tiles, list);
+        if (lane == 0) *group_count = found;
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     cluster_sync_all();                          // both CTAs' barriers exist before either signals the other's
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
+    // Feature tiles vary fastest in the grouped form: a group's weights serve its units of tokens while they are in L2, and the
+    // units that run together share few units' rows.
+    const int tiles_n = GROUPED ? tiles : 0;                     // (the grouped form has no use for the other's counts)
+    if (GROUPED) {
+        // As many pairs as the rounds need: 448 units on 74 pairs are six rounds and four units, which stream their weights alone;
+        // on 64 they are seven even ones (2,048 tokens on 6 of 64 experts, 1,792 x 4,096: 222 -> 211 us).
+        n_units = *group_count * tiles_n;
+        const int rounds = (n_units + n_pairs - 1) / n_pairs;
+        if (rounds > 0) n_pairs = (n_units + rounds - 1) / rounds;
+        if (pair >= n_pairs) first_unit = n_units;
+    }
+    auto unit_of = [&](int u) {
+        if (!GROUPED) return pair_unit(u, tiles_m, tiles, splits, kb_total, M);
+        PairUnit w;
+        const int i = u / tiles_n;
+        const uint32_t unit = group_unit(tile_group, n_tiles, list, i);
+        w.mt = (int)(unit & 0xffffffu) * P_GROUP_TILE;           // (the first row itself)
+        w.nt = u - i * tiles_n;
+        w.split = 0;
+        w.kb_begin = 0;
+        w.n_kb = kb_total;
+        w.n_tok = (int)(unit >> 24) * P_GROUP_TILE;
+        return w;
+    };
 
     if (warp == 0) {
         // ---------------- copies: this CTA's weight rows and its half of the tokens ----------------
         if (elect_one()) {
             uint32_t it = 0;
             bool first = true;
-            for (int u = pair; u < n_units && !*(volatile int*)bail; u += n_pairs) {
-                const PairUnit w = pair_unit(u, tiles_m, tiles, splits, kb_total, M);
-                const int n0 = w.nt * (2 * PBM) + (int)rank * PBM;
-                const int m0 = w.mt * PBN + (int)rank * (w.n_tok / 2);    // this CTA's half of the tile's tokens
+            for (int u = first_unit; u < n_units && !*(volatile int*)bail; u += n_pairs) {
+                const PairUnit w = unit_of(u);
+                const int n0 = w.nt * (2 * PBM) + (int)rank * PBM + (GROUPED ? tile_group[w.mt / P_GROUP_TILE] * N : 0);
+                const int m0 = (GROUPED ? w.mt : w.mt * PBN) + (int)rank * (w.n_tok / 2);    // this CTA's half of the tile's tokens
+                const int boxes = w.n_tok / (2 * P_GROUP_BOX);
+                const uint32_t stage_bytes = GROUPED ? P_A_BYTES + (uint32_t)boxes * P_GROUP_BOX * PBK * 2 : P_STAGE_BYTES;
                 int i = 0;
-                if (first) {
+                if (!GROUPED && first) {
                     // weights do not depend on the kernel before this one; the activations do
                     first = false;
                     const int pre = w.n_kb < S ? w.n_kb : S;
@@ -185,11 +271,17 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     const int s = (int)(it % S);
                     const uint32_t round = it / S;
                     if (!mbar_wait(smem_u32(&bars[S + s]), (round & 1u) ^ 1u, status)) { *bail = 1; break; }
-                    if (rank == 0) mbar_expect_tx(smem_u32(&bars[s]), 2u * P_STAGE_BYTES);
+                    if (rank == 0) mbar_expect_tx(smem_u32(&bars[s]), 2u * stage_bytes);
                     const uint32_t full = in_cta(smem_u32(&bars[s]), 0);
                     uint8_t* stage = smem + (size_t)s * P_STAGE_BYTES;
                     tma_load_2d_pair(smem_u32(stage), &map_w, full, (w.kb_begin + i) * PBK, n0);
-                    tma_load_2d_pair(smem_u32(stage + P_A_BYTES), &map_x, full, (w.kb_begin + i) * PBK, m0);
+                    if (GROUPED) {
+                        for (int b = 0; b < boxes; ++b)
+                            tma_load_2d_pair(smem_u32(stage + P_A_BYTES + b * (P_GROUP_BOX * PBK * 2)), &map_x, full, i * PBK,
+                                             m0 + b * P_GROUP_BOX);
+                    } else {
+                        tma_load_2d_pair(smem_u32(stage + P_A_BYTES), &map_x, full, (w.kb_begin + i) * PBK, m0);
+                    }
                 }
             }
             if (first) fb_pdl_wait();
@@ -200,8 +292,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         if (rank == 0 && elect_one()) {
             uint32_t it = 0;
             int j = 0;
-            for (int u = pair; u < n_units && !*(volatile int*)bail; u += n_pairs, ++j) {
-                const PairUnit w = pair_unit(u, tiles_m, tiles, splits, kb_total, M);
+            for (int u = first_unit; u < n_units && !*(volatile int*)bail; u += n_pairs, ++j) {
+                const PairUnit w = unit_of(u);
                 const int n_kb = w.n_kb;
                 const uint32_t idesc = umma_idesc(w.n_tok, false, 2 * PBM);
                 const int b = j & 1;
@@ -239,9 +331,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         const int row_local = quarter * 32 + lane;
         uint32_t boxes = 0;                                     // boxes this group of warps has staged: the buffers take turns
         int j = 0;
-        for (int u = pair; u < n_units; u += n_pairs, ++j) {
-            const PairUnit w = pair_unit(u, tiles_m, tiles, splits, kb_total, M);
-            const int m0 = w.mt * PBN;
+        for (int u = first_unit; u < n_units; u += n_pairs, ++j) {
+            const PairUnit w = unit_of(u);
+            const int m0 = GROUPED ? w.mt : w.mt * PBN;
             const int n = w.nt * (2 * PBM) + (int)rank * PBM + row_local;
             TO* dst = out + (size_t)w.split * (size_t)slab_stride;     // this share's slab (the whole sum: slab 0)
             const int b = j & 1;
@@ -355,7 +447,7 @@ int launch_pair(const void* X, long lda, const void* W, long ldw, void* out, lon
     const int boxed = fb_tensor_map_out(&mo, out, (int)sizeof(TO), M, gated.act ? N / 2 : N, ldo, splits, slab_stride,
                                         gated.act ? PBM / 2 : PBM, P_OUT_TOKENS);
     if (boxed < 0) return boxed;
-    auto kern = gemm_tc_pair_kernel<TO, ACT>;
+    auto kern = gemm_tc_pair_kernel<TO, ACT, false>;
     static bool configured[FB_MAX_DEVICES] = {};
     if (fb_needs_setup(configured)) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM_BYTES);
@@ -370,14 +462,45 @@ int launch_pair(const void* X, long lda, const void* W, long ldw, void* out, lon
     const int pairs = (int)(n_units < pair_slots() ? n_units : pair_slots());
     fb_launch_class(FB_LAUNCH_GEMM_PAIR, (kern), 2 * pairs, P_THREADS, P_SMEM_BYTES, stream, mw, mx, mo,
                     boxed == 0 ? 1 : 0, (TO*)out, ldo, slab_stride, M, N, K, tiles_m, (int)tiles, splits, (int)n_units,
-                    gated, plain_act, accumulate, status);
+                    gated, plain_act, accumulate, status, (const int*)nullptr, 0);
     return fb_check_launch("gemm_tc_pair");
+}
+
+template <typename TO, bool ACT>
+int launch_pair_grouped(const void* X, long lda, const void* W, long ldw, int groups, const int* tile_group, void* out, long ldo,
+                        int M, int N, int K, FbGate gated, int plain_act, int* status, cudaStream_t stream) {
+    CUtensorMap mw, mx, mo;
+    int rc = fb_tensor_map_bf16(&mw, W, (long)groups * N, K, ldw, PBK, PBM);
+    if (rc) return rc;
+    rc = fb_tensor_map_bf16(&mx, X, M, K, lda, PBK, P_GROUP_BOX);
+    if (rc) return rc;
+    const int boxed = fb_tensor_map_out(&mo, out, (int)sizeof(TO), M, gated.act ? N / 2 : N, ldo, 1, 0, gated.act ? PBM / 2 : PBM,
+                                        P_OUT_TOKENS);
+    if (boxed < 0) return boxed;
+    auto kern = gemm_tc_pair_kernel<TO, ACT, true>;
+    constexpr int smem = P_SMEM_BYTES + 4 * P_LIST;
+    static bool configured[FB_MAX_DEVICES] = {};
+    if (fb_needs_setup(configured)) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return fb_fail(-2, "gemm_tc_pair: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
+        fb_setup_done(configured);
+    }
+    const int n_tiles = M / P_GROUP_TILE, tiles_n = (N + 2 * PBM - 1) / (2 * PBM);
+    const long most = (long)n_tiles * tiles_n;
+    const int pairs = (int)(most < pair_slots() ? most : pair_slots());
+    fb_launch_class(FB_LAUNCH_GEMM_PAIR, (kern), 2 * pairs, P_THREADS, smem, stream, mw, mx, mo, boxed == 0 ? 1 : 0, (TO*)out, ldo, 0L,
+                    M, N, K, 0, tiles_n, 1, 0, gated, plain_act, 0, status, tile_group, n_tiles);
+    return fb_check_launch("gemm_tc_pair_grouped");
 }
 
 }  // namespace
 
 static int g_pair_on = -1;                       // -1: not yet read from the environment
 FB_API void fb_set_gemm_pair(int on) { g_pair_on = on ? 1 : 0; }
+static bool pair_on() {
+    if (g_pair_on < 0) g_pair_on = (getenv("FLAMBEAU_GEMM_PAIR") && atoi(getenv("FLAMBEAU_GEMM_PAIR")) == 0) ? 0 : 1;
+    return g_pair_on != 0;
+}
 
 // Shares of K for the pairs: as many as make the rounds of the resident pairs shortest, each share beyond the first
 // costing one more float32 copy of the output (written here, added by the consumer), counted in k-block times.
@@ -397,8 +520,7 @@ static int pair_splits(long tiles, int kb_total, int max_splits, int M, int N) {
 }
 
 int fb_gemm_pair_plan(int M, int N, int K, int max_slabs) {
-    if (g_pair_on < 0) g_pair_on = (getenv("FLAMBEAU_GEMM_PAIR") && atoi(getenv("FLAMBEAU_GEMM_PAIR")) == 0) ? 0 : 1;
-    if (!g_pair_on || K <= 0 || M <= PBNH) return 0;
+    if (!pair_on() || K <= 0 || M <= PBNH) return 0;
     const long tiles = (long)((M + PBN - 1) / PBN) * ((N + 2 * PBM - 1) / (2 * PBM));
     const int kb_total = (K + PBK - 1) / PBK;
     const int splits = pair_splits(tiles, kb_total, max_slabs < 1 ? 1 : (max_slabs > 16 ? 16 : max_slabs), M, N);
@@ -406,6 +528,22 @@ int fb_gemm_pair_plan(int M, int N, int K, int max_slabs) {
     // shares meet in scratch, is the better choice.
     if (splits == 1 && tiles < 48 && kb_total >= 128) return 0;
     return splits;
+}
+
+// The grouped product (gemm_tc.cu: fb_gemm_tc_grouped) over tiles of 32 rows on the pairs; 1: not here (switched off, or this type
+// with this activation has no such kernel).
+int fb_launch_gemm_pair_grouped(const void* X, long lda, const void* W, long ldw, int groups, const int* tile_group, void* out, int o_dtype,
+                                long ldo, int M, int N, int K, FbGate gated, int plain_act, int* status, cudaStream_t stream) {
+    if (!pair_on() || M % P_GROUP_TILE != 0 || (long)M / P_GROUP_TILE >= (1L << 24) ||
+        ((long)M / P_GROUP_TILE) * ((N + 2 * PBM - 1) / (2 * PBM)) > 2000000000L)
+        return 1;
+    if (plain_act) {
+        if (o_dtype != FB_BF16) return 1;
+        return launch_pair_grouped<__nv_bfloat16, true>(X, lda, W, ldw, groups, tile_group, out, ldo, M, N, K, gated, plain_act, status, stream);
+    }
+    if (o_dtype == FB_F32)
+        return launch_pair_grouped<float, false>(X, lda, W, ldw, groups, tile_group, out, ldo, M, N, K, gated, 0, status, stream);
+    return launch_pair_grouped<__nv_bfloat16, false>(X, lda, W, ldw, groups, tile_group, out, ldo, M, N, K, gated, 0, status, stream);
 }
 
 int fb_launch_gemm_pair(const void* X, long lda, const void* W, long ldw, void* out, int o_dtype, long ldo,

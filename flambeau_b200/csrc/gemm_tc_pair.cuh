@@ -14,3 +14,7 @@ int fb_gemm_pair_plan(int M, int N, int K, int max_slabs);
 int fb_launch_gemm_pair(const void* X, long lda, const void* W, long ldw, void* out, int o_dtype, long ldo,
                         long slab_stride, int splits, int M, int N, int K, FbGate gated, int accumulate, int* status,
                         cudaStream_t stream, int plain_act = 0);
+// The grouped form: row tiles of 32 of one group each (tile_group, negative: skipped), every group with N rows of W of its own.
+// 1 where the caller should take the one-SM kernel, else 0 or a negative error.
+int fb_launch_gemm_pair_grouped(const void* X, long lda, const void* W, long ldw, int groups, const int* tile_group, void* out, int o_dtype,
+                                long ldo, int M, int N, int K, FbGate gated, int plain_act, int* status, cudaStream_t stream);

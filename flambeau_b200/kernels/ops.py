@@ -719,13 +719,11 @@ _GROUPED_TC = [os.environ.get("FLAMBEAU_MOE_TC", "1") != "0"]
 
 def grouped_tile(pairs: int, groups: int, tensor_cores: bool) -> int:
     """Rows of a tile of the grouped products for `pairs` rows spread over `groups` groups: small tiles while a
-    group holds few rows (decoding: a tile of 16 streams an expert's weights once), larger ones as the groups fill
-    (128 on the tensor cores, whose instruction takes as long for 64 columns as for 128)."""
+    group holds few rows (decoding: a tile of 16 streams an expert's weights once), else 32 on the tensor cores, where the
+    kernel of two SMs joins a group's neighbouring tiles, and 64 on the CUDA cores."""
     if pairs <= 16 * groups:
         return 16
-    if tensor_cores and pairs >= 192 * groups:
-        return 128
-    return 64
+    return 32 if tensor_cores else 64
 
 
 def gather_rows(h: torch.Tensor, place_token: torch.Tensor, out: torch.Tensor, share=None, place_pair=None, tile_group=None,
