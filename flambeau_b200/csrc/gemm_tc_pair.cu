@@ -97,20 +97,20 @@ __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
 }
 
 // One unit of work: output tile (nt, mt) and share `split` of its K range.  Token tiles vary fastest, so pairs
-// that run together share weight tiles through L2; shares of K vary slowest.  The last token tile of a product
-// whose rows do not fill it is multiplied at its own width: n_tok = the tile's rows rounded up to 32 (the N of
-// the MMA; each CTA supplies n_tok / 2 tokens), so a step of 2,048 + 32 rows pays for 32 rows more, not for 256.
-struct PairUnit { int mt, nt, split, kb_begin, n_kb, n_tok; };
-__device__ __forceinline__ PairUnit pair_unit(int u, int tiles_m, int tiles, int splits, int kb_total, int M) {
+// that run together share weight tiles through L2; shares of K vary slowest.  Token tiles are `tile_w` rows wide (a
+// multiple of 32, chosen by the launcher), the last one as wide as its rows rounded up to 32: n_tok is the N of the MMA, of
+// which each CTA supplies n_tok / 2 tokens.
+struct PairUnit { int m0, nt, split, kb_begin, n_kb, n_tok; };
+__device__ __forceinline__ PairUnit pair_unit(int u, int tiles_m, int tiles, int splits, int kb_total, int M, int tile_w) {
     PairUnit w;
     const int t = u % tiles;
     w.split = u / tiles;
-    w.mt = t % tiles_m;
+    w.m0 = t % tiles_m * tile_w;
     w.nt = t / tiles_m;
     w.kb_begin = (int)((long)w.split * kb_total / splits);
     w.n_kb = (int)((long)(w.split + 1) * kb_total / splits) - w.kb_begin;
-    const int rows_left = M - w.mt * PBN;
-    w.n_tok = rows_left >= PBN ? PBN : ((rows_left + 31) / 32) * 32;
+    const int rows_left = M - w.m0;
+    w.n_tok = rows_left >= tile_w ? tile_w : ((rows_left + 31) / 32) * 32;
     return w;
 }
 
@@ -166,7 +166,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     const __grid_constant__ CUtensorMap map_o, int boxed_out,
                     TO* __restrict__ out, long ldo, long slab_stride, int M, int N, int K, int tiles_m, int tiles,
                     int splits, int n_units, FbGate gated, int plain_act, int accumulate, int* status,
-                    const int* __restrict__ tile_group, int n_tiles) {
+                    const int* __restrict__ tile_group, int n_tiles, int tile_w) {
     constexpr int S = P_STAGES;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -216,7 +216,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     const uint32_t tmem_base = *tmem_slot;
     // Feature tiles vary fastest in the grouped form: a group's weights serve its units of tokens while they are in L2, and the
     // units that run together share few units' rows.
-    const int tiles_n = GROUPED ? tiles : 0;                     // (the grouped form has no use for the other's counts)
+    const int tiles_n = tiles;                                   // (in the grouped form, which has no use for the other's counts)
     if (GROUPED) {
         // As many pairs as the rounds need: 448 units on 74 pairs are six rounds and four units, which stream their weights alone;
         // on 64 they are seven even ones (2,048 tokens on 6 of 64 experts, 1,792 x 4,096: 222 -> 211 us).
@@ -226,17 +226,20 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         if (pair >= n_pairs) first_unit = n_units;
     }
     auto unit_of = [&](int u) {
-        if (!GROUPED) return pair_unit(u, tiles_m, tiles, splits, kb_total, M);
-        PairUnit w;
-        const int i = u / tiles_n;
-        const uint32_t unit = group_unit(tile_group, n_tiles, list, i);
-        w.mt = (int)(unit & 0xffffffu) * P_GROUP_TILE;           // (the first row itself)
-        w.nt = u - i * tiles_n;
-        w.split = 0;
-        w.kb_begin = 0;
-        w.n_kb = kb_total;
-        w.n_tok = (int)(unit >> 24) * P_GROUP_TILE;
-        return w;
+        if constexpr (GROUPED) {
+            PairUnit w;
+            const int i = u / tiles_n;
+            const uint32_t unit = group_unit(tile_group, n_tiles, list, i);
+            w.m0 = (int)(unit & 0xffffffu) * P_GROUP_TILE;
+            w.nt = u - i * tiles_n;
+            w.split = 0;
+            w.kb_begin = 0;
+            w.n_kb = kb_total;
+            w.n_tok = (int)(unit >> 24) * P_GROUP_TILE;
+            return w;
+        } else {
+            return pair_unit(u, tiles_m, tiles, splits, kb_total, M, tile_w);
+        }
     };
 
     if (warp == 0) {
@@ -246,17 +249,17 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             bool first = true;
             for (int u = first_unit; u < n_units && !*(volatile int*)bail; u += n_pairs) {
                 const PairUnit w = unit_of(u);
-                const int n0 = w.nt * (2 * PBM) + (int)rank * PBM + (GROUPED ? tile_group[w.mt / P_GROUP_TILE] * N : 0);
-                const int m0 = (GROUPED ? w.mt : w.mt * PBN) + (int)rank * (w.n_tok / 2);    // this CTA's half of the tile's tokens
+                const int n0 = w.nt * (2 * PBM) + (int)rank * PBM + (GROUPED ? tile_group[w.m0 / P_GROUP_TILE] * N : 0);
+                const int m0 = w.m0 + (int)rank * (w.n_tok / 2);    // this CTA's half of the tile's tokens
                 const int boxes = w.n_tok / (2 * P_GROUP_BOX);
-                const uint32_t stage_bytes = GROUPED ? P_A_BYTES + (uint32_t)boxes * P_GROUP_BOX * PBK * 2 : P_STAGE_BYTES;
+                const uint32_t stage_bytes = GROUPED ? P_A_BYTES + (uint32_t)boxes * P_GROUP_BOX * PBK * 2 : P_A_BYTES + (uint32_t)(tile_w / 2) * PBK * 2;
                 int i = 0;
                 if (!GROUPED && first) {
                     // weights do not depend on the kernel before this one; the activations do
                     first = false;
                     const int pre = w.n_kb < S ? w.n_kb : S;
                     for (int j = 0; j < pre; ++j) {
-                        if (rank == 0) mbar_expect_tx(smem_u32(&bars[j]), 2u * P_STAGE_BYTES);
+                        if (rank == 0) mbar_expect_tx(smem_u32(&bars[j]), 2u * stage_bytes);
                         tma_load_2d_pair(smem_u32(smem + (size_t)j * P_STAGE_BYTES), &map_w,
                                          in_cta(smem_u32(&bars[j]), 0), (w.kb_begin + j) * PBK, n0);
                     }
@@ -333,7 +336,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         int j = 0;
         for (int u = first_unit; u < n_units; u += n_pairs, ++j) {
             const PairUnit w = unit_of(u);
-            const int m0 = GROUPED ? w.mt : w.mt * PBN;
+            const int m0 = w.m0;
             const int n = w.nt * (2 * PBM) + (int)rank * PBM + row_local;
             TO* dst = out + (size_t)w.split * (size_t)slab_stride;     // this share's slab (the whole sum: slab 0)
             const int b = j & 1;
@@ -435,12 +438,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 }
 
 template <typename TO, bool ACT = false>
-int launch_pair(const void* X, long lda, const void* W, long ldw, void* out, long ldo, long slab_stride, int splits,
+int launch_pair(const void* X, long lda, const void* W, long ldw, void* out, long ldo, long slab_stride, int splits, int tile_w,
                 int M, int N, int K, FbGate gated, int accumulate, int* status, cudaStream_t stream, int plain_act = 0) {
     CUtensorMap mw, mx;
     int rc = fb_tensor_map_bf16(&mw, W, N, K, ldw, PBK, PBM);
     if (rc) return rc;
-    rc = fb_tensor_map_bf16(&mx, X, M, K, lda, PBK, PBNH);
+    rc = fb_tensor_map_bf16(&mx, X, M, K, lda, PBK, tile_w / 2);
     if (rc) return rc;
     // the output as boxes of 16 tokens x a CTA's features (half as many where the epilogue folds gate and up)
     CUtensorMap mo;
@@ -455,14 +458,14 @@ int launch_pair(const void* X, long lda, const void* W, long ldw, void* out, lon
                                              P_SMEM_BYTES, cudaGetErrorString(e));
         fb_setup_done(configured);
     }
-    const int tiles_m = (M + PBN - 1) / PBN, tiles_n = (N + 2 * PBM - 1) / (2 * PBM);
+    const int tiles_m = (M + tile_w - 1) / tile_w, tiles_n = (N + 2 * PBM - 1) / (2 * PBM);
     const long tiles = (long)tiles_m * tiles_n;
     const long n_units = tiles * splits;
     if (n_units > 2000000000L) return fb_fail(-1, "gemm_tc_pair: too many tiles (M=%d N=%d)", M, N);
     const int pairs = (int)(n_units < pair_slots() ? n_units : pair_slots());
     fb_launch_class(FB_LAUNCH_GEMM_PAIR, (kern), 2 * pairs, P_THREADS, P_SMEM_BYTES, stream, mw, mx, mo,
                     boxed == 0 ? 1 : 0, (TO*)out, ldo, slab_stride, M, N, K, tiles_m, (int)tiles, splits, (int)n_units,
-                    gated, plain_act, accumulate, status, (const int*)nullptr, 0);
+                    gated, plain_act, accumulate, status, (const int*)nullptr, 0, tile_w);
     return fb_check_launch("gemm_tc_pair");
 }
 
@@ -489,7 +492,7 @@ int launch_pair_grouped(const void* X, long lda, const void* W, long ldw, int gr
     const long most = (long)n_tiles * tiles_n;
     const int pairs = (int)(most < pair_slots() ? most : pair_slots());
     fb_launch_class(FB_LAUNCH_GEMM_PAIR, (kern), 2 * pairs, P_THREADS, smem, stream, mw, mx, mo, boxed == 0 ? 1 : 0, (TO*)out, ldo, 0L,
-                    M, N, K, 0, tiles_n, 1, 0, gated, plain_act, 0, status, tile_group, n_tiles);
+                    M, N, K, 0, tiles_n, 1, 0, gated, plain_act, 0, status, tile_group, n_tiles, PBN);
     return fb_check_launch("gemm_tc_pair_grouped");
 }
 
@@ -502,7 +505,7 @@ static bool pair_on() {
     return g_pair_on != 0;
 }
 
-// Shares of K for the pairs: as many as make the rounds of the resident pairs shortest, each share beyond the first
+// Shares of K for tiles of 256 tokens: as many as make the rounds of the resident pairs shortest, each share beyond the first
 // costing one more float32 copy of the output (written here, added by the consumer), counted in k-block times.
 static int pair_splits(long tiles, int kb_total, int max_splits, int M, int N) {
     const double kb_seconds = 2.0 * PBM * PBN * PBK / FB_MODEL_SM_FLOPS;
@@ -519,14 +522,47 @@ static int pair_splits(long tiles, int kb_total, int max_splits, int M, int N) {
     return best;
 }
 
+// The width of the token tiles and the shares of K with the least time, of at least `least_splits` shares.  A k-block of a unit
+// takes its MMAs (2 w cycles) or its bytes (its CTA's weight rows and tokens at PAIR_L2 bytes a cycle), whichever is more, plus
+// PAIR_EXTRA; the pairs work in rounds of units, and all together need no less than the weights' time from HBM.  Tiles as wide
+// as the rows divide evenly are what helps: 537 rows as 3 x 192 and not 2 x 256 + 32.  Measured (us, tiles of 256 with the best
+// number of shares / here), outputs x inputs 6,144 x 4,096: 300 rows 24.8 / 22.0, 537 rows 29.5 / 24.9, 1,029 rows 47.8 / 42.2;
+// 4,096 x 4,096: 300 rows 19.6 / 16.1, 537 rows 23.6 / 21.0, 1,029 rows 38.3 / 34.9; 28,672 x 5,120: 300 rows 110.6 / 95.6, 537
+// rows 136.9 / 125.5.
+struct PairPlan { int tile_w, splits; };
+constexpr double PAIR_L2 = 64.0, PAIR_EXTRA = 10.0, PAIR_HZ = 1.8e9;
+static PairPlan pair_plan(int M, int N, int K, int least_splits, int max_splits) {
+    const long tiles_n = (N + 2 * PBM - 1) / (2 * PBM), least = (M + PBN - 1) / PBN;
+    const int kb_total = (K + PBK - 1) / PBK, slots = pair_slots();
+    const double share = (double)M * N * 8.0 / FB_MODEL_HBM_BYTES_PER_S * PAIR_HZ;
+    const double weights = 2.0 * N * K / FB_MODEL_HBM_BYTES_PER_S * PAIR_HZ;
+    PairPlan best = {PBN, least_splits};
+    double best_cost = 1e300;
+    for (long tiles_m = least; tiles_m <= least + 2; ++tiles_m) {
+        const int w = (int)(((M + tiles_m - 1) / tiles_m + 31) / 32 * 32);
+        if ((M + w - 1) / w != tiles_m || w > PBN) continue;
+        const double kb = fmax(2.0 * w, (P_A_BYTES + w * PBK) / PAIR_L2) + PAIR_EXTRA;
+        for (int s = least_splits; s <= max_splits && s <= kb_total; ++s) {
+            const long rounds = (tiles_m * tiles_n * s + slots - 1) / slots;
+            const double cost = fmax(rounds * ((kb_total + s - 1) / s + 0.5) * kb, weights) + (s - 1) * share;
+            if (cost < best_cost * (1.0 - 1e-9)) { best_cost = cost; best = PairPlan{w, s}; }
+        }
+    }
+    return best;
+}
+// The width that goes with `splits` shares, which the caller has from fb_gemm_pair_plan (or has settled itself).
+static int pair_tile_w(int M, int N, int K, int splits) { return pair_plan(M, N, K, splits, splits).tile_w; }
+
 int fb_gemm_pair_plan(int M, int N, int K, int max_slabs) {
     if (!pair_on() || K <= 0 || M <= PBNH) return 0;
     const long tiles = (long)((M + PBN - 1) / PBN) * ((N + 2 * PBM - 1) / (2 * PBM));
-    const int kb_total = (K + PBK - 1) / PBK;
-    const int splits = pair_splits(tiles, kb_total, max_slabs < 1 ? 1 : (max_slabs > 16 ? 16 : max_slabs), M, N);
+    const int most = max_slabs < 1 ? 1 : (max_slabs > 16 ? 16 : max_slabs);
+    // (At least as many shares as tiles of 256 would have: the tensor cores cut their sums off, so fewer and longer sums of K
+    // would be less exact where they stay float32.)
+    const int splits = pair_plan(M, N, K, pair_splits(tiles, (K + PBK - 1) / PBK, most, M, N), most).splits;
     // A long K on few tiles needs shares of K; where the caller has no slabs for them, the one-SM kernel, whose
     // shares meet in scratch, is the better choice.
-    if (splits == 1 && tiles < 48 && kb_total >= 128) return 0;
+    if (splits == 1 && tiles < 48 && (K + PBK - 1) / PBK >= 128) return 0;
     return splits;
 }
 
@@ -549,19 +585,20 @@ int fb_launch_gemm_pair_grouped(const void* X, long lda, const void* W, long ldw
 int fb_launch_gemm_pair(const void* X, long lda, const void* W, long ldw, void* out, int o_dtype, long ldo,
                         long slab_stride, int splits, int M, int N, int K, FbGate gated, int accumulate, int* status,
                         cudaStream_t stream, int plain_act) {
+    const int tile_w = pair_tile_w(M, N, K, splits);
     if (plain_act) {
         if (splits != 1 || accumulate || gated.act || o_dtype != FB_BF16)
             return fb_fail(-1, "gemm_tc_pair: a plain activation needs a whole product in bfloat16 of its own");
-        return launch_pair<__nv_bfloat16, true>(X, lda, W, ldw, out, ldo, 0, 1, M, N, K, gated, 0, status, stream, plain_act);
+        return launch_pair<__nv_bfloat16, true>(X, lda, W, ldw, out, ldo, 0, 1, tile_w, M, N, K, gated, 0, status, stream, plain_act);
     }
     if (splits < 1 || (splits > 1 && (slab_stride <= 0 || o_dtype != FB_F32 || gated.act)))
         return fb_fail(-1, "gemm_tc_pair: %d shares of K need float32 slabs", splits);
     if (accumulate && (o_dtype != FB_F32 || splits != 1 || gated.act))
         return fb_fail(-1, "gemm_tc_pair: only a whole float32 product can be added to its output");
     if (o_dtype == FB_F32)
-        return launch_pair<float>(X, lda, W, ldw, out, ldo, slab_stride, splits, M, N, K, gated, accumulate, status,
+        return launch_pair<float>(X, lda, W, ldw, out, ldo, slab_stride, splits, tile_w, M, N, K, gated, accumulate, status,
                                   stream);
     if (o_dtype == FB_BF16)
-        return launch_pair<__nv_bfloat16>(X, lda, W, ldw, out, ldo, 0, 1, M, N, K, gated, 0, status, stream);
+        return launch_pair<__nv_bfloat16>(X, lda, W, ldw, out, ldo, 0, 1, tile_w, M, N, K, gated, 0, status, stream);
     return fb_fail(-1, "gemm_tc_pair: unknown output dtype code %d", o_dtype);
 }
