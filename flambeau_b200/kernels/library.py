@@ -90,6 +90,7 @@ _SIGNATURES = {
     "fb_gla_recurrent": (I, [P, P, P, L, P, P, P, I, I, I, P, I, I, I, STREAM]),
     # latent_attention.cu
     "fb_mla_latents": (I, [P, L, I, L, I, P, P, I, I, I, P, I, F, P, P, I, I, P, P, P, I, P, P, I, I, I, I, P, STREAM]),
+    "fb_head_linear_tc": (I, [P, I, L, L, I, L, P, P, L, L, I, I, I, I, P, STREAM]),
     "fb_head_linear": (I, [P, I, L, L, I, L, P, I, P, I, L, L, P, L, I, L, I, P, P, I, I, I, I, I, I, I, STREAM]),
     "fb_rope_neighbours": (I, [P, L, P, P, I, I, I, I, STREAM]),
     # diff_attention.cu

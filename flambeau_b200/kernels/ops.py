@@ -1451,16 +1451,24 @@ def mla_latents(proj, Rq: int, wq, cq, kv_off: int, Rc: int, r: int, wkv, eps: f
 
 def head_linear(a, a_head: int, w, out, o_head: int, n: int, n_partials: int = 1, partial_stride: int = 0, gate=None,
                 gate_off: int = 0, gate_partials: int = 1, gate_partial_stride: int = 0, cos=None, sin=None,
-                half: int = 0, rot: int = 0, pairing: str = "neighbours") -> None:
+                half: int = 0, rot: int = 0, pairing: str = "neighbours", status=None) -> None:
     """out[t, h*o_head + c] = sum_k w[h, c, k] * a[t, h*a_head + k] for every head h (w [H, N, K]); `a` may be the
     first of float32 shares.  gate (float32 rows, possibly shares): the result is multiplied by
     sigmoid(gate[t, gate_off + h*N + c]).  rot > 0: columns K .. K+rot of a's head go, their first 2*half dimensions
     turned pairwise by (cos, sin), to columns N .. N+rot of out's head; `pairing` says which dimensions form a pair
-    (ROTARY_PAIRING)."""
+    (ROTARY_PAIRING).  With `status` (the word kernels report into) a portion's plain bfloat16 map may run on the tcgen05
+    kernel (csrc/head_linear_tc.cu)."""
     _cuda(a, w, out, gate, cos, sin)
     H, N, K = w.shape
     if not w.is_contiguous() or a.shape[0] < n or out.shape[0] < n:
         raise KernelError("head_linear: bad shapes")
+    if status is not None and gate is None and rot == 0 and w.dtype == out.dtype == torch.bfloat16:
+        rc = lib().fb_head_linear_tc(a.data_ptr(), dtype_code(a), _rows(a), int(a_head), int(n_partials), int(partial_stride),
+                                     w.data_ptr(), out.data_ptr(), _rows(out), int(o_head), int(n), H, N, K, status.data_ptr(),
+                                     _stream())
+        if rc != 1:
+            check(rc, "head_linear_tc", (n * H, N, K))
+            return
     check(lib().fb_head_linear(a.data_ptr(), dtype_code(a), _rows(a), int(a_head), int(n_partials), int(partial_stride),
                                w.data_ptr(), dtype_code(w), out.data_ptr(), dtype_code(out), _rows(out), int(o_head),
                                _ptr(gate), _rows(gate) if gate is not None else 0, int(gate_partials),

@@ -136,13 +136,13 @@ class LatentAttention(Mixer):
                 qs, q_parts = slabs, parts                 # the first columns of the stacked product
             q = ctx.ws.alloc((n, H * hd), rt.dtype)
             ops.head_linear(qs[0], d + r, self.uk_t, q, hd, n, n_partials=q_parts, partial_stride=qs.stride(0),
-                            cos=cos, sin=sin, half=half, rot=r, pairing=pairing)
+                            cos=cos, sin=sin, half=half, rot=r, pairing=pairing, status=rt.status)
             a = ctx.ws.alloc((n, H * hd), rt.dtype)
             ops.paged_attention(ctx, q, a, cache, H, 1, hd, self.window, self.scale, vd=hd, weights_float32=True,
                                 sinks=self.sinks)
             og = ctx.ws.alloc((n, H * e), rt.dtype)
             ops.head_linear(a, hd, self.uv, og, e, n, gate=slabs[0] if self.gate else None, gate_off=self.gate_off,
-                            gate_partials=parts, gate_partial_stride=stride)
+                            gate_partials=parts, gate_partial_stride=stride, status=rt.status)
             ctx.to_stream(self.o, og)
 
 

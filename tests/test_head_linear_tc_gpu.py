@@ -1,0 +1,40 @@
+"""The map per head of portions (tcgen05) against float64: row counts around its tiles, every size, heads with numbers between
+them, shares; and what it leaves to the kernel of 64 x 64 tiles."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [128, 129, 255, 300, 1031])
+@pytest.mark.parametrize("N,K", [(64, 64), (256, 128), (128, 256), (192, 64), (64, 512), (256, 192)])
+@pytest.mark.parametrize("shares", [0, 1, 3])
+def test_rows_of_heads(n, N, K, shares):
+    from flambeau_b200.kernels import ops
+    H, apad, opad = 3 if shares < 2 else 150, 8, 16         # (shares: where every SM has a tile)
+    g = torch.Generator(device="cuda").manual_seed(n + N)
+    w = torch.randn(H, N, K, generator=g, device="cuda").bfloat16()
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    a = torch.randn(max(shares, 1), n, H * (K + apad), generator=g, device="cuda")
+    a = a if shares else a.bfloat16()
+    out = torch.full((n, H * (N + opad)), 7.0, device="cuda").bfloat16()
+    ops.head_linear(a[0], K + apad, w, out, N + opad, n, n_partials=max(shares, 1), partial_stride=a.stride(0), status=status)
+    assert int(status) == 0
+    x = a.sum(0) if shares < 3 else (a[0] + a[1]) + a[2]                   # float32 shares are added in their order
+    x = x.bfloat16().double().view(n, H, K + apad)[..., :K]
+    want, size = (torch.einsum("nhk,hck->nhc", p, q) for p, q in ((x, w.double()), (x.abs(), w.double().abs())))
+    got = out.double().view(n, H, N + opad)
+    assert bool(((got[..., :N] - want).abs() <= K * 2.0 ** -23 * size + 2.0 ** -8 * want.abs() + 1e-30).all())
+    assert bool((got[..., N:] == 7.0).all())
+
+
+def test_left_to_the_other_kernel():
+    """Few rows, sizes off 64, rows off 16-byte borders: the same map by the kernel of 64 x 64 tiles."""
+    from flambeau_b200.kernels import ops
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for n, N, K, pad in ((127, 64, 64, 0), (200, 72, 64, 0), (200, 64, 40, 0), (200, 320, 64, 0), (200, 64, 64, 1)):
+        a, w = torch.randn(n, 2 * K + pad, device="cuda").bfloat16(), torch.randn(2, N, K, device="cuda").bfloat16()
+        outs = [torch.zeros(n, 2 * N, device="cuda").bfloat16() for _ in range(2)]
+        ops.head_linear(a, K, w, outs[0], N, n, status=status)
+        ops.head_linear(a, K, w, outs[1], N, n)
+        assert torch.equal(*outs) and float(outs[0].abs().max()) > 0
