@@ -1,5 +1,6 @@
 // Paged causal (sliding-window) attention in float32 on the CUDA cores, in tiles: the attention of the true 32-bit path for
-// head sizes that are multiples of 4 up to 256 (attention_simt.cu takes every other size and the bfloat16 forms).
+// head sizes that are multiples of 4 up to 256 (attention_f32_tc.cu takes heads of 128 without caps, slopes and kept first keys,
+// attention_simt.cu every other size and the bfloat16 forms).
 //
 // A CTA of 128 threads owns one key/value head, BM query rows = (BM / G) tokens x the G query heads that share the head, and
 // some of the 32-key tiles that its rows see.  K and V tiles come through the block table by 16-byte asynchronous copies, V
@@ -21,67 +22,13 @@
 // Sums run in float32 throughout; sinks, caps, gates, slopes and kept first keys as in attention_simt.cu.
 #include <type_traits>
 
-#include "common.cuh"
+#include "attention_f32.cuh"
 
 namespace {
 
 constexpr int THREADS = 128;
 constexpr int KEYS = 32;                // keys of a tile
-constexpr int STRETCH = 256;            // keys of a stretch: joined on their own, whoever takes them
 constexpr int TPS = STRETCH / KEYS;
-constexpr long long SCRATCH_FLOATS = 1LL << 25;      // most that stretches of one launch may leave for joining
-
-struct F32Args {
-    const float* q; long q_stride;
-    float* out; long out_stride;
-    const float* k_pool; const float* v_pool;
-    int page_size, n_pages;
-    const int* block_table; int table_stride; const int* table_base; int table_head;
-    const int* seq_q_start; const int* seq_q_len; const int* seq_pos_start;
-    int n_seqs, n, nh, nkv, hd, vd, window, keep_first;
-    float scale, softcap;
-    const float* score_slopes; const float* sinks;
-    const float* head_gate; long gate_stride; int gate_partials; long gate_partial_stride;
-    int token_tiles;                    // CTAs that the tokens of a (sequence, key/value head) are laid over
-    int short_rows;                     // sequences with at most this many rows (tokens x G) run with BM 16
-    int slots, per;                     // stretches that a row's keys have at most, and that a CTA takes
-    int part_rows;                      // rows of a pair in the parts of BM 16
-    float* part_o; float* part_ml;      // per stretch and row: output x vd, and (maximum, sum); nullptr: a CTA takes all
-    int* status;
-};
-
-// What a stretch (maximum m, sum l) adds to the stretches before it (M, L): the factors of the output so far and of its own.
-struct Join { float before, own; };
-__device__ __forceinline__ Join join(float& M, float& L, float m, float l) {
-    const float top = fmaxf(M, m);
-    Join j;
-    j.before = M == -INFINITY ? 0.0f : expf(M - top);
-    j.own = m == -INFINITY ? 0.0f : expf(m - top);
-    L = fmaf(L, j.before, __fmul_rn(l, j.own));
-    M = top;
-    return j;
-}
-__device__ __forceinline__ float joined(const Join& j, float before, float own) { return fmaf(before, j.before, __fmul_rn(own, j.own)); }
-
-// What a row's joined output is multiplied with in the end.
-__device__ __forceinline__ float finish(const F32Args& a, int row, int head, float M, float L) {
-    float f = 1.0f, sum = L;
-    if (a.sinks) {                                               // the slot without key and value
-        const float sk = a.sinks[head], top = fmaxf(M, sk);
-        f = M == -INFINITY ? 0.0f : expf(M - top);
-        sum = fmaf(sum, f, expf(sk - top));
-    }
-    f = sum > 0.0f ? f / sum : 0.0f;
-    if (a.head_gate)
-        f /= 1.0f + expf(-fb_slab_sum(a.head_gate + (size_t)row * a.gate_stride, head, a.gate_partials, a.gate_partial_stride));
-    return f;
-}
-
-// Row r of a CTA, in the parts of a stretch.
-template <int BM>
-__device__ __forceinline__ size_t part_at(const F32Args& a, int slot, int pair, int row, int head, int r) {
-    return BM == 16 ? ((size_t)slot * a.n_seqs * a.nkv + pair) * a.part_rows + r : ((size_t)slot * a.n + row) * a.nh + head;
-}
 
 __device__ __forceinline__ void copy16(float* dst, const float* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
@@ -347,44 +294,6 @@ attention_f32_kernel(const F32Args a) {
                 *reinterpret_cast<float2*>(a.part_ml + 2 * part_at<BM>(a, slot, pair, q_start + r / G, kvh * G + r % G, r)) = make_float2(-INFINITY, 0.0f);
 }
 
-// One warp a row of the CTAs above (blockIdx.y: four rows each): its stretches joined.
-template <int BM>
-__global__ void __launch_bounds__(128)
-attention_f32_join_kernel(const F32Args a) {
-    fb_pdl_launch_dependents();
-    fb_pdl_wait();
-    const int G = a.nh / a.nkv, lane = threadIdx.x & 31, r = blockIdx.y * 4 + (threadIdx.x >> 5);
-    const int pair = blockIdx.x / a.token_tiles, tile = blockIdx.x - pair * a.token_tiles;
-    const int seq = pair / a.nkv, kvh = pair - seq * a.nkv, q_len = a.seq_q_len[seq];
-    if ((q_len * G <= a.short_rows) != (BM == 16)) return;
-    const int TQ = BM / G, tok0 = (a.token_tiles - 1 - tile) * TQ;
-    if (tok0 >= q_len || r >= min(TQ, q_len - tok0) * G) return;
-    const int row = a.seq_q_start[seq] + tok0 + r / G, head = kvh * G + r % G;
-    float M = -INFINITY, L = 0.0f;
-    float4 acc[2] = {};
-#pragma unroll 4
-    for (int s = 0; s < a.slots; ++s) {
-        const size_t at = part_at<BM>(a, s, pair, row, head, r);
-        const float2 ml = *reinterpret_cast<const float2*>(a.part_ml + 2 * at);
-        if (ml.x == -INFINITY && ml.y == 0.0f) continue;         // nothing was seen there (and nothing left)
-        const Join j = join(M, L, ml.x, ml.y);
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            const int d = 4 * lane + 128 * c;
-            if (d >= a.vd) continue;
-            const float4 x = *reinterpret_cast<const float4*>(a.part_o + at * a.vd + d);
-            acc[c] = make_float4(joined(j, acc[c].x, x.x), joined(j, acc[c].y, x.y), joined(j, acc[c].z, x.z), joined(j, acc[c].w, x.w));
-        }
-    }
-    const float f = finish(a, row, head, M, L);
-    float* op = a.out + (size_t)row * a.out_stride + (size_t)head * a.vd;
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-        const int d = 4 * lane + 128 * c;
-        if (d < a.vd) *reinterpret_cast<float4*>(op + d) = make_float4(acc[c].x * f, acc[c].y * f, acc[c].z * f, acc[c].w * f);
-    }
-}
-
 size_t smem_bytes(int bm, int hd, int vdp) {
     return ((size_t)(bm + KEYS) * (hd + 4) + (size_t)KEYS * vdp + (size_t)KEYS * (bm + 4) + 4 * bm + 2 * KEYS) * sizeof(float);
 }
@@ -416,9 +325,6 @@ int launch(const F32Args& a, int max_q_len, cudaStream_t stream) {
     if (a.vd <= 128) return launch<BM, 128>(a, max_q_len, stream);
     return launch<BM, 256>(a, max_q_len, stream);
 }
-
-// (vd + 2 floats a row are no multiple of 16 bytes, the outputs are read by 16)
-long long border4(long long floats) { return (floats + 3) / 4 * 4; }
 
 // How a step's stretches are laid over CTAs.
 struct Plan {

@@ -61,6 +61,8 @@ _SIGNATURES = {
     # attention_tc.cu
     "fb_attention_tc_stretches": (I, [L, I, I, I]),
     # attention_f32.cu
+    "fb_attention_f32_tc_scratch_floats": (L, [I, I, I, I, I, I, L]),
+    "fb_attention_f32_tc": (I, [P, L, P, L, P, P, I, I, P, I, P, I, P, P, P, I, I, I, L, I, I, I, I, F, P, P, L, I, L, P, L, P, STREAM]),
     "fb_attention_f32_scratch_floats": (L, [I, I, I, I, I, I, I, I, I, L, L]),
     "fb_paged_attention_f32": (I, [P, L, P, L, P, P, I, I, P, I, P, I, P, P, P, I, I, I, L, L, I, I, I, I, I, I, I, F, F, P, P, P, L, I, L,
                                    P, L, P, STREAM]),

@@ -519,6 +519,20 @@ def paged_attention_f32(q, out, k_pool, v_pool, block_table, seq_q_start, seq_q_
         raise KernelError("attention: cache pools must be contiguous")
     G = nh // nkv
     lens = [int(m) for m in seq_lens] if seq_lens is not None else [max_q_len] * n_seqs
+    if hd == vd == 128 and softcap == 0.0 and score_slopes is None and keep_first == 0:
+        # heads of 128 without extras: the tensor cores (the rule looks at the model alone, never at the rows of the step)
+        tiles = sum(-(-m // (128 // G)) for m in lens)
+        floats = lib().fb_attention_f32_tc_scratch_floats(n, nh, nkv, int(max_q_len), int(max_kv_len), int(window), tiles)
+        part = None
+        if floats > 0:
+            part = alloc(floats) if alloc is not None else torch.empty(floats, dtype=torch.float32, device=q.device)
+        check(lib().fb_attention_f32_tc(
+            q.data_ptr(), _rows(q), out.data_ptr(), _rows(out), k_pool.data_ptr(), v_pool.data_ptr(), page_size, n_pages,
+            block_table.data_ptr(), block_table.stride(0), _ptr(table_base), int(table_head), seq_q_start.data_ptr(),
+            seq_q_len.data_ptr(), seq_pos_start.data_ptr(), n_seqs, max_q_len, int(max_kv_len), tiles, n, nh, nkv, int(window),
+            float(scale), _ptr(sinks), *_head_gate(head_gate, n, nh), _ptr(part), floats, status.data_ptr(), _stream()),
+            "paged_attention_f32")
+        return
     short = [G <= 16 and m * G <= 16 for m in lens] if seq_lens is not None else [not any_long] * n_seqs
     tokens = 64 // G
     short_tiles = sum(short) if seq_lens is not None else n_seqs if any_short else 0
