@@ -1481,7 +1481,7 @@ def head_linear(a, a_head: int, w, out, o_head: int, n: int, n_partials: int = 1
                                      w.data_ptr(), out.data_ptr(), _rows(out), int(o_head), int(n), H, N, K, status.data_ptr(),
                                      _stream())
         if rc != 1:
-            check(rc, "head_linear_tc", (n * H, N, K))
+            check(rc, "head_linear", (n * H, N, K))
             return
     check(lib().fb_head_linear(a.data_ptr(), dtype_code(a), _rows(a), int(a_head), int(n_partials), int(partial_stride),
                                w.data_ptr(), dtype_code(w), out.data_ptr(), dtype_code(out), _rows(out), int(o_head),
