@@ -10,6 +10,9 @@
 //                  takes 64 rows x 64 outputs (or several such tiles one after the other); the middle is rounded once to
 //                  bfloat16
 //   low_rank_fma   any types: float32 multiply-adds, 32 rows x 64 outputs a CTA
+#include <algorithm>
+#include <type_traits>
+
 #include "attention_common.cuh"
 #include "rows.cuh"
 
@@ -155,9 +158,11 @@ __device__ __forceinline__ float lr_finish_fast(int act, float z, float bias, fl
     return z;
 }
 
-template <int NT>
-__global__ void __launch_bounds__(128)
-low_rank_tiles_kernel(const LowRankArgs a) {
+// What bounds it: the functions behind the products, some 25 instructions an output, beside stores of 4 bytes an output.  2,048
+// rows to 2 x 4,096 outputs through 128 columns (a decay and a sigmoid): AAAA us, BBBB with the middles fetched element by element
+// across branches, fragments by 4-byte loads and CTAs of four tiles in two rounds.
+__global__ void __launch_bounds__(128, 4)
+low_rank_tiles_kernel(const LowRankArgs a, int NT) {
     using bf16 = __nv_bfloat16;
     fb_pdl_launch_dependents();
     extern __shared__ __align__(16) unsigned char lt_raw[];
@@ -171,16 +176,23 @@ low_rank_tiles_kernel(const LowRankArgs a) {
     bf16* Ws = As + LM_T * P;                                         // [2][64][P]
     float* col = reinterpret_cast<float*>(Ws + 2 * LM_T * P);         // [2][bias: 64 | rate: 64]
     const bf16* w = static_cast<const bf16*>(m.w);
+    // (thread tid fetches the chunks tid, tid + 128, ... of 8 numbers: their places by addition)
+    const int chunks = K / 8, r_first = tid / chunks, k_first = tid - r_first * chunks, r_step = 128 / chunks, k_step = 128 - r_step * chunks;
     auto fetch = [&](int tile) {
         bf16* dst = Ws + (tile & 1) * LM_T * P;
-        const int n0 = (tile0 + tile) * LM_T, chunks = K / 8;
-        for (int idx = tid; idx < LM_T * chunks; idx += 128) {
-            const int r = idx / chunks, k = (idx - r * chunks) * 8;
-            if (n0 + r < m.N && k < m.R)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + r * P + k)),
-                             "l"(w + (size_t)(n0 + r) * m.R + k) : "memory");
+        const int n0 = (tile0 + tile) * LM_T;
+        for (int r = r_first, k = k_first; r < LM_T;) {
+            if (n0 + r < m.N && 8 * k < m.R)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + r * P + 8 * k)),
+                             "l"(w + (size_t)(n0 + r) * m.R + 8 * k) : "memory");
             else
-                *reinterpret_cast<uint4*>(dst + r * P + k) = make_uint4(0u, 0u, 0u, 0u);
+                *reinterpret_cast<uint4*>(dst + r * P + 8 * k) = make_uint4(0u, 0u, 0u, 0u);
+            r += r_step;
+            k += k_step;
+            if (k >= chunks) {
+                k -= chunks;
+                ++r;
+            }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
         if (tid < LM_T && n0 + tid < m.N) {
@@ -192,26 +204,33 @@ low_rank_tiles_kernel(const LowRankArgs a) {
     fetch(0);                                          // (not of this step: it need not wait for the kernel before)
     fb_pdl_wait();
     const bool a_vec = m.mid_off % 4 == 0 && a.proj_stride % 4 == 0 && a.partial_stride % 4 == 0 && (uintptr_t)a.proj % 16 == 0;
-    const int quads = K / 4;
-#pragma unroll 4
-    for (int idx = tid; idx < LM_T * quads; idx += 128) {
-        const int r = idx / quads, k = (idx - r * quads) * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (m0 + r < a.n && k < m.R) {
-            const float* src = a.proj + (size_t)(m0 + r) * a.proj_stride + m.mid_off + k;
-            if (a_vec) {
-                v = slab_sum4(src, a.n_partials, a.partial_stride);
-            } else {
-                v.x = fb_slab_sum(src, 0, a.n_partials, a.partial_stride); v.y = fb_slab_sum(src, 1, a.n_partials, a.partial_stride);
-                v.z = fb_slab_sum(src, 2, a.n_partials, a.partial_stride); v.w = fb_slab_sum(src, 3, a.n_partials, a.partial_stride);
+    // The middles: a warp's rows eight at a time, their loads unconditional so that all are on their way at once.
+    for (int k = 4 * lane; k < K; k += 128)
+        for (int r0 = warp * 16; r0 < min(warp * 16 + 16, a.n - m0); r0 += 8) {       // (rows behind the last are nobody's)
+            float4 v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const float* src = a.proj + (size_t)min(m0 + r0 + u, a.n - 1) * a.proj_stride + m.mid_off + (k < m.R ? k : 0);
+                if (a_vec) {
+                    v[u] = slab_sum4(src, a.n_partials, a.partial_stride);
+                } else {
+                    v[u].x = fb_slab_sum(src, 0, a.n_partials, a.partial_stride); v[u].y = fb_slab_sum(src, 1, a.n_partials, a.partial_stride);
+                    v[u].z = fb_slab_sum(src, 2, a.n_partials, a.partial_stride); v[u].w = fb_slab_sum(src, 3, a.n_partials, a.partial_stride);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const bool there = m0 + r0 + u < a.n && k < m.R;
+                uint2 raw;
+                raw.x = there ? fb_attn::pack_bf16(v[u].x, v[u].y) : 0u;
+                raw.y = there ? fb_attn::pack_bf16(v[u].z, v[u].w) : 0u;
+                *reinterpret_cast<uint2*>(As + (r0 + u) * P + k) = raw;
             }
         }
-        uint2 raw;
-        raw.x = fb_attn::pack_bf16(v.x, v.y);
-        raw.y = fb_attn::pack_bf16(v.z, v.w);
-        *reinterpret_cast<uint2*>(As + r * P + k) = raw;
-    }
     const bool pairs = m.N % 2 == 0 && (uintptr_t)m.out % 8 == 0;
+    // (ldmatrix: lane l gives the address of row l % 8 of the 8 x 8 block l / 8)
+    const bf16* a_at = As + (warp * 16 + (lane & 15)) * P + (lane >> 4) * 8;
+    const bf16* w_at = Ws + ((lane >> 4) * 8 + (lane & 7)) * P + ((lane >> 3) & 1) * 8;
     for (int tile = 0; tile < tiles; ++tile) {
         if (tile + 1 < tiles) {
             fetch(tile + 1);                           // (its buffer's last readers passed the barrier at the loop's end)
@@ -225,35 +244,40 @@ low_rank_tiles_kernel(const LowRankArgs a) {
             float acc[LM_T / 8][4];
 #pragma unroll
             for (int j = 0; j < LM_T / 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
-            const bf16* ar = As + (warp * 16 + g) * P + 2 * t;
-            const bf16* wr = Ws + (tile & 1) * LM_T * P + g * P + 2 * t;
+            const bf16* w_tile = w_at + (tile & 1) * LM_T * P;
             for (int kk = 0; kk < K; kk += 16) {
                 uint32_t af[4];
-                af[0] = *reinterpret_cast<const uint32_t*>(ar + kk);
-                af[1] = *reinterpret_cast<const uint32_t*>(ar + 8 * P + kk);
-                af[2] = *reinterpret_cast<const uint32_t*>(ar + kk + 8);
-                af[3] = *reinterpret_cast<const uint32_t*>(ar + 8 * P + kk + 8);
+                fb_attn::ldmatrix_x4(af, a_at + kk);
 #pragma unroll
-                for (int j = 0; j < LM_T / 8; ++j)
-                    fb_attn::mma_bf16(acc[j], af, *reinterpret_cast<const uint32_t*>(wr + j * 8 * P + kk),
-                                      *reinterpret_cast<const uint32_t*>(wr + j * 8 * P + kk + 8));
-            }
-            const float* c0 = col + (tile & 1) * 2 * LM_T;
-#pragma unroll
-            for (int j = 0; j < LM_T / 8; ++j) {
-                const int cc = j * 8 + 2 * t, c = n0 + cc;
-                const float b0 = c0[cc], b1 = c0[cc + 1], r0 = c0[LM_T + cc], r1 = c0[LM_T + cc + 1];
-#pragma unroll
-                for (int hi = 0; hi < 2; ++hi) {
-                    const int r = m0 + warp * 16 + g + hi * 8;
-                    if (r >= a.n || c >= m.N) continue;
-                    float* dst = m.out + (size_t)r * m.N + c;
-                    const float y0 = lr_finish_fast(m.act, acc[j][2 * hi], b0, r0), y1 = lr_finish_fast(m.act, acc[j][2 * hi + 1], b1, r1);
-                    if (pairs) { *reinterpret_cast<float2*>(dst) = make_float2(y0, y1); continue; }
-                    dst[0] = y0;
-                    if (c + 1 < m.N) dst[1] = y1;
+                for (int j = 0; j < LM_T / 8; j += 2) {
+                    uint32_t bf[4];                    // outputs 8 j .. and 8 (j + 1) .., channels kk .. and kk + 8 .. of each
+                    fb_attn::ldmatrix_x4(bf, w_tile + j * 8 * P + kk);
+                    fb_attn::mma_bf16(acc[j], af, bf[0], bf[1]);
+                    fb_attn::mma_bf16(acc[j + 1], af, bf[2], bf[3]);
                 }
             }
+            const float* c0 = col + (tile & 1) * 2 * LM_T;
+            auto finish = [&](auto act_of) {           // (the function is the map's: chosen once, not per output)
+                constexpr int ACT = decltype(act_of)::value;
+#pragma unroll
+                for (int j = 0; j < LM_T / 8; ++j) {
+                    const int cc = j * 8 + 2 * t, c = n0 + cc;
+                    const float2 b = *reinterpret_cast<const float2*>(c0 + cc), rate = *reinterpret_cast<const float2*>(c0 + LM_T + cc);
+#pragma unroll
+                    for (int hi = 0; hi < 2; ++hi) {
+                        const int r = m0 + warp * 16 + g + hi * 8;
+                        if (r >= a.n || c >= m.N) continue;
+                        float* dst = m.out + (size_t)r * m.N + c;
+                        const float y0 = lr_finish_fast(ACT, acc[j][2 * hi], b.x, rate.x), y1 = lr_finish_fast(ACT, acc[j][2 * hi + 1], b.y, rate.y);
+                        if (pairs) { *reinterpret_cast<float2*>(dst) = make_float2(y0, y1); continue; }
+                        dst[0] = y0;
+                        if (c + 1 < m.N) dst[1] = y1;
+                    }
+                }
+            };
+            if (m.act == FB_LR_DECAY) finish(std::integral_constant<int, FB_LR_DECAY>());
+            else if (m.act == FB_LR_SIGMOID) finish(std::integral_constant<int, FB_LR_SIGMOID>());
+            else finish(std::integral_constant<int, FB_LR_PLAIN>());
         }
         __syncthreads();
     }
@@ -336,14 +360,16 @@ FB_API int fb_low_rank_maps(const float* proj, long long proj_stride, int n_part
             widest = R[i] > widest ? R[i] : widest;
         }
         if (resident) {
-            const int NT = n > 64 ? 4 : 1;             // (few rows: the tiles spread over the device)
-            auto groups = [&](int i) { return ((N[i] + LM_T - 1) / LM_T + NT - 1) / NT; };
-            a.tiles_first = groups(0);
-            const dim3 grid((n + LM_T - 1) / LM_T, groups(0) + (count > 1 ? groups(1) : 0));
-            auto kernel = NT == 4 ? low_rank_tiles_kernel<4> : low_rank_tiles_kernel<1>;
+            // Tiles a CTA: as few as let all CTAs in at once (few rows spread over the device), at most 16.
             const size_t smem = lt_smem(widest);
-            if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            fb_launch(kernel, grid, dim3(128), smem, stream, a);
+            const long blocks = (n + LM_T - 1) / LM_T, slots = (long)fb_sm_count() * std::min<long>(4, 220 * 1024 / (long)(smem + 1024));
+            int NT = 1;
+            auto groups = [&](int i) { return ((N[i] + LM_T - 1) / LM_T + NT - 1) / NT; };
+            while (NT < 16 && blocks * (groups(0) + (count > 1 ? groups(1) : 0)) > slots) ++NT;
+            a.tiles_first = groups(0);
+            const dim3 grid((unsigned)blocks, groups(0) + (count > 1 ? groups(1) : 0));
+            if (smem > 48 * 1024) cudaFuncSetAttribute(low_rank_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            fb_launch(low_rank_tiles_kernel, grid, dim3(128), smem, stream, a, NT);
             return fb_check_launch("low_rank_maps");
         }
         fb_launch(low_rank_mma_kernel, dim3((n + LM_T - 1) / LM_T, tiles), dim3(128), 0, stream, a);
