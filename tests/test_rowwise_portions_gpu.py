@@ -52,6 +52,44 @@ def test_query_key_norms_of_portions(sizes, dtype):
         assert float(got[0][0].float().abs().max()) > 0
 
 
+def fma(a, b, c):
+    """Rounded once: a float32 product is exact in float64 (and twice-rounded sums are rare: none among these numbers)."""
+    return (a.double() * b.double() + c.double()).float()
+
+
+@pytest.mark.parametrize("n", [20, 77])                # (a warp a head; a CTA a row)
+@pytest.mark.parametrize("d,rot", [(32, 24), (64, 64), (64, 0), (128, 128), (128, 64)])
+def test_order_of_the_norm_and_the_rotation(n, d, rot):
+    """Bit by bit what the sum of squares and the rotation are written as."""
+    from flambeau_b200.cache.manager import LayerCacheView
+    from flambeau_b200.kernels import ops
+    H, half, page = 6, rot // 2, 8
+    g = torch.Generator(device=DEV).manual_seed(d + n)
+    proj = torch.randn(n, 2 * H * d + H * d, generator=g, device=DEV)
+    weight = torch.randn(d, generator=g, device=DEV) + 2.0
+    angles = torch.randn(n, max(half, 1), generator=g, device=DEV)
+    cos, sin = angles.cos(), angles.sin()
+    pools = [torch.zeros(10, H, page, d, device=DEV) for _ in range(2)]
+    cache = LayerCacheView(*pools, i32([list(range(10))]), i32([0]), page, True, 0, None)
+    for norm in (False, True):
+        q, status = torch.zeros(n, H * d, device=DEV), i32([0])
+        ops.qk_norm_rope_kv_write(proj, weight if norm else None, weight if norm else None, "head" if norm else None, 1e-3, 0.0,
+                                  cos if rot else None, sin if rot else None, half, q, cache, i32(list(range(n))), i32([0] * n), H, H, d, d, status)
+        assert int(status) == 0
+        keys = pools[0].transpose(1, 2).reshape(-1, H, d)[:n]
+        for got, x in ((q.view(n, H, d), proj[:, :H * d].view(n, H, d)), (keys, proj[:, H * d:2 * H * d].view(n, H, d))):
+            if norm:
+                v = x.reshape(n, H, d // 4, 4).unbind(-1)
+                s = fma(v[3], v[3], fma(v[2], v[2], fma(v[0], v[0], v[1] * v[1])))
+                while s.shape[-1] > 1:                 # lanes that differ in their highest bit meet first
+                    s = s[..., :s.shape[-1] // 2] + s[..., s.shape[-1] // 2:]
+                x = x * ((1.0 / torch.sqrt(s / d + 1e-3)) * weight)
+            if rot:
+                a, b, c, e = x[..., :half], x[..., half:rot], cos[:, None], sin[:, None]
+                x = torch.cat([fma(b, -e, a * c), fma(a, e, b * c), x[..., rot:]], -1)
+            assert torch.equal(got, x)
+
+
 @pytest.mark.parametrize("sizes", [(2, 4, 128, 128, 4), (1, 3, 20, 36, 3), (2, 2, 136, 256, 4), (3, 3, 64, 8, 2), (2, 4, 32, 32, 1)], ids=str)
 @pytest.mark.parametrize("lengths", [(77,), (3, 1, 70), (40, 9, 2, 30), (1, 1, 8, 7, 60)], ids=str)
 def test_recurrences_prepared_in_portions(sizes, lengths):
