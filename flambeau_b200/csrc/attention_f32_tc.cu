@@ -127,7 +127,6 @@ attention_f32_tc_kernel(const __grid_constant__ F32Args a) {
     const int G = a.nh / a.nkv;
     const int pair = blockIdx.x / a.token_tiles, tile = blockIdx.x - pair * a.token_tiles;
     const int seq = pair / a.nkv, kvh = pair - seq * a.nkv;
-    fb_pdl_launch_dependents();
     fb_pdl_wait();
     const int q_len = a.seq_q_len[seq], TQ = TROWS / G;
     const int tok0 = (a.token_tiles - 1 - tile) * TQ;            // later tokens see more keys: start them first
@@ -164,6 +163,7 @@ attention_f32_tc_kernel(const __grid_constant__ F32Args a) {
     if (warp == 11) tmem_alloc(tmem_slot, 512);                  // (behind the wait: the kernels ahead have given theirs back)
     tmem_fence_before();
     __syncthreads();
+    fb_pdl_launch_dependents();                                  // (behind the allocation: see umma.cuh)
     tmem_fence_after();
     const uint32_t tmem = *tmem_slot;
     auto wait_for = [&](uint32_t bar, int phase) { return mbar_wait(bar, (uint32_t)phase & 1u, a.status); };

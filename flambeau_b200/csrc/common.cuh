@@ -91,8 +91,10 @@ __device__ __forceinline__ float fb_plain_act(int act, float z) {
 // ---- launches ---------------------------------------------------------------
 // Kernels of a step run back to back on one stream.  With programmatic dependent launch the next kernel of the
 // stream may be scheduled while this one is still draining: every kernel begins with fb_pdl_launch_dependents()
-// (which lets the kernel after it start being placed once all of this kernel's blocks have begun) and calls
+// (which lets the kernel after it start being placed once all of this kernel's blocks have come that far) and calls
 // fb_pdl_wait() before its first read of what the kernel before it produced and before its first global write.
+// A kernel that takes tensor memory lets dependents in only behind its allocation and a barrier of the block: a block of the
+// kernel after it that got its columns first would hold them until this kernel ends, which then cannot (umma.cuh).
 // fb_pdl_wait() returns once all earlier kernels of the stream have completed and their writes are visible, so
 // the order of results is that of ordinary stream launches; only launch latency and prologues overlap.
 extern int g_fb_pdl;        // 1: launch with the programmatic-serialization attribute; 0: plain launches

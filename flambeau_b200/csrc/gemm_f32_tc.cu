@@ -186,7 +186,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
-    fb_pdl_launch_dependents();                  // (behind the allocation: no later kernel's CTA can take its columns first)
+    fb_pdl_launch_dependents();                  // (behind the allocation: see umma.cuh)
     const uint32_t tmem = *tmem_slot;
     auto stages_of = [&](const FUnit& w) { return min(w.last * SHARE_STAGES, a.stages) - w.first * SHARE_STAGES; };
 

@@ -48,13 +48,15 @@ head_linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         for (int k = 0; k < K; k += HT_KB)
             tma_load_2d(smem_u32(Ws + (size_t)(k / HT_KB) * N * 128), &map_w, smem_u32(&bars[0]), k, h * N);
     }
-    fb_pdl_launch_dependents();
     fb_pdl_wait();
     if (BY_TMA && tid == 0)
         for (int k = 0; k < K; k += HT_KB)
             tma_load_2d(smem_u32(As + k / HT_KB * HT_BLOCK), &map_a, smem_u32(&bars[0]), (int)(h * a_head) + k, m0);
-    // (behind the wait: a CTA of the kernel before may not have taken its tensor memory yet)
+    // (behind the wait, so that it waits for no column of the kernel before; dependents behind it, who could hold theirs for good)
     if (warp == 1) tmem_alloc(tmem_slot, cols);
+    tmem_fence_before();
+    __syncthreads();
+    fb_pdl_launch_dependents();
     if (!BY_TMA) {
         constexpr int U = 8;                            // groups of four numbers a thread has in flight
         const float* from = reinterpret_cast<const float*>(a) + (size_t)h * a_head;
@@ -87,9 +89,8 @@ head_linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
     }
-    tmem_fence_before();
-    __syncthreads();
     tmem_fence_after();
     const uint32_t tmem = *tmem_slot;
     bool ok = true;

@@ -63,7 +63,10 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
 __device__ __forceinline__ void tmem_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tmem_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// A whole warp allocates `cols` columns (a power of two >= 32) of tensor memory; the base address lands in *slot.
+// A whole warp allocates `cols` columns (a power of two >= 32) of tensor memory; the base address lands in *slot.  The
+// instruction waits, without a limit, until the SM has as many columns to give.  What holds them may be a block of an earlier
+// kernel, which ends by itself, or one of the kernel after this one, placed early, which does not end before this kernel has:
+// hence no fb_pdl_launch_dependents() ahead of the allocation, in any thread of the block, and a __syncthreads() between them.
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                  ::"r"(smem_u32(slot)), "r"(cols) : "memory");

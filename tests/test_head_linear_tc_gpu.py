@@ -38,3 +38,32 @@ def test_left_to_the_other_kernel():
         ops.head_linear(a, K, w, outs[0], N, n, status=status)
         ops.head_linear(a, K, w, outs[1], N, n)
         assert torch.equal(*outs) and float(outs[0].abs().max()) > 0
+
+
+@pytest.mark.parametrize("rank", [64, 128])
+def test_a_portion_whose_maps_and_attention_fit_an_sm_together(rank):
+    """Latents of 64 and 128: a block of the map and one of the attention behind it, which takes all of tensor memory before it
+    waits, have room on an SM side by side; more of both than there are SMs."""
+    from flambeau_b200.cache.manager import CallPlan
+    from flambeau_b200.parts.latent_attention import LatentAttention
+    from test_parts_gpu import Bench, bind_random, rel
+    n, w, H, d, e = 1280, 256, 16, 128 if rank == 64 else 64, 64
+    part = LatentAttention(None, "m.", width=w, num_heads=H, head_dim=d, rot_dim=0, value_dim=e, kv_rank=rank, q_rank=None,
+                           window=0, scale=d ** -0.5, eps=1e-5, gate=False)
+    b = Bench("bfloat16", [CallPlan(kv=part.cache_requirement())], cache_tokens=4096, max_step_tokens=n)
+    part.runtime = b.rt
+    W = {name[2:]: t for name, t in bind_random(part, torch.bfloat16).items()}
+    ctx, _ = b.begin([("a", [1] * n, [])], w)
+    h = torch.randn(n, w, generator=torch.Generator().manual_seed(rank)).bfloat16()
+    part.forward(ctx, h.cuda(), ctx.delta, 0)
+    b.end()
+    y = ctx.delta_slabs[:ctx.pending_slabs].sum(0)
+    h = h.double()
+    z = h @ W["dkv"].T
+    c = z / torch.sqrt((z * z).mean(-1, keepdim=True) + 1e-5) * W["dkv.norm"]
+    q = (h @ W["q"].T).view(n, H, d)
+    uk, uv = W["uk"].view(H, d, rank), W["uv"].view(H, e, rank)
+    seen = torch.ones(n, n, dtype=torch.bool).tril()
+    heads = [torch.softmax((q[:, i] @ uk[i] @ c.T * d ** -0.5).masked_fill(~seen, -torch.inf), -1) @ c @ uv[i].T for i in range(H)]
+    # five roundings to bfloat16 on the way (queries, latents, both maps' results, heads), of numbers no larger than the result's
+    assert rel(y, torch.cat(heads, -1) @ W["o"].T) < 5 * 2.0 ** -9

@@ -1,4 +1,9 @@
-"""Rules by which launches are cut, on the CPU."""
+"""Rules by which launches are cut and placed, on the CPU."""
+import re
+
+import pytest
+
+from flambeau_b200.kernels.build import CSRC
 from flambeau_b200.kernels.library import lib
 
 SMS = 148
@@ -20,3 +25,27 @@ def test_stretches_of_decoded_tokens_over_latents_fill_whole_rounds():
             s = lib().fb_attention_tc_stretches(pairs, tiles, 64, SMS)
             assert 1 <= s <= -(-tiles // 4)
     assert lib().fb_attention_tc_stretches(8, 125, 0, SMS) == 0 and lib().fb_attention_tc_stretches(8, 125, 2, SMS) == 2
+
+
+def kernels(path):
+    """(name, source) of every kernel of a file."""
+    text = re.sub(r"//[^\n]*", "", path.read_text())
+    for m in re.finditer(r"__global__[^;{]*?(\w+)\(const __grid_constant__[^{]*\{", text):
+        depth, end = 1, m.end()
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[end], 0)
+            end += 1
+        yield m.group(1), text[m.end():end]
+
+
+@pytest.mark.parametrize("file", ["attention_f32_tc", "gemm_f32_tc", "head_linear_tc"])
+def test_dependents_come_behind_tensor_memory(file):
+    """A kernel placed early that got its columns first would wait for this one's end, and this one for its columns."""
+    found = 0
+    for name, source in kernels(CSRC / f"{file}.cu"):
+        alloc = re.search(r"tmem_alloc\(|tcgen05\.alloc", source)
+        if alloc:
+            found += 1
+            lets_in = source.index("fb_pdl_launch_dependents()")
+            assert alloc.start() < lets_in and "__syncthreads()" in source[alloc.start():lets_in], name
+    assert found == 1
