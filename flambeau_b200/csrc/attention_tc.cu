@@ -104,7 +104,6 @@ template <int HD, int RT, bool SHARED, bool DIFF> struct TcSmem {
 template <int HD, int RT, bool HILO, bool SHARED, bool DIFF, bool SPLIT>
 __global__ void __launch_bounds__(tc_threads(RT), 1)
 attention_tc_kernel(const __grid_constant__ AttnArgs a) {
-    fb_pdl_launch_dependents();
     static_assert(RT * 128 + RT * (HD > 128 ? HD : 128) <= TMEM_COLS, "tensor memory");
     static_assert(!DIFF || (HD == 128 && RT == 2 && !SHARED), "two maps of 64 over values of 128");
     using SM = TcSmem<HD, RT, SHARED, DIFF>;
@@ -200,6 +199,7 @@ attention_tc_kernel(const __grid_constant__ AttnArgs a) {
     if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
     tmem_fence_before();
     __syncthreads();
+    fb_pdl_launch_dependents();                                 // (behind the allocation: see umma.cuh)
     tmem_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     fb_pdl_wait();                                              // from here on: Q and the cache

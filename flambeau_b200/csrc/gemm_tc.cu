@@ -95,7 +95,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     int* last_flag = (int*)(tmem_slot + 1);
     int* bail = last_flag + 1;                   // a bounded wait ran out somewhere in this CTA
 
-    fb_pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kb_total = (K + Cfg::KSTEP - 1) / Cfg::KSTEP;
 
@@ -118,6 +117,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    fb_pdl_launch_dependents();                  // (behind the allocation: see umma.cuh)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
 

@@ -180,7 +180,6 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
     uint32_t* list = (uint32_t*)(out_stage + 4 * P_OUT_BYTES);
 
-    fb_pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const int pair = blockIdx.x >> 1;
@@ -204,15 +203,19 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                      ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)P_TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
-    if (GROUPED && warp == 2) {
-        fb_pdl_wait();                           // which weights a tile wants is the work of the kernels before this one
-        const int found = group_units(tile_group, n_tiles, list);
-        if (lane == 0) *group_count = found;
-    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     cluster_sync_all();                          // both CTAs' barriers exist before either signals the other's
+    fb_pdl_launch_dependents();                  // (behind the allocation: see umma.cuh)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (GROUPED) {
+        if (warp == 2) {
+            fb_pdl_wait();                       // which weights a tile wants is the work of the kernels before this one
+            const int found = group_units(tile_group, n_tiles, list);
+            if (lane == 0) *group_count = found;
+        }
+        __syncthreads();
+    }
     const uint32_t tmem_base = *tmem_slot;
     // Feature tiles vary fastest in the grouped form: a group's weights serve its units of tokens while they are in L2, and the
     // units that run together share few units' rows.

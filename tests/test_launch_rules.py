@@ -38,7 +38,10 @@ def kernels(path):
         yield m.group(1), text[m.end():end]
 
 
-@pytest.mark.parametrize("file", ["attention_f32_tc", "gemm_f32_tc", "head_linear_tc"])
+TAKE_TENSOR_MEMORY = sorted(p.stem for p in CSRC.glob("*.cu") if re.search(r"tmem_alloc\(|tcgen05\.alloc", p.read_text()))
+
+
+@pytest.mark.parametrize("file", TAKE_TENSOR_MEMORY)
 def test_dependents_come_behind_tensor_memory(file):
     """A kernel placed early that got its columns first would wait for this one's end, and this one for its columns."""
     found = 0
