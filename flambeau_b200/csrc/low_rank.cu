@@ -11,6 +11,7 @@
 //                  bfloat16
 //   low_rank_fma   any types: float32 multiply-adds, 32 rows x 64 outputs a CTA
 #include <algorithm>
+#include <climits>
 #include <type_traits>
 
 #include "attention_common.cuh"
@@ -158,9 +159,11 @@ __device__ __forceinline__ float lr_finish_fast(int act, float z, float bias, fl
     return z;
 }
 
-// What bounds it: the functions behind the products, some 25 instructions an output, beside stores of 4 bytes an output.  2,048
-// rows to 2 x 4,096 outputs through 128 columns (a decay and a sigmoid): AAAA us, BBBB with the middles fetched element by element
-// across branches, fragments by 4-byte loads and CTAs of four tiles in two rounds.
+// What bounds it: the functions behind the products, some 25 instructions an output, beside stores of 4 bytes an output; for few
+// rows the way of the middles into shared memory.  To 2 x 4,096 outputs (a decay and a sigmoid) through 128 columns of one share /
+// of three: 2,048 rows 50 / 51 us, 343 rows 14 / 16, 65 rows 7.6 / 9.2; with the middles fetched one by one across branches,
+// fragments by 4-byte loads and CTAs of four tiles 55 / 67, 26 / 31 and 24 / 28.  Through 16 columns 2,048 rows 27 (30 so), but
+// 4,096 rows 54 (51): those CTAs had fewer registers, and six of them an SM hide the functions better than four.
 __global__ void __launch_bounds__(128, 4)
 low_rank_tiles_kernel(const LowRankArgs a, int NT) {
     using bf16 = __nv_bfloat16;
@@ -204,29 +207,66 @@ low_rank_tiles_kernel(const LowRankArgs a, int NT) {
     fetch(0);                                          // (not of this step: it need not wait for the kernel before)
     fb_pdl_wait();
     const bool a_vec = m.mid_off % 4 == 0 && a.proj_stride % 4 == 0 && a.partial_stride % 4 == 0 && (uintptr_t)a.proj % 16 == 0;
-    // The middles: a warp's rows eight at a time, their loads unconditional so that all are on their way at once.
-    for (int k = 4 * lane; k < K; k += 128)
-        for (int r0 = warp * 16; r0 < min(warp * 16 + 16, a.n - m0); r0 += 8) {       // (rows behind the last are nobody's)
-            float4 v[8];
+    // The middles of a warp's 16 rows, four columns an item; an item's loads are unconditional, so that those of U items are on
+    // their way at once.
+    const int quads = K / 4, rows = min(16, a.n - m0 - warp * 16);                  // (rows behind the last are nobody's)
+    const int r_more = 32 / quads, q_more = 32 - r_more * quads;                      // from an item to the lane's next
+    const float* mids = a.proj + (size_t)(m0 + warp * 16) * a.proj_stride + m.mid_off;
+    auto stage = [&](auto at_once) {
+        constexpr int U = decltype(at_once)::value;
+        for (int i = lane, r = lane / quads, q = lane - r * quads; i < rows * quads; i += 32 * U) {
+            float4 v[U];
+            const float* src[U];
+            int to[U];
+            bool there[U];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const float* src = a.proj + (size_t)min(m0 + r0 + u, a.n - 1) * a.proj_stride + m.mid_off + (k < m.R ? k : 0);
-                if (a_vec) {
-                    v[u] = slab_sum4(src, a.n_partials, a.partial_stride);
-                } else {
-                    v[u].x = fb_slab_sum(src, 0, a.n_partials, a.partial_stride); v[u].y = fb_slab_sum(src, 1, a.n_partials, a.partial_stride);
-                    v[u].z = fb_slab_sum(src, 2, a.n_partials, a.partial_stride); v[u].w = fb_slab_sum(src, 3, a.n_partials, a.partial_stride);
+            for (int u = 0; u < U; ++u) {
+                there[u] = 4 * q < m.R;
+                src[u] = mids + (size_t)min(r, rows - 1) * a.proj_stride + (there[u] ? 4 * q : 0);
+                to[u] = r < rows ? (warp * 16 + r) * P + 4 * q : -1;
+                r += r_more;
+                q += q_more;
+                if (q >= quads) { q -= quads; ++r; }
+            }
+            if (a_vec && a.n_partials == 1) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) v[u] = Vec4<float>::load(src[u]);
+            } else if (a_vec && a.n_partials <= 3 && U > 1) {     // (no loop between the loads of two items)
+                const bool third = a.n_partials == 3;
+                const long second_at = a.partial_stride, third_at = third ? 2 * a.partial_stride : 0;
+#pragma unroll
+                for (int u0 = 0; u0 + 4 <= U; u0 += 4) {
+                    float4 x[4], y[4], z[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        x[u] = Vec4<float>::load(src[u0 + u]);
+                        y[u] = Vec4<float>::load(src[u0 + u] + second_at);
+                        z[u] = Vec4<float>::load(src[u0 + u] + third_at);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const float4 s = make_float4(x[u].x + y[u].x, x[u].y + y[u].y, x[u].z + y[u].z, x[u].w + y[u].w);
+                        v[u0 + u] = third ? make_float4(s.x + z[u].x, s.y + z[u].y, s.z + z[u].z, s.w + z[u].w) : s;
+                    }
                 }
+            } else if (a_vec) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) v[u] = slab_sum4(src[u], a.n_partials, a.partial_stride);
+            } else {
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    v[u] = make_float4(fb_slab_sum(src[u], 0, a.n_partials, a.partial_stride), fb_slab_sum(src[u], 1, a.n_partials, a.partial_stride),
+                                       fb_slab_sum(src[u], 2, a.n_partials, a.partial_stride), fb_slab_sum(src[u], 3, a.n_partials, a.partial_stride));
             }
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const bool there = m0 + r0 + u < a.n && k < m.R;
-                uint2 raw;
-                raw.x = there ? fb_attn::pack_bf16(v[u].x, v[u].y) : 0u;
-                raw.y = there ? fb_attn::pack_bf16(v[u].z, v[u].w) : 0u;
-                *reinterpret_cast<uint2*>(As + (r0 + u) * P + k) = raw;
-            }
+            for (int u = 0; u < U; ++u)
+                if (to[u] >= 0)
+                    *reinterpret_cast<uint2*>(As + to[u]) = there[u] ? make_uint2(fb_attn::pack_bf16(v[u].x, v[u].y), fb_attn::pack_bf16(v[u].z, v[u].w))
+                                                                     : make_uint2(0u, 0u);
         }
+    };
+    if (rows * quads <= 64) stage(std::integral_constant<int, 1>());
+    else stage(std::integral_constant<int, 8>());
     const bool pairs = m.N % 2 == 0 && (uintptr_t)m.out % 8 == 0;
     // (ldmatrix: lane l gives the address of row l % 8 of the 8 x 8 block l / 8)
     const bf16* a_at = As + (warp * 16 + (lane & 15)) * P + (lane >> 4) * 8;
@@ -360,14 +400,23 @@ FB_API int fb_low_rank_maps(const float* proj, long long proj_stride, int n_part
             widest = R[i] > widest ? R[i] : widest;
         }
         if (resident) {
-            // Tiles a CTA: as few as let all CTAs in at once (few rows spread over the device), at most 16.
+            // Tiles a CTA, by the time of the fullest SM: its CTAs one after the other, a CTA's tiles and the fetch of its rows
+            // (a tile's time for 48 columns); fewer than four CTAs on an SM do not keep it busy.  Measured over 1 to 16 tiles, 65
+            // to 4,096 rows and middles of 16 to 256, three shares (us, one tile / the rule's / sixteen): 2,048 rows to 2 x 4,096
+            // through 16 columns 43 / 30 (four) / 62, through 128 101 / 58 (eight) / 95, through 256 310 / 119 (sixteen); 343
+            // rows through 128 28 / 21 (two) / 71; 65 rows 14 (one) / 71.
             const size_t smem = lt_smem(widest);
-            const long blocks = (n + LM_T - 1) / LM_T, slots = (long)fb_sm_count() * std::min<long>(4, 220 * 1024 / (long)(smem + 1024));
+            const long blocks = (n + LM_T - 1) / LM_T, busy = std::min<long>(4, 220 * 1024 / (long)(smem + 1024));
+            auto groups = [&](int i, int nt) { return ((N[i] + LM_T - 1) / LM_T + nt - 1) / nt; };
             int NT = 1;
-            auto groups = [&](int i) { return ((N[i] + LM_T - 1) / LM_T + NT - 1) / NT; };
-            while (NT < 16 && blocks * (groups(0) + (count > 1 ? groups(1) : 0)) > slots) ++NT;
-            a.tiles_first = groups(0);
-            const dim3 grid((unsigned)blocks, groups(0) + (count > 1 ? groups(1) : 0));
+            long best = LONG_MAX;
+            for (int nt = 1; nt <= 16; ++nt) {
+                const long ctas = blocks * (groups(0, nt) + (count > 1 ? groups(1, nt) : 0));
+                const long cost = (48L * nt + widest) * std::max((ctas + fb_sm_count() - 1) / fb_sm_count(), busy);
+                if (cost < best) { best = cost; NT = nt; }
+            }
+            a.tiles_first = groups(0, NT);
+            const dim3 grid((unsigned)blocks, groups(0, NT) + (count > 1 ? groups(1, NT) : 0));
             if (smem > 48 * 1024) cudaFuncSetAttribute(low_rank_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             fb_launch(low_rank_tiles_kernel, grid, dim3(128), smem, stream, a, NT);
             return fb_check_launch("low_rank_maps");

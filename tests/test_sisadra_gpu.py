@@ -258,6 +258,34 @@ def test_maps_through_narrow_middles(shape, dtype):
                 assert float((out.double().cpu() - ref).abs().max()) / max(1.0, float(ref.abs().max())) < (5e-6 if dtype == "float32" else 4e-3)
 
 
+@pytest.mark.parametrize("shares", [1, 2, 3, 5])
+# (with 148 SMs a CTA takes 1, 2, 8, 16 and 4 tiles of outputs, the last one of a map fewer)
+@pytest.mark.parametrize("shape", [(65, 24, 200, 128, 4100), (400, 128, 4160, 16, 3100), (2049, 128, 4096, 120, 4160), (2048, 256, 4096, 248, 4100),
+                                   (2050, 16, 4160, 8, 4100)], ids=str)
+def test_maps_of_portions_through_narrow_middles(shape, shares):
+    """CTAs of several tiles, whose weights come a tile ahead."""
+    from flambeau_b200.kernels import ops
+    n, R1, N1, R2, N2 = shape
+    g = torch.Generator(device=DEV).manual_seed(n)
+    z = torch.randn(shares, n, R1 + R2 + 8, generator=g, device=DEV) * 0.6
+    w1, w2 = (torch.randn(N, R, generator=g, device=DEV).bfloat16() * 0.1 for N, R in ((N1, R1), (N2, R2)))
+    bias, rate = (torch.randn(k, generator=g, device=DEV).bfloat16() for k in (N1, -(-N1 // 128)))
+    outs = [torch.full((n, N), float("nan"), device=DEV) for N in (N1, N2)]
+    ops.low_rank_maps(z[0], [ops.LowRankMap(w1, 8, outs[0], "decay", bias=bias, log_rate=rate, group=128), ops.LowRankMap(w2, 8 + R1, outs[1], "sigmoid")],
+                      n_partials=shares, partial_stride=z.stride(0))
+    mid = z[0]
+    for share in z[1:]:
+        mid = mid + share                                    # (the middle is summed in the order of its shares and rounded once)
+    mid = mid.bfloat16().double()
+    y1, y2 = mid[:, 8:8 + R1] @ w1.double().T + bias.double(), mid[:, 8 + R1:] @ w2.double().T
+    e1, e2 = (2.0 ** -23 * R * (mid[:, a:a + R].abs() @ w.double().abs().T + 1) for a, R, w in ((8, R1, w1), (8 + R1, R2, w2)))
+    rates = torch.exp(rate.double())[torch.arange(N1, device=DEV) // 128]
+    # a float32 sum of R products; the functions' slopes are at most the rate (of what falls below 1) and a quarter, their own
+    # error a few units of 2^-21 (approximate exponentials, logarithms and quotients)
+    assert bool(((outs[0].double() - torch.exp(-rates * ps.softplus(y1))).abs() <= (rates * e1).clamp(max=1) + 2.0 ** -20 * (1 + rates)).all())
+    assert bool(((outs[1].double() - torch.sigmoid(y2)).abs() <= e2 / 4 + 2.0 ** -20).all())
+
+
 @pytest.mark.parametrize("sizes", [(4, 2, 8, 16, 4), (2, 1, 16, 24, 3), (3, 3, 24, 8, 2), (2, 2, 40, 12, 1), (1, 1, 136, 72, 4),
                                    (4, 1, 300, 20, 2), (2, 1, 64, 128, 4), (2, 1, 128, 128, 4), (3, 1, 10, 6, 3), (1, 1, 513, 4, 2)], ids=str)
 def test_delta_rule_with_a_decay_per_channel_across_steps(sizes):
