@@ -259,7 +259,7 @@ def test_maps_through_narrow_middles(shape, dtype):
 
 
 @pytest.mark.parametrize("shares", [1, 2, 3, 5])
-# (with 148 SMs a CTA takes 1, 2, 8, 16 and 4 tiles of outputs, the last one of a map fewer)
+# (with 148 SMs a CTA takes 1, 2, 8, 16 and 6 tiles of outputs, the last one of a map fewer)
 @pytest.mark.parametrize("shape", [(65, 24, 200, 128, 4100), (400, 128, 4160, 16, 3100), (2049, 128, 4096, 120, 4160), (2048, 256, 4096, 248, 4100),
                                    (2050, 16, 4160, 8, 4100)], ids=str)
 def test_maps_of_portions_through_narrow_middles(shape, shares):
