@@ -17,9 +17,10 @@
 // that the tile's maximum asks for: nothing is summed in tensor memory over more than 128 channels or 64 keys.
 //
 // Numbers from 1e18 on, infinities and NaN, whose parts or products may overflow: a tile that holds one, or a row whose query
-// does, is computed by the row's threads in float32 multiply-adds, key by key, and what a row does not see does not reach it; so
-// is a tile whose values are all below 1e-24 (parts below bfloat16's range would be lost; what queries, keys and weights lose
-// there changes a score by less than 1e-20).
+// does, is computed by the row's threads in float32 multiply-adds, key by key, and what a row does not see does not reach it.
+// Values are multiplied by 2^48 on their way into parts and their products by 2^-48 on the way out, so that every part of every
+// float32 (subnormal ones too) is a normal bfloat16; what queries, keys and weights lose below bfloat16's range changes a score
+// by less than 1e-20.
 //
 // What bounds it: shared memory, 4,900 cycles a tile (72 MMAs' operands 3,070, the stage and the parts written and read 1,800);
 // decoded tokens take 4,800 a tile, full rows 6,700, the three warps that split being the longest chain there.  What a loop runs
@@ -42,7 +43,8 @@ constexpr int T_SMEM = 3 * Q_PART + 6 * KV_PART + STAGE + 2048 + 640;
 static_assert(T_SMEM <= 227 * 1024, "shared memory of an SM");
 constexpr int COL_SL = 0, COL_SS = 64, COL_P = 128, COL_OL = 256, COL_OS = 384;
 constexpr int BAD_K = 1, BAD_V = 2, GAPS = 4;    // a tile with keys or values that have no parts; with keys that nobody sees or without a page
-constexpr float T_MOST = 1.0e18f, T_LEAST = 1.0e-24f;  // (2^60, 2^-80)
+constexpr float T_MOST = 1.0e18f;        // (2^60)
+constexpr float V_IN = 281474976710656.0f, V_OUT = 1.0f / V_IN;          // (2^48: sums of 64 weighted values stay below 2^114)
 
 __device__ __forceinline__ void split2(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(b), "f"(a));
@@ -258,7 +260,8 @@ attention_f32_tc_kernel(const __grid_constant__ F32Args a) {
                 if ((values ? i > 0 : i >= 0) && ok) settle(!bailed() && wait(values ? pv_done : s_full, i - values));
                 int flag = __any_sync(0xffffffffu, !(most < T_MOST)) ? (values ? BAD_V : BAD_K) : 0;
                 if (values) {
-                    if (!__any_sync(0xffffffffu, most >= T_LEAST || most == 0.0f)) flag = BAD_V;
+#pragma unroll
+                    for (int j = 0; j < R; ++j) v[j] = make_float4(v[j].x * V_IN, v[j].y * V_IN, v[j].z * V_IN, v[j].w * V_IN);
                 } else {
                     if (missing_k) flag |= GAPS;
                     // (set next by whom these keys' scores have reached; read last six tiles ago)
@@ -384,7 +387,7 @@ attention_f32_tc_kernel(const __grid_constant__ F32Args a) {
                 float x[16], y[16];
                 tmem_ld16_two(lanes + (uint32_t)(COL_OL + half * 64 + c0), lanes + (uint32_t)(COL_OS + half * 64 + c0), x, y);
 #pragma unroll
-                for (int c = 0; c < 16; ++c) o[c0 + c] = fmaf(o[c0 + c], corr, slow ? 0.0f : x[c] + y[c]);
+                for (int c = 0; c < 16; ++c) o[c0 + c] = fmaf(o[c0 + c], corr, slow ? 0.0f : (x[c] + y[c]) * V_OUT);
             }
             if (slow)
                 for (int t = max(tile_start(i), t0_row); t <= min(tile_start(i) + TKEYS - 1, p_row); ++t) {

@@ -99,6 +99,28 @@ def test_a_value_without_parts():
     assert bool(((got - want).abs() <= bound).all()) and float(want[90:130].abs().max()) < 1e3
 
 
+@pytest.mark.parametrize("power", [-60, -83, -100, -110, -121])
+@pytest.mark.parametrize("beside", ["nothing", "zeros", "ordinary channels", "a value of 1e17"])
+def test_results_scale_with_the_values(power, beside):
+    """Values smaller by a power of two give the same bits as much smaller, down to where a value's lowest part lies below
+    bfloat16's range, whatever lies beside them in their tile."""
+    def spoil(factor):
+        def change(k, v):
+            for x in v:
+                x[..., :64] *= factor
+            if beside == "zeros":
+                v[0][..., 40:], v[1][..., ::2] = 0.0, 0.0
+            elif beside == "a value of 1e17":
+                v[0][250, :, 100], v[1][20, :, 100] = 1e17, -1e17
+            elif beside == "nothing":
+                v[0][..., 64:], v[1][..., 64:] = v[0][..., :64], v[1][..., :64]
+        return change
+    sc = Scene([(300, 90), (0, 50)], 4, 2, 128, 0, torch.float32, seed=5)
+    got, whole = (run(sc, 4, 2, 0, False, spoil(2.0 ** p))[0][..., :64] for p in (power, 0))
+    # (below the normal range half a step of 2^-149 for each rounding: of the value, two a tile of seven, three a stretch of two)
+    assert bool(((got - whole * 2.0 ** power).abs() <= 11 * 2.0 ** -149).all()), float(((got - whole * 2.0 ** power).norm() / got.norm()))
+
+
 def test_numbers_that_a_row_does_not_see():
     sc = Scene([(100, 60)], 4, 2, 128, 0, torch.float32, seed=6)
 
