@@ -76,25 +76,29 @@ attention_f32_join_kernel(const F32Args a) {
     const int TQ = BM / G, tok0 = (a.token_tiles - 1 - tile) * TQ;
     if (tok0 >= q_len || r >= min(TQ, q_len - tok0) * G) return;
     const int row = a.seq_q_start[seq] + tok0 + r / G, head = kvh * G + r % G;
+    // (a row's stretches are numbered in the order of their positions, the first at most by its own number: those behind the row's
+    // position are empty.  A step may have room for many more of them: decoded tokens have it for the longest context.  8 x 32 rows
+    // of 100 keys where contexts of 131,072 are allowed: attention 101 us with all of them read, 21 so)
+    const int slots = min(a.slots, (a.seq_pos_start[seq] + tok0 + r / G) / STRETCH + 1);
     float M = -INFINITY, L = 0.0f;
     float4 acc[2] = {};
     // Several stretches' numbers on their way at once, four where there are no more: one after the other, 17 of 8 x 32 rows took
     // 18 us, eight at a time 12.
     auto all = [&](auto ahead, auto pieces) {
         constexpr int A = decltype(ahead)::value, P = decltype(pieces)::value;
-        for (int s0 = 0; s0 < a.slots; s0 += A) {
+        for (int s0 = 0; s0 < slots; s0 += A) {
             float2 ml[A];
             float4 x[A][P];
 #pragma unroll
             for (int i = 0; i < A; ++i) {
-                const size_t at = part_at<BM>(a, min(s0 + i, a.slots - 1), pair, row, head, r);
+                const size_t at = part_at<BM>(a, min(s0 + i, slots - 1), pair, row, head, r);
                 ml[i] = *reinterpret_cast<const float2*>(a.part_ml + 2 * at);
 #pragma unroll
                 for (int c = 0; c < P; ++c) x[i][c] = *reinterpret_cast<const float4*>(a.part_o + at * a.vd + min(4 * lane + 128 * c, a.vd - 4));
             }
 #pragma unroll
             for (int i = 0; i < A; ++i) {
-                if (s0 + i >= a.slots || (ml[i].x == -INFINITY && ml[i].y == 0.0f)) continue;    // nothing was seen there (and nothing left)
+                if (s0 + i >= slots || (ml[i].x == -INFINITY && ml[i].y == 0.0f)) continue;    // nothing was seen there (and nothing left)
                 const Join j = join(M, L, ml[i].x, ml[i].y);
 #pragma unroll
                 for (int c = 0; c < P; ++c)
@@ -108,7 +112,7 @@ attention_f32_join_kernel(const F32Args a) {
     const std::integral_constant<int, 4> four;
     const std::integral_constant<int, 8> eight;
     if (a.vd > 128) all(four, two);
-    else if (a.slots > 4) all(eight, one);
+    else if (slots > 4) all(eight, one);
     else all(four, one);
     const float f = finish(a, row, head, M, L);
     float* op = a.out + (size_t)row * a.out_stride + (size_t)head * a.vd;
