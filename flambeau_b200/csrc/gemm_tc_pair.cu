@@ -115,9 +115,10 @@ __device__ __forceinline__ PairUnit pair_unit(int u, int tiles_m, int tiles, int
 }
 
 // The grouped form (routed experts): its weights come from HBM once, and a CTA's share of a tile's tokens from L2 is half of what
-// the one-SM kernel of 128 x 128 wants, whose 128 bytes a cycle and SM were its bound.  2,048 / 1,024 / 180 tokens on 6 of 64
-// experts of 1,792 x 4,096, both products: 491 -> 413, 396 -> 360, 327 -> 315 us, of which 287 are the weights at the copy rate;
-// 512 tokens 326 -> 335 (48 rows an expert fit tiles of 64 well, and this kernel is not launched ahead of the one before it ends).
+// the one-SM kernel of 128 x 128 wants, whose 128 bytes a cycle and SM were its bound.  2,048 / 1,024 / 512 / 180 tokens on 6 of 64
+// experts of 1,792 x 4,096, both products on the one-SM kernel's tiles of 64 and 128 / here: 560 / 417, 414 / 352, 331 / 330, 326 /
+// 317 us, of which 287 are the weights at the copy rate.  (Of 512 experts of 512 x 2,048 with 8 a token: 8,192 tokens 283 / 265,
+// 16,384 410 / 431, where the list below is too short.)
 // Rows come in tiles of 32 that belong to one group (an expert) each, negative groups are skipped.  A unit of
 // tokens is up to eight neighbouring tiles of one group, multiplied at their own width with that group's weight rows.  Every CTA
 // lists the units when it starts: one warp walks the tiles 32 at a time.  A unit is its first tile and, from bit 24 on, its tiles.
@@ -127,23 +128,35 @@ __device__ __forceinline__ uint32_t group_unit_at(const int* tile_group, int n_t
     while (c < PBN / P_GROUP_TILE && t + c < n_tiles && tile_group[t + c] == g) ++c;
     return (uint32_t)t | (uint32_t)c << 24;
 }
-// All 32 lanes.  Writes the first P_LIST units and returns how many there are.
+// All 32 lanes.  Writes the first P_LIST units and returns how many there are.  The groups of two stretches of 32 tiles are on their
+// way while one is looked at; where the runs of a stretch and of the next begin is a mask of 64 bits.  (With the loads of every
+// stretch, and of every unit's eight tiles, waited for where they were wanted, 2,048 tokens on 6 of 64 experts took 8 us longer a
+// product, 16,384 on 8 of 512 65.)
 __device__ __forceinline__ int group_units(const int* tile_group, int n_tiles, uint32_t* list) {
     constexpr int MOST = PBN / P_GROUP_TILE;
     const int lane = threadIdx.x & 31;
-    int found = 0, run = 0, before = -1;                 // run: where the run that reaches into this stretch began
-    for (int t0 = 0; t0 < n_tiles; t0 += 32) {
-        const int t = t0 + lane, g = t < n_tiles ? tile_group[t] : -1;
+    auto at = [&](int t) { return t < n_tiles ? tile_group[t] : -1; };
+    auto begins_of = [&](int g, int before) {
         const int left = __shfl_up_sync(0xffffffffu, g, 1);
-        const uint32_t begins = __ballot_sync(0xffffffffu, g != (lane ? left : before));
+        return __ballot_sync(0xffffffffu, g != (lane ? left : before));
+    };
+    int found = 0, run = 0, g = at(lane), next = at(32 + lane), after = at(64 + lane);      // run: where the one that reaches in began
+    uint32_t begins = begins_of(g, -1);
+    for (int t0 = 0; t0 < n_tiles; t0 += 32) {
+        const int further = at(t0 + 96 + lane);
+        const uint32_t begins_next = begins_of(next, __shfl_sync(0xffffffffu, g, 31));
         const uint32_t mine = begins & (0xffffffffu >> (31 - lane));
-        const int from = mine ? t0 + 31 - __clz(mine) : run;
+        const int t = t0 + lane, from = mine ? t0 + 31 - __clz(mine) : run;
         const uint32_t units = __ballot_sync(0xffffffffu, g >= 0 && (t - from) % MOST == 0);
-        const int at = found + __popc(units & ((1u << lane) - 1u));
-        if ((units >> lane & 1u) && at < P_LIST) list[at] = group_unit_at(tile_group, n_tiles, t);
+        const int place = found + __popc(units & ((1u << lane) - 1u));
+        const int left = __ffsll((long long)(((unsigned long long)begins_next << 32 | begins) >> (lane + 1)));      // tiles of the run from t on
+        if ((units >> lane & 1u) && place < P_LIST) list[place] = (uint32_t)t | (uint32_t)(left == 0 || left > MOST ? MOST : left) << 24;
         found += __popc(units);
         run = __shfl_sync(0xffffffffu, from, 31);
-        before = __shfl_sync(0xffffffffu, g, 31);
+        g = next;
+        next = after;
+        after = further;
+        begins = begins_next;
     }
     return found;
 }

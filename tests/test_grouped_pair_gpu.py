@@ -19,6 +19,7 @@ def product(x, w, group, out, **more):
 
 
 PATTERNS = {"sorted": [0] * 6 + [1] * 8 + [2] * 9 + [3] + [4] * 17 + [-1] * 3, "mixed": [2, 2, -1, 0, 2, 1, 1, -1, -1, 4, 3, 3, 3],
+            "stretches": [0] * 31 + [1] * 2 + [2] * 64 + [3] * 25 + [-1] * 40 + [4] * 41 + [0] + [1] * 7 + [-1],        # (a CTA lists 32 tiles at a time)
             "one": [1], "none": [-1, -1], "many": [i % 5 for i in range(450)] + [3] * 12 + [-1, 0]}
 
 
