@@ -524,6 +524,8 @@ static bool pair_on() {
     return g_pair_on != 0;
 }
 
+FB_API int fb_gemm_pair_on() { return pair_on() ? 1 : 0; }
+
 // Shares of K for tiles of 256 tokens: as many as make the rounds of the resident pairs shortest, each share beyond the first
 // costing one more float32 copy of the output (written here, added by the consumer), counted in k-block times.
 static int pair_splits(long tiles, int kb_total, int max_splits, int M, int N) {

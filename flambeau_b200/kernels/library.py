@@ -25,6 +25,7 @@ _SIGNATURES = {
     "fb_set_plain_launch_classes": (None, [I]),
     "fb_set_attention_tc": (None, [I]),
     "fb_set_gemm_pair": (None, [I]),
+    "fb_gemm_pair_on": (I, []),
     # elementwise.cu
     "fb_embedding": (I, [P, I, P, P, I, I, I, F, P, STREAM]),
     "fb_norm_add_rmsnorm": (I, [P, P, I, L, P, I, F, F, P, I, P, I, P, I, I, F, F, STREAM]),

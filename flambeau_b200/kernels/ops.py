@@ -734,10 +734,15 @@ _GROUPED_TC = [os.environ.get("FLAMBEAU_MOE_TC", "1") != "0"]
 def grouped_tile(pairs: int, groups: int, tensor_cores: bool) -> int:
     """Rows of a tile of the grouped products for `pairs` rows spread over `groups` groups: small tiles while a
     group holds few rows (decoding: a tile of 16 streams an expert's weights once), else 32 on the tensor cores, where the
-    kernel of two SMs joins a group's neighbouring tiles, and 64 on the CUDA cores."""
+    kernel of two SMs joins a group's neighbouring tiles, and 64 on the CUDA cores.  With that kernel switched off the one-SM
+    kernel multiplies tiles as they are: 64 rows, or 128 as the groups fill (its instruction takes as long for 64 columns)."""
     if pairs <= 16 * groups:
         return 16
-    return 32 if tensor_cores else 64
+    if not tensor_cores:
+        return 64
+    if lib().fb_gemm_pair_on():
+        return 32
+    return 128 if pairs >= 192 * groups else 64
 
 
 def gather_rows(h: torch.Tensor, place_token: torch.Tensor, out: torch.Tensor, share=None, place_pair=None, tile_group=None,

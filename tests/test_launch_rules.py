@@ -27,6 +27,20 @@ def test_stretches_of_decoded_tokens_over_latents_fill_whole_rounds():
     assert lib().fb_attention_tc_stretches(8, 125, 0, SMS) == 0 and lib().fb_attention_tc_stretches(8, 125, 2, SMS) == 2
 
 
+def test_rows_of_a_grouped_products_tiles():
+    """Tiles of 32 only for the kernel that joins them; the one-SM kernel has tiles of its own sizes."""
+    from flambeau_b200.kernels import ops
+    try:
+        ops.set_gemm_pair(True)
+        assert [ops.grouped_tile(n, 4, True) for n in (1, 64, 65, 767, 768, 9999)] == [16, 16, 32, 32, 32, 32]
+        assert [ops.grouped_tile(n, 4, False) for n in (64, 65, 9999)] == [16, 64, 64]
+        ops.set_gemm_pair(False)
+        assert [ops.grouped_tile(n, 4, True) for n in (1, 64, 65, 767, 768, 9999)] == [16, 16, 64, 64, 128, 128]
+        assert [ops.grouped_tile(n, 4, False) for n in (64, 65, 9999)] == [16, 64, 64]
+    finally:
+        ops.set_gemm_pair(True)
+
+
 def kernels(path):
     """(name, source) of every kernel of a file."""
     text = re.sub(r"//[^\n]*", "", path.read_text())
