@@ -309,6 +309,9 @@ __global__ void moe_gather_rows_kernel(const T* __restrict__ h, long h_stride, c
         group[i] = r < rows ? (tile_group ? tile_group[r / tile] : 0) : -1;   // (a tile that no product reads)
     }
 #pragma unroll
+    for (int i = 0; i < R; ++i)
+        if (group[i] < 0) src[i] = -1;                 // (what stands in its places is nobody's)
+#pragma unroll
     for (int i = 0; i < R; ++i) w[i] = share && src[i] >= 0 ? share[place_pair[r0 + i]] : 1.0f;
     struct alignas(sizeof(T) * 8) Chunk { T v[8]; };
     for (int c = threadIdx.x; c < chunks; c += blockDim.x) {

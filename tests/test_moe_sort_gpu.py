@@ -60,3 +60,24 @@ def test_rows_of_tiles_that_have_a_group(dtype, width, shared):
     for bad in (dict(tile_group=group[:4].cuda(), tile=tile), dict(tile_group=group.cuda(), tile=0), dict(tile_group=group.cuda(), tile=15)):
         with pytest.raises(KernelError):
             ops.gather_rows(h, token.cuda(), out, **bad)
+
+
+@pytest.mark.parametrize("rows", [192, 8256])                      # (a CTA a row; four)
+def test_places_of_tiles_without_a_group_are_not_followed(rows):
+    """Whatever stands there: no such token, no such pair."""
+    from flambeau_b200.kernels import ops
+    tile, D, tokens = 32, 136, 50
+    g = torch.Generator().manual_seed(rows)
+    group = torch.arange(rows // tile, dtype=torch.int32) % 3 - 1       # every third tile has none
+    token, pair = (torch.randint(0, tokens, (rows,), generator=g, dtype=torch.int32) for _ in range(2))
+    none = (group < 0).repeat_interleave(tile)
+    token[none], pair[none] = 2 ** 31 - 1, -2 ** 31
+    h, share = torch.randn(tokens, D, generator=g).bfloat16(), torch.rand(tokens, generator=g)
+    for more in ({}, dict(share=share.cuda(), place_pair=pair.cuda())):
+        out = torch.full((rows, D), 7.0, device="cuda").bfloat16()
+        ops.gather_rows(h.cuda(), token.cuda(), out, tile_group=group.cuda(), tile=tile, **more)
+        want = torch.full((rows, D), 7.0).bfloat16()
+        want[~none] = h[token[~none].long()]
+        if more:
+            want[~none] = (want[~none].float() * share[pair[~none].long(), None]).bfloat16()
+        assert torch.equal(out.cpu(), want)
