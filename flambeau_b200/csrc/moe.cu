@@ -290,8 +290,7 @@ __global__ void moe_combine_kernel(const float* __restrict__ expert_out, long ex
 // order, for the products that fetch their rows by tensor-map copies.  With `share` and `place_pair` the row is
 // multiplied by the share of the pair that the place stands for (experts whose weight scales what they read).
 // A CTA takes R rows, whose places and then numbers are in flight together: a row's way (tile, place, number) is
-// three latencies long, and with a CTA a row 12,288 rows of 4,096 took 42 us (64 experts' tiles of 128), 35 so (tiles of 32).
-// (A few rows stay with a CTA each: there the CTAs are what is missing.)
+// three latencies long.
 template <typename T, int R>
 __global__ void moe_gather_rows_kernel(const T* __restrict__ h, long h_stride, const int* __restrict__ place_token,
                                        T* __restrict__ out, int rows, int D, const float* __restrict__ share,
@@ -363,7 +362,10 @@ FB_API int fb_moe_gather_rows(const void* h, long long h_stride, int dtype, cons
         FB_DISPATCH_DTYPE(dtype, T,                                                                                     \
             (fb_launch((moe_gather_rows_kernel<T, R_>), dim3((unsigned)((rows + R_ - 1) / R_)), dim3(D / 8 <= 128 ? 128 : 256), 0, stream, \
                        (const T*)h, (long)h_stride, place_token, (T*)out, rows, D, share, place_pair, tile_group, tile)))
-        if (rows >= 4096) FB_GATHER(4);
+        // (us with 1 / 2 / 4 / 8 rows a CTA: 14,336 rows of 4,096 26.0 / 23.6 / 25.1 / 29.9, of 2,048 18.5 / 13.8 / 15.3 / 18.7, of
+        // 7,168 41.7 / 40.4 / 41.5 / 50.4; 3,136 of 4,096 6.0 / 5.6 / 6.5 / 8.0; 1,408, where the CTAs are what is missing, 3.7 /
+        // 3.9 / 5.1 / 7.2)
+        if (rows >= 2048) FB_GATHER(2);
         else FB_GATHER(1);
 #undef FB_GATHER
     } else {

@@ -62,7 +62,7 @@ def test_rows_of_tiles_that_have_a_group(dtype, width, shared):
             ops.gather_rows(h, token.cuda(), out, **bad)
 
 
-@pytest.mark.parametrize("rows", [192, 8256])                      # (a CTA a row; four)
+@pytest.mark.parametrize("rows", [192, 8256])                      # (a CTA a row; two)
 def test_places_of_tiles_without_a_group_are_not_followed(rows):
     """Whatever stands there: no such token, no such pair."""
     from flambeau_b200.kernels import ops
