@@ -175,9 +175,16 @@ int launch(const TA* a, long a_stride, long a_head, int n_partials, long partial
 }  // namespace
 
 // Bfloat16 weights [H, N, K] and outputs, inputs in bfloat16 or as float32 shares: portions of at least 128 rows (fewer leave a
-// tile half empty), and where shares are to be added a tile for every SM (130 rows of 32 heads, three shares, 128 -> 256: 21 us
-// here, 16 by 64 x 64 tiles, whose CTAs have more loads in flight together; 800 rows 8.6 and 17), sizes that are multiples of 64, at most 256 outputs, rows and
-// heads on 16-byte borders.  Returns 1, nothing done, for anything else: the caller takes fb_head_linear.
+// tile half empty), sizes that are multiples of 64, at most 256 outputs, rows and heads on 16-byte borders, and as many tiles of
+// 128 rows as it takes to be faster than 64 x 64 tiles, whose CTAs share a few rows' work among more SMs.  Measured over 2 to
+// 1,024 tiles (us there / here, inputs -> outputs):
+//   bfloat16: wherever there are as many inputs as outputs (256 -> 128: 8 tiles 5.8 / 4.4, 256 30.4 / 15.8), else from a quarter
+//   of the SMs on (64 -> 256: 8 tiles 1.4 times as long, 32 1.1, 40 even; 128 -> 256: 16 tiles 1.2 times, 40 0.8)
+//   float32: no more inputs than outputs, of which 128 at least, from half of the SMs on (128 -> 256: 8 tiles 4.1 / 7.4, 64 6.9 /
+//   7.5, 80 8.9 / 7.5, 512 39.0 / 17.6; 64 -> 64: 80 tiles 3.5 / 4.4, 448 7.1 / 7.8; 256 -> 128: 448 tiles 1.1 times as long)
+//   several float32 shares: from a tile for every SM on (130 rows of 32 heads, three shares, 128 -> 256: 21 us here, 16 there;
+//   800 rows 8.6 and 17)
+// Returns 1, nothing done, for anything else: the caller takes fb_head_linear.
 FB_API int fb_head_linear_tc(const void* a, int a_dtype, long long a_stride, long long a_head, int n_partials, long long partial_stride,
                              const void* w, void* out, long long o_stride, long long o_head, int n, int H, int N, int K, int* status,
                              cudaStream_t stream) {
@@ -187,7 +194,9 @@ FB_API int fb_head_linear_tc(const void* a, int a_dtype, long long a_stride, lon
     const long long per = a_dtype == FB_F32 ? 4 : 8;
     auto aligned = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
     const long tiles = (long)((n + HT_ROWS - 1) / HT_ROWS) * H;
-    const bool takes = n >= 128 && (n_partials == 1 || tiles >= fb_sm_count()) && N % HT_KB == 0 && N <= 256 && K % HT_KB == 0 && K <= 4096 && ht_smem(N, K) <= 227 * 1024 && H <= 65535 &&
+    const bool enough = n_partials > 1 ? tiles >= fb_sm_count()
+                        : a_dtype == FB_F32 ? N >= 128 && K <= N && tiles >= fb_sm_count() / 2 : K >= N || tiles >= fb_sm_count() / 4;
+    const bool takes = n >= 128 && enough && N % HT_KB == 0 && N <= 256 && K % HT_KB == 0 && K <= 4096 && ht_smem(N, K) <= 227 * 1024 && H <= 65535 &&
                        (long long)H * N < 2147483647LL && a_head >= 0 && a_head < 2147483647LL / H && o_head >= N && o_head < 2147483647LL / H &&
                        a_stride >= (H - 1) * a_head + K && o_stride >= (H - 1) * o_head + N && a_stride % per == 0 && a_head % per == 0 &&
                        (n_partials == 1 || partial_stride % per == 0) && o_stride % 8 == 0 && o_head % 8 == 0 && aligned(a) && aligned(w) &&

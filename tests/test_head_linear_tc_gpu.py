@@ -28,6 +28,24 @@ def test_rows_of_heads(n, N, K, shares):
     assert bool((got[..., N:] == 7.0).all())
 
 
+@pytest.mark.parametrize("n", [128, 300])
+@pytest.mark.parametrize("N,K", [(256, 128), (128, 128), (192, 64), (256, 192), (64, 64), (128, 256)])
+@pytest.mark.parametrize("H", [40, 80])                     # (float32 from half of the SMs on, and not towards fewer outputs)
+def test_rows_of_many_heads(H, N, K, n):
+    """One float32 share and bfloat16, on either side of the tiles from which on the kernel takes them: the same map."""
+    from flambeau_b200.kernels import ops
+    g = torch.Generator(device="cuda").manual_seed(n + N + H)
+    w = torch.randn(H, N, K, generator=g, device="cuda").bfloat16()
+    a, status = torch.randn(n, H * K, generator=g, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    x = a.bfloat16().double().view(n, H, K)
+    want, size = (torch.einsum("nhk,hck->nhc", p, q) for p, q in ((x, w.double()), (x.abs(), w.double().abs())))
+    for inputs in (a, a.bfloat16()):
+        out = torch.full((n, H * N), 7.0, device="cuda").bfloat16()
+        ops.head_linear(inputs, K, w, out, N, n, status=status)
+        assert int(status) == 0
+        assert bool(((out.double().view(n, H, N) - want).abs() <= K * 2.0 ** -23 * size + 2.0 ** -8 * want.abs() + 1e-30).all())
+
+
 def test_left_to_the_other_kernel():
     """Few rows, sizes off 64, rows off 16-byte borders: the same map by the kernel of 64 x 64 tiles."""
     from flambeau_b200.kernels import ops
