@@ -46,13 +46,6 @@ constexpr int BAD_K = 1, BAD_V = 2, GAPS = 4;    // a tile with keys or values t
 constexpr float T_MOST = 1.0e18f;        // (2^60)
 constexpr float V_IN = 281474976710656.0f, V_OUT = 1.0f / V_IN;          // (2^48: sums of 64 weighted values stay below 2^114)
 
-__device__ __forceinline__ void split2(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(b), "f"(a));
-    const float ra = a - __uint_as_float(h << 16), rb = b - __uint_as_float(h & 0xffff0000u);
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(m) : "f"(rb), "f"(ra));
-    const float sa = ra - __uint_as_float(m << 16), sb = rb - __uint_as_float(m & 0xffff0000u);
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(l) : "f"(sb), "f"(sa));
-}
 // The largest magnitude, NaN if there was one.
 __device__ __forceinline__ float larger(float a, float b) {
     float c;
@@ -65,8 +58,8 @@ template <int ROWS>
 __device__ __forceinline__ void place(uint32_t parts, int r, int lane, float4 v) {
     constexpr uint32_t PART = ROWS * THD * 2;
     uint2 h, m, l;
-    split2(v.x, v.y, h.x, m.x, l.x);
-    split2(v.z, v.w, h.y, m.y, l.y);
+    split_bf16x3(v.x, v.y, h.x, m.x, l.x);
+    split_bf16x3(v.z, v.w, h.y, m.y, l.y);
     const uint32_t at = parts + (uint32_t)((lane >> 4) * ROWS * 128 + r * 128 + ((((lane >> 1) & 7) ^ (r & 7)) << 4) + (lane & 1) * 8);
     asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(h.x), "r"(h.y) : "memory");
     asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at + PART), "r"(m.x), "r"(m.y) : "memory");
@@ -75,15 +68,9 @@ __device__ __forceinline__ void place(uint32_t parts, int r, int lane, float4 v)
 // Sixteen columns from each of two places, waited for once.
 __device__ __forceinline__ void tmem_ld16_two(uint32_t at, uint32_t too, float* x, float* y) {
     uint32_t r[16], q[16];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(at));
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7]), "=r"(q[8]), "=r"(q[9]),
-                   "=r"(q[10]), "=r"(q[11]), "=r"(q[12]), "=r"(q[13]), "=r"(q[14]), "=r"(q[15])
-                 : "r"(too));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    tmem_ld16_nowait(at, r);
+    tmem_ld16_nowait(too, q);
+    tmem_wait_ld();
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
         x[i] = __uint_as_float(r[i]);
@@ -515,7 +502,7 @@ attention_f32_tc_kernel(const __grid_constant__ F32Args a) {
             for (int c = 0; c < 32; c += 2) {
                 const float x = expf(s[c] - m_use), y = expf(s[c + 1] - m_use);
                 sum += x + y;
-                split2(x, y, ph[c / 2], pm[c / 2], pl[c / 2]);
+                split_bf16x3(x, y, ph[c / 2], pm[c / 2], pl[c / 2]);
             }
             l = l * corr + sum;
             m = m_new;

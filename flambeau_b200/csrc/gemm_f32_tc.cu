@@ -71,15 +71,9 @@ __device__ __forceinline__ uint64_t umma_desc_64(uint32_t smem_addr) {
 constexpr float SCALE_IN = 16777216.0f;                              // 2^24
 constexpr float SCALE_OUT = 1.0f / (SCALE_IN * SCALE_IN);
 
-// Two float32, scaled, into their three bfloat16 parts, packed (a in the lower half).
+// Two float32, scaled, into their three bfloat16 parts.
 __device__ __forceinline__ void split2(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
-    a *= SCALE_IN;
-    b *= SCALE_IN;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(b), "f"(a));
-    const float ra = a - __uint_as_float(h << 16), rb = b - __uint_as_float(h & 0xffff0000u);
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(m) : "f"(rb), "f"(ra));
-    const float sa = ra - __uint_as_float(m << 16), sb = rb - __uint_as_float(m & 0xffff0000u);
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(l) : "f"(sb), "f"(sa));
+    split_bf16x3(a * SCALE_IN, b * SCALE_IN, h, m, l);
 }
 
 // Xp[part][m][k] for k below Kp (a multiple of 32; zeros behind K).

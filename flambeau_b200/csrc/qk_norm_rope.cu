@@ -470,7 +470,13 @@ FB_API int fb_qk_norm_rope_kv_write(const float* proj, long long proj_stride, in
             // (threads: the row's columns in steps of four groups of four a thread, so that a common row is one step)
             const long cols = (long)nh * hd + (write_kv ? (long)nkv * hd + (v_is_k ? 0 : (long)nv * vd) : 0);
             const long steps = (cols + 6143) / 6144, threads = ((cols + 16 * steps - 1) / (16 * steps) + 31) / 32 * 32;
-#define FB_QKR_ROWS(LANES_)                                                                                                       FB_DISPATCH_DTYPE(w_dtype, TW, FB_DISPATCH_DTYPE(out_dtype, T,                                                            (fb_launch((qk_norm_rope_rows_kernel<TW, T, LANES_, 4>), dim3(n), dim3((unsigned)threads), 0, stream,                            proj, (long)proj_stride, n_partials, (long)partial_stride, (const TW*)bias, (const TW*)q_weight, (const TW*)k_weight,                            eps, weight_offset, cos_t, sin_t, half, (T*)q_out, (long)q_out_stride, positions, row_seq, block_table,                            table_stride, table_base, table_head, (T*)k_pool, (T*)v_pool, page_size, n_pages, nh, nkv, maps, vd,                            v_off, v_is_k, write_kv, status))))
+#define FB_QKR_ROWS(LANES_)                                                                                           \
+            FB_DISPATCH_DTYPE(w_dtype, TW, FB_DISPATCH_DTYPE(out_dtype, T,                                            \
+                (fb_launch((qk_norm_rope_rows_kernel<TW, T, LANES_, 4>), dim3(n), dim3((unsigned)threads), 0, stream, proj, \
+                           (long)proj_stride, n_partials, (long)partial_stride, (const TW*)bias, (const TW*)q_weight,  \
+                           (const TW*)k_weight, eps, weight_offset, cos_t, sin_t, half, (T*)q_out, (long)q_out_stride, \
+                           positions, row_seq, block_table, table_stride, table_base, table_head, (T*)k_pool,          \
+                           (T*)v_pool, page_size, n_pages, nh, nkv, maps, vd, v_off, v_is_k, write_kv, status))))
             if (hd == 32) FB_QKR_ROWS(8);
             else if (hd == 64) FB_QKR_ROWS(16);
             else FB_QKR_ROWS(32);
