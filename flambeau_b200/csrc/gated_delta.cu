@@ -152,6 +152,17 @@ gdr_prepare_vec_kernel(const float* __restrict__ proj, long proj_stride, int n_p
     auto fetch = [&](float4* x, int count, int row, int place, int of, int c, bool in) {
         const float* kept = state + (size_t)seq_slot[of] * state_stride + tail_off + c;
         const float* fresh = proj + c;
+        if (ROWS == 1 && n_partials > 1) {              // one number a tap, its shares eight at a time
+#pragma unroll
+            for (int m = 0; m < TAPS; ++m) {
+                const int off = m - (TAPS - 1);
+                x[m] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (!in) continue;
+                if (place + off >= 0) x[m] = slab_sum4(fresh + (long)(row + off) * proj_stride, n_partials, partial_stride);
+                else x[m] = Vec4<float>::load(kept + (long)(TAPS - 1 + place + off) * C);
+            }
+            return;
+        }
 #pragma unroll
         for (int m = 0; m < ROWS + TAPS - 1; ++m) {
             const int off = m - (TAPS - 1);
@@ -159,22 +170,15 @@ gdr_prepare_vec_kernel(const float* __restrict__ proj, long proj_stride, int n_p
             x[m] = in && m < count ? Vec4<float>::load(p) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         if (n_partials > 1 && in) {
-            if (ROWS == 1) {                            // one number, its shares eight at a time
+            for (int s = 1; s < n_partials; ++s)
 #pragma unroll
-                for (int m = 0; m < ROWS + TAPS - 1; ++m)
-                    if (m < count && place + m - (TAPS - 1) >= 0)
-                        x[m] = slab_sum4(fresh + (long)(row + m - (TAPS - 1)) * proj_stride, n_partials, partial_stride);
-            } else {
-                for (int s = 1; s < n_partials; ++s)
-#pragma unroll
-                    for (int m = 0; m < ROWS + TAPS - 1; ++m) {
-                        if (m >= count) break;
-                        const int off = m - (TAPS - 1);
-                        if (place + off < 0) continue;
-                        const float4 v = Vec4<float>::load(fresh + (size_t)s * partial_stride + (long)(row + off) * proj_stride);
-                        x[m].x += v.x; x[m].y += v.y; x[m].z += v.z; x[m].w += v.w;
-                    }
-            }
+                for (int m = 0; m < ROWS + TAPS - 1; ++m) {
+                    if (m >= count) break;
+                    const int off = m - (TAPS - 1);
+                    if (place + off < 0) continue;
+                    const float4 v = Vec4<float>::load(fresh + (size_t)s * partial_stride + (long)(row + off) * proj_stride);
+                    x[m].x += v.x; x[m].y += v.y; x[m].z += v.z; x[m].w += v.w;
+                }
         }
     };
     auto mix = [&](int i, const float4* x) -> float4 {  // the convolution over x[0 .. TAPS) with its SiLU
