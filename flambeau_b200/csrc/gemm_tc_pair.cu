@@ -1,12 +1,14 @@
 // out[M,N] = X[M,K] * W[N,K]^T in bfloat16 with two SMs on one tile (tcgen05.mma cta_group::2), for products with
 // hundreds of rows (portions of prompts).
 //
-// A cluster of two CTAs owns 256 output features x 256 tokens.  Each CTA stages its own 128 weight rows and its
-// own 128 of the 256 tokens, so a CTA fetches and holds half of what the one-CTA kernel (gemm_tc.cu) does for
-// the token operand; the even CTA of the pair issues one MMA of M = 256, N = 256 that reads both CTAs' shared
-// memory and writes both CTAs' tensor memory (128 features x 256 tokens in each).  Otherwise it is the
+// A cluster of two CTAs owns 256 output features x up to 256 tokens (w: a multiple of 32 that the launcher chooses, so that the
+// tiles divide the rows evenly; the last tile as wide as what is left).  Each CTA stages its own 128 weight rows and its
+// own half of the tile's tokens, so a CTA fetches and holds half of what the one-CTA kernel (gemm_tc.cu) does for
+// the token operand; the even CTA of the pair issues one MMA of M = 256, N = w that reads both CTAs' shared
+// memory and writes both CTAs' tensor memory (128 features x w tokens in each).  Otherwise it is the
 // arrangement of gemm_tc.cu: swap-AB, K-major operands with the 128-byte swizzle, 64 elements of K a stage,
 // two accumulators so that the epilogue of one tile overlaps the products of the next, persistent pairs.
+// The grouped form (routed experts) joins neighbouring row tiles of one group to tiles of up to 256 tokens.
 //
 // Barriers.  full[s] lives in the even CTA and counts the bytes of both CTAs' copies (the copies carry
 // cta_group::2, which lets them signal the peer's barrier).  empty[s] and acc_full[b] exist in both CTAs and are
