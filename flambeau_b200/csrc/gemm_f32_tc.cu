@@ -475,11 +475,26 @@ FPlan plan_f32_tc(long M, long N, int shares, int stages, long partial_floats, i
     return best;
 }
 
+constexpr long SPLIT_FLOATS = 16L << 20;         // most that the shares of one product may take
+
+int stages_of_k(int K) { return (K + FBK - 1) / FBK; }
+int shares_of_k(int K) { return (stages_of_k(K) + SHARE_STAGES - 1) / SHARE_STAGES; }
+
 }  // namespace
+
+// Floats of `partials` that fb_gemm_f32_tc wants for the same sizes with `n_counters` counters: 0 where K is not split.
+FB_API long long fb_gemm_f32_tc_scratch_floats(int M, int N, int K, int n_counters) {
+    if (M <= 0 || N <= 0 || K <= 0) return 0;
+    const int shares = shares_of_k(K);
+    const FPlan p = plan_f32_tc(M, N, shares, stages_of_k(K), SPLIT_FLOATS, n_counters);
+    if (p.splits == 1) return 0;
+    return (long long)((M + p.bn - 1) / p.bn) * ((N + FBM - 1) / FBM) * shares * p.bn * FBM;
+}
 
 // X [M,K] and out [M,N] float32 with any strides of at least a row; W [N,K] float32 whose rows start on 16-byte borders, K a
 // multiple of 4.  `parts` takes 3 M Kp bfloat16 (Kp: K rounded up to a multiple of 32), 16-byte aligned; `partials` and
-// `counters` (zero before the call and after it) are the scratch of split K, as in fb_gemm_tc; without them K is not split.
+// `counters` (zero before the call and after it) are the scratch of split K, as in fb_gemm_tc, of calls that run one after the
+// other; without them, or with fewer floats than fb_gemm_f32_tc_scratch_floats asks for, K is split less or not at all.
 FB_API int fb_gemm_f32_tc(const void* X, long long lda, const void* W, long long ldw, void* out, long long ldo, int M, int N,
                           int K, void* parts, long long parts_elems, float* partials, long long partial_floats, int* counters,
                           int n_counters, int* status, cudaStream_t stream) {
@@ -491,7 +506,7 @@ FB_API int fb_gemm_f32_tc(const void* X, long long lda, const void* W, long long
     const int Kp = (K + FBK - 1) / FBK * FBK;
     FB_REQUIRE(parts && ((uintptr_t)parts & 15) == 0 && parts_elems >= 3LL * M * Kp, "gemm_f32_tc: scratch for the rows' parts missing");
     FB_REQUIRE(3LL * M < 2147483647LL, "gemm_f32_tc: too many rows (M=%d)", M);
-    const int stages = Kp / FBK, shares = (stages + SHARE_STAGES - 1) / SHARE_STAGES;
+    const int stages = stages_of_k(K), shares = shares_of_k(K);
     const FPlan plan = plan_f32_tc(M, N, shares, stages, partials && counters ? partial_floats : 0, counters ? n_counters : 0);
     F32Tc a = {};
     a.X = (const float*)X; a.lda = (long)lda; a.W = (const float*)W; a.ldw = (long)ldw; a.out = (float*)out; a.ldo = (long)ldo;

@@ -43,12 +43,18 @@ class Workspace:
     It grows by replacing its buffer with a larger one; tensors handed out
     before keep the old storage alive until they are dropped.  While `frozen`
     (during graph capture and replay) it refuses to grow.
+
+    `counters` are zero between launches: a kernel whose CTAs count each other's
+    arrivals there leaves them so.  They belong to the arena, whose steps run one
+    after the other, and not to the device, where engines on other streams run too.
     """
     ALIGN = 256
+    COUNTERS = 8192
 
     def __init__(self, device, nbytes: int = 1 << 20):
         self.device = device
         self.buffer = torch.empty(max(nbytes, self.ALIGN), dtype=torch.uint8, device=device)
+        self.counters = torch.zeros(self.COUNTERS, dtype=torch.int32, device=device)
         self.top = 0
         self.high_water = 0
         self.frozen = False

@@ -49,6 +49,7 @@ _SIGNATURES = {
     "fb_gemm_simt": (I, [P, I, L, P, I, L, P, I, L, I, I, I, STREAM]),
     "fb_gemm_simt_grouped": (I, [P, I, L, P, P, I, L, L, P, I, P, I, L, I, I, I, I, STREAM]),
     # gemm_f32_tc.cu
+    "fb_gemm_f32_tc_scratch_floats": (L, [I, I, I, I]),
     "fb_gemm_f32_tc": (I, [P, L, P, L, P, L, I, I, I, P, L, P, L, P, I, P, STREAM]),
     # gemm_tc.cu
     "fb_gemm_tc_add": (I, [P, L, P, L, P, L, I, I, I, I, P, STREAM]),

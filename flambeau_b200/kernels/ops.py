@@ -645,7 +645,7 @@ def f32_tc_supported(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> boo
 
 def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: torch.Tensor, ws) -> None:
     """out[M,N] = a[M,K] @ w[N,K]^T in float32 on the tensor cores: every float32 as three bfloat16 numbers (see
-    csrc/gemm_f32_tc.cu).  `ws` is the step's arena, which holds the parts of `a` meanwhile."""
+    csrc/gemm_f32_tc.cu).  `ws` is the step's arena, which holds the parts of `a` and the shares of K meanwhile."""
     _cuda(a, w, out, status)
     M, K = a.shape
     N = w.shape[0]
@@ -653,11 +653,13 @@ def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: tor
         raise KernelError(f"gemm: shapes a{tuple(a.shape)} w{tuple(w.shape)} out{tuple(out.shape)} do not agree")
     if not (a.dtype == w.dtype == out.dtype == torch.float32):
         raise KernelError("gemm_f32_tc: operands must be float32")
-    partials, counters = _SplitScratch.get(a.device)
+    counters = ws.counters
+    floats = lib().fb_gemm_f32_tc_scratch_floats(M, N, K, counters.numel())
     with ws.scope():
         parts = ws.alloc((3 * M * ((K + 31) // 32 * 32),), torch.bfloat16)
+        partials = ws.alloc((floats,), torch.float32) if floats > 0 else None
         check(lib().fb_gemm_f32_tc(a.data_ptr(), _rows(a), w.data_ptr(), _rows(w), out.data_ptr(), _rows(out), M, N, K,
-                                   parts.data_ptr(), parts.numel(), partials.data_ptr(), partials.numel(),
+                                   parts.data_ptr(), parts.numel(), _ptr(partials), floats,
                                    counters.data_ptr(), counters.numel(), status.data_ptr(), _stream()),
               "gemm_f32_tc", (M, N, K))
 
@@ -855,7 +857,7 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, ctx=None) -> Non
     float32 operands they can fetch by TMA, the float32-FMA kernel for everything else."""
     if ctx is not None and tc_supported(a, w, out):
         gemm_tc(a, w, out, ctx.runtime.status)
-    elif ctx is not None and f32_tc_supported(a, w, out):
+    elif getattr(ctx, "ws", None) is not None and f32_tc_supported(a, w, out):
         gemm_f32_tc(a, w, out, ctx.runtime.status, ctx.ws)
     else:
         gemm_simt(a, w, out)

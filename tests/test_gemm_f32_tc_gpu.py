@@ -60,3 +60,37 @@ def test_numbers_without_parts(M, N):
     err = (got.double() - want.double()).abs()
     # (both lie within their own bounds of the exact values; below the normal range half of the smallest number an addition)
     assert bool((err[fine] <= ((5 + K / 64 + K / 512) * 2.0 ** -23 + (K / 2 + 2) * 2.0 ** -24) * size[fine] + K * 2.0 ** -149).all())
+
+
+def test_engines_on_two_streams():
+    """Products whose shares of K meet in scratch, on two streams at a time: the scratch is an arena's, not the device's."""
+    from flambeau_b200.engine.runtime import Workspace
+    from flambeau_b200.kernels import ops
+    M, N, K, times = 8, 512, 8192, 60
+    g = torch.Generator(device="cuda").manual_seed(0)
+    side = []
+    for _ in range(2):
+        a, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
+        side.append((a, w, product(a, w), torch.zeros(times, M, N, device="cuda"), Workspace("cuda"), torch.cuda.Stream(),
+                     torch.zeros(1, dtype=torch.int32, device="cuda")))
+    assert ops.lib().fb_gemm_f32_tc_scratch_floats(M, N, K, Workspace.COUNTERS) > 0, "K is to be split"
+    torch.cuda.synchronize()
+    for i in range(times):
+        for a, w, _, outs, ws, stream, status in side:
+            with torch.cuda.stream(stream):
+                ops.gemm_f32_tc(a, w, outs[i], status, ws)
+    torch.cuda.synchronize()
+    for _, _, want, outs, ws, _, status in side:
+        assert int(status) == 0 and not bool(ws.counters.any())
+        assert torch.equal(outs, want.expand_as(outs))
+
+
+def test_contexts_without_an_arena():
+    """What has no arena to split its rows in is multiplied on the CUDA cores, as before."""
+    from types import SimpleNamespace
+    from flambeau_b200.kernels import ops
+    a, w = torch.randn(3, 512, device="cuda"), torch.randn(64, 512, device="cuda")
+    out, want = torch.empty(3, 64, device="cuda"), torch.empty(3, 64, device="cuda")
+    ops.linear(a, w, out, SimpleNamespace(runtime=SimpleNamespace(status=torch.zeros(1, dtype=torch.int32, device="cuda"))))
+    ops.gemm_simt(a, w, want)
+    assert torch.equal(out, want)
